@@ -351,6 +351,14 @@ int qe_w4_gemv_static(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream)
 int qe_w4_plan_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, qe_w4_plan* plan);
 int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream);
 
+/* Packs W [M, K] (row stride ld0; dtype 0 bf16, 1 fp16, 2 fp32) into the wire format on the GPU: qw
+ * int32 [Mp/16, Kp/64, 32, 4] (16-byte aligned), scales fp16 [Mp/16, Kp/128, 16]. With w1 != NULL w0 / w1
+ * are a gate / up pair, both [M, K], whose rows are interleaved in blocks of 8 for QE_EPI_SWIGLU
+ * (Mp / 2 = M rounded up to 8). Bit-identical to python/qengine/quant.py:41-148 of the reference, which
+ * packs with torch operators; it has no launcher for it. */
+int qe_w4_pack(const void* w0, const void* w1, int dtype, int M, int K, long ld0, long ld1, void* qw,
+               void* scales, void* stream);
+
 /* The weight rings are fed by bulk copies whose completion waits are bounded; this returns the
  * sticky error word those waits set on expiry (0 = none) and qe_w4_clear_error resets it. Both
  * synchronise with the device. No counterpart in the reference. */

@@ -113,9 +113,36 @@ def _quantize_pack(W: torch.Tensor, M: int, K: int, gate_up: bool, rows_per_step
     return W4Packed(qw, sc, M, K, gate_up)
 
 
+_PACK_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
+
+
+def _on_gpu(*mats: torch.Tensor) -> bool:
+    """Matrices the GPU packer takes: same CUDA device and type, unit stride along K, not empty."""
+    a = mats[0]
+    return all(m.is_cuda and m.device == a.device and m.dtype == a.dtype and m.dtype in _PACK_DTYPE and m.numel() > 0 and
+               m.stride(1) == 1 and m.stride(0) >= m.shape[1] for m in mats)
+
+
+def _pack_on_gpu(*mats: torch.Tensor) -> W4Packed:
+    """One kernel over the matrix (or the gate / up pair), qe_w4_pack; the bits of `_quantize_pack`."""
+    from ._lib import check, lib
+    (M, K), dev = mats[0].shape, mats[0].device
+    gate_up = len(mats) == 2
+    Mp, Kp = 2 * _ceil(M, 8) if gate_up else _ceil(M, 16), _ceil(K, GROUP)
+    qw = torch.empty(Mp // 16, Kp // 64, 32, 4, dtype=torch.int32, device=dev)
+    sc = torch.empty(Mp // 16, Kp // GROUP, 16, dtype=torch.float16, device=dev)
+    with torch.cuda.device(dev):
+        check(lib.qe_w4_pack(mats[0].data_ptr(), mats[1].data_ptr() if gate_up else None, _PACK_DTYPE[mats[0].dtype], M, K,
+                             mats[0].stride(0), mats[-1].stride(0), qw.data_ptr(), sc.data_ptr(),
+                             torch.cuda.current_stream().cuda_stream), "w4_pack")
+    return W4Packed(qw, sc, M, K, gate_up)
+
+
 def quantize_w4(W: torch.Tensor) -> W4Packed:
     """RTN symmetric int4, group 128 along K, fp16 scales. W: [M, K], any float dtype."""
     assert W.dim() == 2
+    if _on_gpu(W):
+        return _pack_on_gpu(W)
     return _quantize_pack(W, W.shape[0], W.shape[1], False)
 
 
@@ -135,6 +162,9 @@ def interleave_gate_up(Wg: torch.Tensor, Wu: torch.Tensor) -> torch.Tensor:
 
 def quantize_w4_gate_up(Wg: torch.Tensor, Wu: torch.Tensor) -> W4Packed:
     """Pack gate [I, K] and up [I, K] for gemv_swiglu (out = silu(x Wg^T) * x Wu^T)."""
+    assert Wg.shape == Wu.shape and Wg.dim() == 2
+    if _on_gpu(Wg, Wu):
+        return _pack_on_gpu(Wg, Wu)
     I, K = Wg.shape
     return _quantize_pack(interleave_gate_up(Wg, Wu), I, K, True)
 

@@ -1,0 +1,52 @@
+"""The GPU packer (qe_w4_pack behind quant.quantize_w4 / quantize_w4_gate_up) against the torch packer, which
+the golden vectors of the reference pin: every bit of codes and scales. (The scale of a group with a NaN in
+it is a NaN on both sides; its payload is 0x7fff on the GPU and 0x7e00 on the CPU, for torch as well.)"""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _w(M, K, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    w = torch.randn(M, K, generator=g) * torch.rand(M, 1, generator=g)
+    w[0] = 0.0                                    # a row of zeros: scale 0, code 8
+    if M > 3 and K > 3:
+        w[1] = torch.randint(-15, 16, (K,), generator=g) / 2.0   # quotients on the middle between two codes
+        w[1, 0] = 7.5
+        w[2] *= 1e-9                              # scale below fp16's smallest number
+        w[3] *= 3e-6                              # scale a denormal fp16
+        w[-1] *= 1e6                              # scale beyond fp16: infinite
+        w[M // 2, K // 2] = float("nan")
+    return w.to(dtype)
+
+
+def _same(a, b):
+    sa, sb = a.scales.cpu(), b.scales
+    assert torch.equal(a.qw.cpu(), b.qw) and torch.equal(sa.isnan(), sb.isnan())
+    assert torch.equal(sa.nan_to_num(-1.0), sb.nan_to_num(-1.0))
+    assert (a.M, a.K, a.gate_up) == (b.M, b.K, b.gate_up)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,K", [(16, 128), (1, 1), (15, 127), (17, 129), (200, 1000), (512, 640), (333, 2056)])
+def test_bits_of_the_torch_packer(M, K, dtype):
+    from qengine_b200 import quant
+    w = _w(M, K, dtype, seed=M + K)
+    w[~w.isfinite() & ~w.isnan()] = 1.0           # fp16 cannot hold the 1e6 row
+    _same(quant.quantize_w4(w.cuda()), quant.quantize_w4(w))
+    u = _w(M, K, dtype, seed=M + K + 1)
+    u[~u.isfinite() & ~u.isnan()] = 1.0
+    _same(quant.quantize_w4_gate_up(w.cuda(), u.cuda()), quant.quantize_w4_gate_up(w, u))
+
+
+def test_views_and_misaligned_rows():
+    from qengine_b200 import quant
+    big = torch.randn(300, 1030, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
+    dev = big.cuda()
+    for rows, cols in ((slice(0, 256), slice(0, 1024)), (slice(3, 200), slice(1, 900)), (slice(0, 300, 2), slice(8, 776))):
+        _same(quant.quantize_w4(dev[rows, cols]), quant.quantize_w4(big[rows, cols]))
+    _same(quant.quantize_w4(dev.T), quant.quantize_w4(big.T))                    # no unit stride along K: torch path
+    _same(quant.quantize_w4(dev.double()), quant.quantize_w4(big.double()))
