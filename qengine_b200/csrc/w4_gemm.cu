@@ -11,8 +11,8 @@
 // GEMV's, so a row agrees with the GEMV to fp32 rounding, not bit for bit.
 //
 // Two kernels behind qe_w4_gemm:
-//   * w4_gemm_tc_kernel (the default): tcgen05.mma, operands in shared memory, accumulator in
-//     tensor memory; described in front of it, further down.
+//   * w4_gemm_tc_kernel (the default): tcgen05.mma, weights and accumulator in tensor
+//     memory; described in front of it, further down.
 //   * w4_gemm_kernel (cfg->variant == 1): mma.sync.m16n8k16 on register fragments, described
 //     next. With 8 row tiles it issues eight times the mma.sync instructions of the GEMV per
 //     unit and saturates near 130 TFLOP/s, the rate of the legacy tensor path on this part: 64
@@ -34,9 +34,12 @@
 // Every mbarrier wait of both kernels is bounded; on expiry the warp records the error word
 // (reported by qe_w4_ring_error), stops working, keeps arriving where others wait for it, and the
 // CTA frees its tensor memory and leaves.
+#include <cuda.h>  // CUtensorMap (types only: the encoder is looked up at run time)
+
 #include <cuda/atomic>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "w4_dev.cuh"
 
@@ -285,56 +288,69 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_gemm_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------------------------
-// The tensor-core path proper: tcgen05.mma with the accumulator in tensor memory.
+// The tensor-core path proper: tcgen05.mma with weights and accumulator in tensor memory.
 //
-// A job is one super-tile, 128 weight rows (eight 16-row tiles of the wire format) over all of K;
-// the CTAs take super-tiles round-robin. One step = one group g (128 k) of a super-tile:
-//   * 16 warps in two halves: warps 0..7 prepare the even steps, warps 8..15 the odd ones, one
-//     tile each. Preparing = pull the tile's 1 KB unit of the step through a private ring of bulk
-//     copies, unpack it to the exact bf16 integers code - 8 (w4_dev.cuh) and store it as rows of
-//     the A operand [128 rows x 128 k] in the K-major 128-byte-swizzle layout the tensor core
-//     reads (row pitch 128 B, 16-byte chunk index XOR row % 8; 16-byte stores, conflict-free);
-//     and copy the step's activations [64 rows x 128 k] from global memory (L2) into the same
-//     layout as the B operand, one own step ahead through registers;
-//   * a seventeenth warp waits for the 16 arrivals of a step and issues its 8 tcgen05.mma (M 128,
-//     N 64, K 16), which leave the group's exact integer dot products D_g[m, n] in one of three
-//     64-column accumulators in tensor memory;
-//   * every one of the 16 warps, every step, reads its 16 columns of D_{g-2} for its row
-//     (tcgen05.ld), multiplies by the row's group scale in fp32 and adds to 16 registers:
-//     acc[m, n] += scale[m, g] * D_g[m, n], groups in ascending order -- the arithmetic of the GEMV
-//     (exact products, fp32 sums inside a group, the scale applied once per group).
-// A, B and the accumulators have three stages and the halves alternate, so one half unpacks
-// step z + 1 while the products of steps z and z - 1 are under way; there is no block-wide barrier
-// in the loop, the warps meet only through two kinds of mbarrier: "step z may be multiplied" (one
-// arrival per warp: its share of the operands is stored, if it had one, and it has read the
-// products of step z - 3 out of the accumulator) and "products of step z complete"
-// (tcgen05.commit). After the last group the registers hold the super-tile's [128 x 64] result:
-// rounded and stored (or combined into SwiGLU) from there. A matrix with fewer super-tiles than
-// half the SMs (the 5,120-row out and down projections: 40) is also split along K, up to as many
-// jobs as there are SMs; the parts of a super-tile meet in a caller-provided fp32 workspace.
+// A job is one super-tile, 128 weight rows (eight 16-row tiles of the wire format), over its part
+// of K. A CTA walks its jobs two at a time (same K, so they share the activations) and a last odd
+// one alone. One step = one group g (128 k) of a walk; one micro-step = that group of one of its
+// super-tiles. Three roles, coupled by mbarriers only:
+//   * unpack (warps 9..16, two groups of four that alternate micro-steps): two tiles' 1 KB units per
+//     warp come from HBM straight into registers, kTcAhead own micro-steps ahead (a lane's 32 bytes
+//     of a unit are contiguous in the wire format, so nothing has to pass through shared memory),
+//     are unpacked to the exact bf16 integers code - 8 and stored as the A operand [128 x 128 k] in
+//     tensor memory. tcgen05.st.16x256b takes from lane (r, t) the words 2 t, 2 t + 1 of rows r, r + 8
+//     of each 8-word block, and a word of the wire format (rows r, r + 8, four consecutive k) unpacks
+//     to just these four registers; transpose4 brings the words of a row pair into ascending k;
+//   * warp 0 issues a micro-step's eight tcgen05.mma (M 128, K 16, A from tensor memory, B from shared
+//     memory) into one of four 64-column accumulators: the group's exact integer dot products D_g[m, n];
+//   * drain (warps 1..8): a pair's super-tiles are read by four warps each, a lone one by all eight,
+//     half the columns each; scale[m, g] * D_g[m, n] is added to fp32 registers, groups in ascending
+//     order -- the arithmetic of the GEMV (exact products, fp32 sums inside a group, the scale applied
+//     once per group). They also request the activations (a tensor map over the rows of x, two steps
+//     per request, K-major, 128-byte swizzle) and their scales, and store the result through shared
+//     memory, four rows at a time.
+// A and D have four stages, B has kTcB. A stage of A is free when the products of the micro-step four
+// before are complete (the barrier the drain warps wait for, too); a stage of B when a drain warp has
+// seen the products of a later step.
+//
+// What bounds it. Per unit of weights (1 KB, 46 clk of HBM time per SM at the copy rate) an SM issues
+// some 240 warp instructions on four schedulers (60 clk) and multiplies for 32 clk; it takes 110 clk:
+// the turns of the issuing thread and of a drain warp, barrier waits of 200 clk and more among them,
+// come one after the other. 64 rows, 27B shapes: gate/up 81.8 -> 44.3 us, in_proj 41.0 -> 26.9,
+// down 53.0 -> 35.5, out 25.2 -> 21.2 against the form with A and the weight ring in shared memory,
+// where every warp did all three roles in turn and their latencies added up.
+//
+// A matrix with fewer super-tiles than half the SMs (the 5,120-row out and down projections: 40) is
+// also split along K, up to as many jobs as there are SMs; the parts of a super-tile meet in a
+// caller-provided fp32 workspace.
 // ---------------------------------------------------------------------------------------------
-constexpr int kTcWarps = 16, kTcThreads = (kTcWarps + 1) * 32, kTcStages = 4, kTcDepth = 3, kTcCols = 256;
-constexpr int kTcScales = 8;                   // buffers of group scales (see the loop)
-constexpr uint32_t kTcStageBytes = 1024 + 32;  // one unit of codes + its 16 scales
-constexpr uint32_t kTcRing = kTcStages * kTcStageBytes;
-constexpr uint32_t kTcA = 128 * 256, kTcB = 64 * 256;  // one stage of A / B
+constexpr int kTcThreads = 17 * 32, kTcAhead = 3, kTcB = 8;
+constexpr uint32_t kTcBStage = 64 * 256;  // 64 rows x 128 k
+constexpr uint32_t kTcPitch = 132;        // floats per row of the output staging: 128 rows of the super-tile + 4
+constexpr int kTcChunk = 28;              // groups per request of scales
+constexpr uint32_t kTcScaleBytes = kTcChunk * 32;  // of one tile
 constexpr uint32_t kTcSmem =
-    kTcDepth * (kTcA + kTcB) + kTcWarps * kTcRing + kTcScales * 128 * sizeof(float) + 1024;
+    kTcB * kTcBStage + 2 * 64 * kTcPitch * sizeof(float) + 8 * 2 * 2 * kTcScaleBytes + 1024;
+static_assert(kTcSmem + 512 <= 227 * 1024, "shared memory of one block");
+constexpr uint32_t kTcACol = 256;         // tensor memory: D in columns 0..255, A in 256..511
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
 __device__ __forceinline__ uint64_t tc_desc(uint32_t smem_addr) {
   return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor: bf16 x bf16 -> fp32, both operands K-major, N = 64, M = 128.
-constexpr uint32_t kTcIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t accumulate) {
+// D (+)= A * B^T: bf16 x bf16 -> fp32, M = 128, N in the instruction descriptor, K = 16.
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(da), "l"(db), "r"(kTcIdesc), "r"(accumulate), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(bar))
@@ -354,316 +370,461 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(u[k]);
 }
+// One 64-k chunk of a unit (16 bytes of codes per lane) -> 16 rows x 32 words of tensor memory.
+__device__ __forceinline__ void tc_st_chunk(uint32_t taddr, const uint4& w) {
+  const AFrag f0 = unpack_word(w.x), f1 = unpack_word(w.y), f2 = unpack_word(w.z), f3 = unpack_word(w.w);
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(f0.a0), "r"(f0.a2), "r"(f0.a1), "r"(f0.a3), "r"(f1.a0), "r"(f1.a2), "r"(f1.a1), "r"(f1.a3),
+        "r"(f2.a0), "r"(f2.a2), "r"(f2.a1), "r"(f2.a3), "r"(f3.a0), "r"(f3.a2), "r"(f3.a1), "r"(f3.a3)
+      : "memory");
+}
+// Word s of lane t (of the four lanes of a row pair) -> word t of lane s: lane t then holds k = 16 b + 4 t
+// .. + 3 in its word b, so that the eight words of a 16-k block are in ascending k and the
+// activations need no permutation.
+__device__ __forceinline__ void transpose4(uint4& w, int t) {
+  const bool hi = t & 2, odd = t & 1;
+  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, hi ? w.x : w.z, 2), r1 = __shfl_xor_sync(0xffffffffu, hi ? w.y : w.w, 2);
+  const uint32_t y00 = hi ? r0 : w.x, y01 = hi ? r1 : w.y, y10 = hi ? w.z : r0, y11 = hi ? w.w : r1;
+  const uint32_t q0 = __shfl_xor_sync(0xffffffffu, odd ? y00 : y01, 1), q1 = __shfl_xor_sync(0xffffffffu, odd ? y10 : y11, 1);
+  w = make_uint4(odd ? q0 : y00, odd ? y01 : q0, odd ? q1 : y10, odd ? y11 : q1);
+}
+// Weights are constant while the kernel runs and read once: no L1 line for them.
+__device__ __forceinline__ uint4 ld_codes(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes 16, or 0: zero fill
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// 64 rows x 256 k of the activations as four 64-k chunks from chunk c: map dimensions (64 k, rows, chunks).
+__device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap* map, int c, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(0), "r"(c), "r"(sa(bar))
+      : "memory");
+}
+// (a0, a1) += s * (b0, b1): two fp32 fused multiply-adds in one instruction.
+__device__ __forceinline__ void fma2(float& a0, float& a1, float s, float b0, float b1) {
+  asm("{\n\t.reg .b64 a, b, s;\n\t"
+      "mov.b64 a, {%0, %1};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 s, {%2, %2};\n\t"
+      "fma.rn.f32x2 a, s, b, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(s), "f"(b0), "f"(b1));
+}
 
-__global__ void __launch_bounds__(kTcThreads, 1) w4_gemm_tc_kernel(const __grid_constant__ GemmArgs a) {
+// Four consecutive output rows (from `row`) of activation row n.
+__device__ __forceinline__ void tc_put4(const OutDesc& o, bool vec, int n, int row, const float4& f) {
+  if (row >= o.M) return;
+  const float e[4] = {f.x, f.y, f.z, f.w};
+  if (o.out_f32) {
+    float* p = static_cast<float*>(o.out) + (long)n * o.ldo + row;
+    if (vec && row + 3 < o.M) {
+      *reinterpret_cast<float4*>(p) = f;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (row + k < o.M) p[k] = e[k];
+    }
+  } else {
+    bf16* p = static_cast<bf16*>(o.out) + (long)n * o.ldo + row;
+    if (vec && row + 3 < o.M) {
+      *reinterpret_cast<uint2*>(p) = make_uint2(pack2(f.x, f.y), pack2(f.z, f.w));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (row + k < o.M) p[k] = tobf16(e[k]);
+    }
+  }
+}
+// The finished sums of a super-tile, get(n, m) = those of its rows m .. m + 3, by `threads` threads.
+template <typename Get>
+__device__ __forceinline__ void tc_store(const OutDesc& o, int tile0, int ti, int threads, Get get) {
+  const bool vec = (o.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(o.out) & (o.out_f32 ? 15 : 7)) == 0;
+  if (o.epi == QE_EPI_SWIGLU) {  // rows 0..7 of a tile are gate rows, 8..15 the matching up rows
+#pragma unroll 2
+    for (int e = ti; e < o.N * 16; e += threads) {
+      const int n = e >> 4, m0 = (e & 14) * 8 + (e & 1) * 4;
+      const float4 g = get(n, m0), u = get(n, m0 + 8);
+      tc_put4(o, vec, n, tile0 * 8 + (e & 15) * 4,
+              make_float4(silu_fast(g.x) * u.x, silu_fast(g.y) * u.y, silu_fast(g.z) * u.z, silu_fast(g.w) * u.w));
+    }
+  } else {
+#pragma unroll 2
+    for (int e = ti; e < o.N * 32; e += threads)
+      tc_put4(o, vec, e >> 5, tile0 * 16 + (e & 31) * 4, get(e >> 5, (e & 31) * 4));
+  }
+}
+// The parts of a super-tile split along K, added in ascending order.
+__device__ __forceinline__ void tc_add_parts(const GemmArgs& a, int st, int ti) {
+  __threadfence();
+  const int KP = a.kparts;
+  const float4* wp = reinterpret_cast<const float4*>(a.ws + (size_t)(st * KP) * (64 * 128));
+  tc_store(a.o, st * 8, ti, 256, [&](int n, int m0) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p0 = 0; p0 < KP; p0 += 4) {
+      float4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p0 + k < KP) x[k] = __ldcg(wp + (size_t)(p0 + k) * (64 * 32) + n * 32 + (m0 >> 2));
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p0 + k < KP) f.x += x[k].x, f.y += x[k].y, f.z += x[k].z, f.w += x[k].w;
+    }
+    return f;
+  });
+}
+
+template <bool kTma>
+__global__ void __launch_bounds__(kTcThreads, 1)
+    w4_gemm_tc_kernel(const __grid_constant__ GemmArgs a, const __grid_constant__ CUtensorMap xmap) {
   dep_release();
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full_w[kTcWarps][kTcStages];
-  __shared__ uint64_t a_full[kTcDepth];  // step z may be multiplied: one arrival per unpacking warp
-  __shared__ uint64_t d_full[kTcDepth];  // its products are in tensor memory (tcgen05.commit)
+  // micro-step may be multiplied: its A is stored (one arrival per unpacking warp of its group) and
+  // the D of the micro-step four before has been read (eight arrivals: one per drain warp, or two
+  // where four of them read it)
+  __shared__ uint64_t ready[4];
+  __shared__ uint64_t d_full[4];     // its products are complete (tcgen05.commit): D readable, A free
+  __shared__ uint64_t b_full[kTcB / 2];  // activations of two steps are stored (bytes, or arrivals of the drain threads)
+  __shared__ uint64_t s_full[8][2];      // a drain warp's next scales have landed
   __shared__ uint32_t tmem_slot;
   __shared__ int s_last;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int r = lane >> 2, t = lane & 3;
-  unsigned char* base = smem_raw + ((1024u - (sa(smem_raw) & 1023u)) & 1023u);  // swizzle atoms: 1 KB aligned
-  unsigned char* Bbase = base + kTcDepth * kTcA;
-  float* sc = reinterpret_cast<float*>(Bbase + kTcDepth * kTcB + (size_t)kTcWarps * kTcRing);  // [kTcScales][128]
+  unsigned char* Bbase = smem_raw + ((1024u - (sa(smem_raw) & 1023u)) & 1023u);  // swizzle atoms: 1 KB aligned
 
-  if (tid == 0) {
-    for (int b = 0; b < kTcDepth; ++b) {
-      bar_init(&a_full[b], kTcWarps);
-      bar_init(&d_full[b], 1);
-    }
+  if (warp == 1) {  // one barrier per lane
+    if (lane < 4) bar_init(&ready[lane], 4 + 8);
+    else if (lane < 8) bar_init(&d_full[lane - 4], 1);
+    else if (lane < 8 + kTcB / 2) bar_init(&b_full[lane - 8], kTma ? 1 : 2 * 256);
+    else if (lane >= 16) bar_init(&s_full[(lane - 16) >> 1][lane & 1], 1);
+    bar_fence_init();
   }
-  if (lane == 0 && warp < kTcWarps) {
-    for (int s = 0; s < kTcStages; ++s) bar_init(&full_w[warp][s], 1);
-  }
-  if (lane == 0) bar_fence_init();
-  __syncwarp();
-  if (warp == kTcWarps) {  // tensor memory: three accumulators of 64 columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&tmem_slot)), "r"(kTcCols)
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
 
-  // ---- this CTA's jobs: (super-tile, part of K), dealt out round-robin ----
+  // ---- this CTA's jobs: (super-tile, part of K), dealt out round-robin, walked in pairs ----
   const int G = a.G, N = a.o.N, KP = a.kparts;
   const int J = ((a.tiles + 7) >> 3) * KP;
   const int cta = blockIdx.x, nctas = gridDim.x;
   const int nj = cta < J ? (J - cta + nctas - 1) / nctas : 0;
-  struct Cur {
-    int j, g, gend, tile0, jidx;
+  // K is split only where every CTA has one job at most
+  const int g_begin = KP > 1 ? share_begin(G, KP, cta % KP) : 0;
+  const int g_end = KP > 1 ? share_begin(G, KP, cta % KP + 1) : G;
+  auto tile0_of = [&](int j) { return (cta + j * nctas) / KP * 8; };
+
+  const int q = warp & 3;  // quarter of the tensor-memory lanes this warp can reach
+  constexpr int kLast = 1 << 30;
+  // Unpacking warps: cursor over the warp's own micro-steps. Pair walks have one per step and
+  // super-tile (group 0 the first super-tile, group 1 the second); a lone super-tile's steps alternate.
+  const int grp = ((warp - 1) >> 2) & 1;
+  int cj = 0, cg = 0;  // first job of the walk, group
+  const uint4* cp = a.qw;
+  long second = 0;  // distance of the second tile's unit (0: beyond the matrix, never stored)
+  auto enter = [&](int j) {
+    cj = j;
+    const bool pair = j + 1 < nj;
+    if (j >= nj) { cg = kLast; return; }
+    cg = g_begin + (pair ? 0 : grp);
+    const int tile = min(tile0_of(pair ? j + grp : j) + 2 * q, a.tiles - 1);
+    cp = a.qw + ((long)tile * G + cg) * 64 + lane;
+    second = tile + 1 < a.tiles ? (long)G * 64 : 0;
   };
-  auto cur_set = [&](Cur& c, int j) {
-    c.j = j;
-    if (j < nj) {
-      c.jidx = cta + j * nctas;
-      const int st = c.jidx / KP, part = c.jidx - st * KP;
-      c.g = share_begin(G, KP, part);
-      c.gend = share_begin(G, KP, part + 1);
-      c.tile0 = st * 8;
-    } else {
-      c.jidx = 0; c.g = 0; c.gend = 1 << 30; c.tile0 = 0;
-    }
+  uint4 wreg[kTcAhead][4];
+  auto load_next = [&](uint4 (&w)[4]) {  // request the own micro-step under the cursor and move on
+    while (cg != kLast && cg >= g_end) enter(cj + 2);
+    if (cg == kLast) return;
+    w[0] = ld_codes(cp);
+    w[1] = ld_codes(cp + 32);
+    w[2] = ld_codes(cp + second);
+    w[3] = ld_codes(cp + second + 32);
+    const int step = cj + 1 < nj ? 1 : 2;
+    cg += step;
+    cp += step * 64;
   };
-  auto cur_next = [&](Cur& c) {
-    if (++c.g == c.gend) cur_set(c, c.j + 1);
-  };
-  int Z = 0;  // steps
-  {
-    Cur c;
-    for (int j = 0; j < nj; ++j) {
-      cur_set(c, j);
-      Z += c.gend - c.g;
-    }
+  if (warp > 8) {  // weights never depend on the kernel before: requested before anything is waited for
+    enter(0);
+#pragma unroll
+    for (int i = 0; i < kTcAhead; ++i) load_next(wreg[i]);
   }
 
-  if (warp == kTcWarps) {
-    // ---- the issuing warp: 8 products per step as soon as the step may be multiplied ----
-    // One thread issues: its instruction latency is what a step waits for, so the descriptors are
-    // built once and only their start-address field (low word, 16-byte units) moves in the loop.
-    const uint64_t da0 = tc_desc(sa(base)), db0 = tc_desc(sa(Bbase));
-    bool ok = true;
-    int s3 = 0, ph = 0;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  const int per_job = g_end - g_begin;
+  const int V = nj * per_job;              // micro-steps
+  const int n16 = (N + 15) >> 4;           // blocks of 16 activation rows
+  // Steps are numbered with every walk rounded up to an even count: two share a load of B.
+  const int walk = (per_job + 1) & ~1, steps = ((nj + 1) >> 1) * walk;
+
+  if (warp == 0) {
+    // ---- the issuing warp ----
+    const uint32_t idesc =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((128u >> 4) << 24);
+    const uint64_t db0 = tc_desc(sa(Bbase));
+    if (elect_one()) {
+      int v = 0, z = 0;
+      bool ok = true;
 #pragma unroll 1
-    for (int z = 0; z < Z && ok; ++z) {
-      if (!warp_wait(&a_full[s3], ph)) {
-        ok = false;
-        atomicExch(&g_gemm_error, 2);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
-        const uint64_t da = da0 + (uint64_t)(s3 * (kTcA >> 4)), db = db0 + (uint64_t)(s3 * (kTcB >> 4));
-        const uint32_t d = tmem + s3 * 64;
+      for (int j = 0; j < nj && ok; j += 2) {
+        const bool pair = j + 1 < nj;
+#pragma unroll 1
+        for (int i = 0; i < per_job && ok; ++i, ++z) {
+          const uint64_t db = db0 + (uint64_t)((z & (kTcB - 1)) * (kTcBStage >> 4));
+          if (!(i & 1)) {
+            ok = bar_wait(&b_full[(z >> 1) & (kTcB / 2 - 1)], (z / kTcB) & 1, kGemmWaitLimit);
+            // Copies made by other threads: the fence that shows them to the tensor core is here because
+            // it waits for its thread's own outstanding memory operations, of which this one has none.
+            if (!kTma) async_proxy_fence();
+          }
+#pragma unroll 1
+          for (int h = 0; h < (pair ? 2 : 1) && ok; ++h, ++v) {
+            const int s = v & 3;
+            ok = bar_wait(&ready[s], (v >> 2) & 1, kGemmWaitLimit);
+            tc_fence_after();
+            const uint32_t d = tmem + s * 64, ac = tmem + kTcACol + s * 64;
+            if (ok) {
 #pragma unroll
-        for (int c2 = 0; c2 < 2; ++c2)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tc_mma(d, da + (uint64_t)(c2 * (16384 >> 4) + kk * 2), db + (uint64_t)(c2 * (8192 >> 4) + kk * 2),
-                   (c2 | kk) ? 1u : 0u);
-        tc_commit(&d_full[s3]);
+              for (int k = 0; k < 8; ++k)
+                tc_mma(d, ac + 8 * k, db + (uint64_t)((k >> 2) * (8192 >> 4) + (k & 3) * 2), idesc, k ? 1u : 0u);
+              tc_commit(&d_full[s]);
+            }
+          }
+        }
+        if (per_job & 1) ++z;
       }
-      __syncwarp();
-      if (++s3 == kTcDepth) { s3 = 0; ph ^= 1; }
+      if (!ok) atomicExch(&g_gemm_error, 2);
+    }
+    __syncwarp();
+  } else if (warp > 8) {
+    // ---- unpacking warps ----
+    const uint32_t t_lane = tmem + kTcACol + ((uint32_t)(32 * q) << 16);
+    bool ok = true;
+#pragma unroll 1
+    for (int v0 = grp; v0 < V && ok; v0 += 2 * kTcAhead) {
+#pragma unroll
+      for (int i = 0; i < kTcAhead; ++i) {
+        const int v = v0 + 2 * i, s = v & 3;
+        if (v >= V || !ok) break;
+        if (v >= 4 && !warp_wait(&d_full[s], ((v >> 2) - 1) & 1)) {
+          ok = false;
+          atomicExch(&g_gemm_error, 1);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t t0 = t_lane + s * 64;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) transpose4(wreg[i][h], lane & 3);
+        tc_st_chunk(t0, wreg[i][0]);
+        tc_st_chunk(t0 + 32, wreg[i][1]);
+        tc_st_chunk(t0 + (16u << 16), wreg[i][2]);
+        tc_st_chunk(t0 + (16u << 16) + 32, wreg[i][3]);
+        load_next(wreg[i]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(&ready[s]);
+      }
     }
   } else {
-    // ---- the 16 unpacking warps ----
-    unsigned char* ring = Bbase + kTcDepth * kTcB + (size_t)warp * kTcRing;
-    const int par = warp >> 3, ti = warp & 7;  // prepares the steps of this parity; tile of the super-tile
-    // the unit of this warp's tile in a step; false beyond the matrix (only the matrix's last
-    // super-tile can lack tiles, and its jobs are the last ones of their CTAs)
-    auto unit_of = [&](const Cur& c, size_t& u) {
-      u = (size_t)(c.tile0 + ti) * G + c.g;
-      return c.j < nj && c.tile0 + ti < a.tiles;
+    // ---- drain warps ----
+    const int wd = warp - 1;
+    const int m = 32 * q + lane;  // this thread's row of a super-tile
+    const uint32_t t_lane = tmem + ((uint32_t)(32 * q) << 16);
+    float* const stage = reinterpret_cast<float*>(Bbase + kTcB * kTcBStage);  // [2 groups][64][kTcPitch]
+    float* const mine = stage + grp * 64 * kTcPitch;
+    // Scales of the warp's two tiles (its 32 rows), kTcChunk groups at a time, two requests ahead. Plain
+    // loads into registers, several groups ahead, cost a memory latency per step: they share the few
+    // scoreboards of the warp with everything else.
+    unsigned char* const scales = Bbase + kTcB * kTcBStage + 2 * 64 * kTcPitch * sizeof(float) + wd * 4 * kTcScaleBytes;
+    int sj = 0, sg = 0, snext = 0;  // walk, first group and number of the next request
+    auto request_scales = [&] {
+      if (sj >= nj) return;
+      const int n = min(kTcChunk, per_job - sg);
+      if (elect_one()) {
+        const int tile = tile0_of(sj + 1 < nj ? sj + grp : sj) + 2 * q;
+        unsigned char* dst = scales + (snext & 1) * 2 * kTcScaleBytes;
+        uint64_t* bar = &s_full[wd][snext & 1];
+        const __half* src = a.scales + ((size_t)min(tile, a.tiles - 1) * G + g_begin + sg) * 16;
+        bar_expect(bar, 2 * n * 32);
+        bulk_g2s(dst, src, n * 32, bar);
+        bulk_g2s(dst + kTcScaleBytes, tile + 1 < a.tiles ? src + (size_t)G * 16 : src, n * 32, bar);
+      }
+      __syncwarp();
+      ++snext;
+      sg += kTcChunk;
+      if (sg >= per_job) sg = 0, sj += 2;
     };
-    auto fill_w = [&](size_t u, int at) {  // lane 0
-      unsigned char* dst = ring + (size_t)at * kTcStageBytes;
-      bar_expect(&full_w[warp][at], kTcStageBytes);
-      bulk_g2s(dst, reinterpret_cast<const unsigned char*>(a.qw) + u * 1024, 1024, &full_w[warp][at]);
-      bulk_g2s(dst + 1024, a.scales + u * 16, 32, &full_w[warp][at]);
+    request_scales();  // constant like the weights: before the wait
+    request_scales();
+    auto sync_group = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+    auto sync_all = [&] { asm volatile("bar.sync 3, 256;" ::: "memory"); };
+
+    int bg = g_begin, bi = 0;  // group of the next step to load, and its number in the walk
+    // rows that a tensor map cannot describe: 16-byte pieces, rows 16 i + 2 wd + lane / 16
+    const int n0 = 2 * wd + (lane >> 4);
+    const bf16* const xsrc = a.x + (long)n0 * a.ldx + (lane & 15) * 8;
+    const uint32_t bdst = sa(Bbase) + ((lane >> 3) & 1) * 8192 + n0 * 128 + (((lane & 7) ^ (n0 & 7)) << 4);
+    auto load_b = [&](int z) {
+      if (z >= steps) return;
+      const uint32_t dst = bdst + (z & (kTcB - 1)) * kTcBStage;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= n16 || bi >= per_job) break;
+        const bool row = n0 + 16 * i < N;
+        cp_async16(dst + i * 2048, row ? xsrc + 16 * i * a.ldx + bg * 128 : a.x, row ? 16u : 0u);
+      }
+      // this thread's copies up to here have landed: one of the 512 arrivals of two steps
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];"
+                   ::"r"(sa(&b_full[(z >> 1) & (kTcB / 2 - 1)])) : "memory");
+      ++bg;
+      if (++bi == walk) bi = 0, bg = g_begin;
     };
-    Cur cz, cr;  // the current step; the next own step to request from HBM
-    cur_set(cz, 0);
-    cur_set(cr, 0);
-    if (par) cur_next(cr);
-    for (int q = 0; q < kTcStages; ++q) {
-      size_t u;
-      if (!unit_of(cr, u)) break;
-      if (lane == 0) fill_w(u, q);
-      cur_next(cr);
-      cur_next(cr);
-    }
     dep_wait();
-
-    // this thread's four 16-byte pieces of the activations of a group (64 rows x 16 pieces,
-    // dealt out over the 256 threads of a half): rows n0 + 16 i, piece j16
-    const int t256 = tid & 255, n0 = t256 >> 4, j16 = t256 & 15;
-    const uint4* xsrc = reinterpret_cast<const uint4*>(a.x + (long)n0 * a.ldx) + j16;
-    const long xstep = 2 * a.ldx;  // 16 rows on, in 16-byte units
-    const uint32_t boff = (j16 >> 3) * 8192 + n0 * 128 + (((j16 & 7) ^ (n0 & 7)) << 4);  // + 2048 i
-    uint4 xr[4];
-    auto load_x = [&](int g) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        xr[i] = n0 + 16 * i < N ? xsrc[(long)i * xstep + g * 16] : make_uint4(0u, 0u, 0u, 0u);
+    // Activations by the copy engine: two steps per request, the requests dealt out over the eight
+    // warps because each holds up its warp for some hundred clocks.
+    auto request_b = [&](int u) {
+      if (2 * u < steps && elect_one()) {
+        uint64_t* bar = &b_full[u & (kTcB / 2 - 1)];
+        bar_expect(bar, 2 * kTcBStage);
+        tma_rows(sa(Bbase) + (u & (kTcB / 2 - 1)) * 2 * kTcBStage, &xmap, 2 * g_begin + u % (walk >> 1) * 4, bar);
+      }
+      __syncwarp();
     };
-    {
-      Cur c = cz;
-      if (par) cur_next(c);
-      if (c.j < nj) load_x(c.g);
+    int unit = wd;   // next request of this warp (two steps)
+    int loaded = 0;  // without a tensor map: steps whose activations have been requested
+    if constexpr (kTma) {
+      if (wd < kTcB / 2) {
+        request_b(wd);
+        unit += 8;
+      }
+    } else {
+      for (; loaded < kTcB - 1; ++loaded) load_b(loaded);
     }
-
-    const int m = 32 * (warp & 3) + lane;  // this thread's row of the super-tile (a tensor-memory lane)
-    const int col0 = 16 * (warp >> 2);     // its 16 activation rows
-    const uint32_t t_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + col0;
-    float acc[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+    if (lane == 0) {  // nothing to read out of D yet
+      for (int s = 0; s < 4; ++s) bar_arrive(&ready[s]);
+    }
 
     bool ok = true;
-    // acc += scale[m, group of step z] * D(z)
-    auto drain = [&](int z) {
-      const int s3 = z % kTcDepth, ph = (z / kTcDepth) & 1;
-      if (ok && !warp_wait(&d_full[s3], ph)) {
-        ok = false;
-        atomicExch(&g_gemm_error, 4);
-      }
-      if (!ok) return;
-      tc_fence_after();
-      float v[16];
-      tc_ld16(t_lane + s3 * 64, v);
-      const float sm = sc[(z & (kTcScales - 1)) * 128 + m];
+    int vb = 0, zb = 0, chunk = 0;  // first micro-step and step of the walk, request of scales
+    // One walk's sums, left in the staging. A pair: this group's super-tile, all columns. A lone
+    // super-tile: all its micro-steps, columns 32 grp .. + 31. Either way one thread adds the groups
+    // of a sum in ascending order.
+    auto drain = [&](auto is_pair) {
+      constexpr bool kPair = decltype(is_pair)::value;
+      constexpr int kBlocks = kPair ? 4 : 2;  // of 16 columns
+      const int col0 = kPair ? 0 : 32 * grp, blocks = n16 - (kPair ? 0 : 2 * grp);
+      float acc[16 * kBlocks];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) acc[k] = fmaf(sm, v[k], acc[k]);
-    };
-    auto store_out = [&](int tile0) {  // the finished sums of a super-tile, from registers
-      const int tile = tile0 + (m >> 4), rr = m & 15;
-      if (a.o.epi == QE_EPI_SWIGLU) {
-        bf16* o = static_cast<bf16*>(a.o.out);
-        const int jrow = tile * 8 + rr;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const float up = __shfl_down_sync(0xffffffffu, acc[k], 8);
-          const int n = col0 + k;
-          if (ok && rr < 8 && jrow < a.o.M && n < N) o[(long)n * a.o.ldo + jrow] = tobf16(silu_fast(acc[k]) * up);
+      for (int k = 0; k < 16 * kBlocks; ++k) acc[k] = 0.f;
+      int i = 0, v = vb + (kPair ? grp : 0);
+#pragma unroll 1
+      for (int c0 = 0; c0 < per_job; c0 += kTcChunk, ++chunk) {
+        if (ok && !warp_wait(&s_full[wd][chunk & 1], (chunk >> 1) & 1)) {
+          ok = false;
+          if (lane == 0) atomicExch(&g_gemm_error, 8);
         }
-      } else {
-        const int mrow = tile * 16 + rr;
-        if (ok && mrow < a.o.M) {
+        const __half* const sc = reinterpret_cast<const __half*>(scales + ((chunk & 1) * 2 + (lane >> 4)) * kTcScaleBytes) +
+                                 (lane & 15) - c0 * 16;
+        const int end = min(c0 + kTcChunk, per_job);
+#pragma unroll 1
+        for (; i < end && ok; ++i, v += kPair ? 2 : 1) {
+          const int s = v & 3;
+          const float scale = __half2float(sc[i * 16]);
+          if (!warp_wait(&d_full[s], (v >> 2) & 1)) {
+            ok = false;
+            if (lane == 0) atomicExch(&g_gemm_error, 4);
+            break;
+          }
+          tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            const int n = col0 + k;
-            if (n >= N) continue;
-            if (a.o.out_f32) static_cast<float*>(a.o.out)[(long)n * a.o.ldo + mrow] = acc[k];
-            else static_cast<bf16*>(a.o.out)[(long)n * a.o.ldo + mrow] = tobf16(acc[k]);
+          for (int h = 0; h < kBlocks; ++h) {
+            if (h >= blocks) break;
+            float d[16];
+            tc_ld16(t_lane + s * 64 + col0 + h * 16, d);
+#pragma unroll
+            for (int k = 0; k < 16; k += 2) fma2(acc[16 * h + k], acc[16 * h + k + 1], scale, d[k], d[k + 1]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(sa(&ready[s])), "n"(kPair ? 2 : 1) : "memory");
+          // all steps before this one are multiplied: their stages of B are free
+          if constexpr (kTma) {
+            if (2 * unit < zb + i + kTcB - 1) {
+              request_b(unit);
+              unit += 8;
+            }
+          } else {
+            for (; loaded < min(steps, zb + i + kTcB); ++loaded) load_b(loaded);
           }
         }
+        __syncwarp();  // every lane has read its scales
+        request_scales();
       }
+      if (!kPair && zb > 0) sync_all();  // both groups have stored the walk before: the staging may be rewritten
+      float* const to = (kPair ? mine : stage + col0 * kTcPitch) + m;
+#pragma unroll
+      for (int k = 0; k < 16 * kBlocks; ++k)
+        if (k < 16 * blocks) to[k * kTcPitch] = acc[k];
     };
 
-    // Three stages of A, B and accumulator; a warp reads the products of step z two steps later.
-    // Before it arrives for step z (and before it writes stage z % 3) it has read the products of
-    // step z - 3, so they are complete, the stage is free, and the issuing warp may overwrite that
-    // accumulator once all 16 have arrived. A writer of the scales of step z + L has seen the
-    // products of step z + L - 3, issued after everybody arrived for that step; a reader still
-    // busy with step z has arrived for z + 2 at most, so L <= 5: eight buffers of scales.
-    int slot = 0, phase = 0, since = 0, s3 = 0;
 #pragma unroll 1
-    for (int z = 0; z < Z; ++z) {
-      if ((z & 1) == par) {
-        unsigned char* As = base + (size_t)s3 * kTcA;
-        unsigned char* Bs = Bbase + (size_t)s3 * kTcB;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(Bs + boff + 2048 * i) = xr[i];
-        size_t u;
-        if (unit_of(cz, u)) {
-          if (ok && !warp_wait(&full_w[warp][slot], phase)) {
-            ok = false;
-            atomicExch(&g_gemm_error, 1);
-          }
-          if (ok) {
-            const unsigned char* st = ring + (size_t)slot * kTcStageBytes;
-            const uint4 w0 = reinterpret_cast<const uint4*>(st)[lane], w1 = reinterpret_cast<const uint4*>(st)[32 + lane];
-            if (lane < 16)
-              sc[(z & (kTcScales - 1)) * 128 + 16 * ti + lane] = __half2float(reinterpret_cast<const __half*>(st + 1024)[lane]);
-            unsigned char* rowp = As + (16 * ti + r) * 128;  // row r of the tile; row r + 8 is 1 KB on
-            const uint32_t c0 = (uint32_t)((2 * t) ^ r) << 4, c1 = (uint32_t)((2 * t + 1) ^ r) << 4;
-#pragma unroll
-            for (int ch = 0; ch < 2; ++ch) {  // the two 64-k chunks of the unit
-              const uint4 wv = ch ? w1 : w0;
-              const AFrag f0 = unpack_word(wv.x), f1 = unpack_word(wv.y), f2 = unpack_word(wv.z), f3 = unpack_word(wv.w);
-              unsigned char* q = rowp + ch * 16384;
-              *reinterpret_cast<uint4*>(q + c0) = make_uint4(f0.a0, f0.a2, f1.a0, f1.a2);
-              *reinterpret_cast<uint4*>(q + c1) = make_uint4(f2.a0, f2.a2, f3.a0, f3.a2);
-              *reinterpret_cast<uint4*>(q + 1024 + c0) = make_uint4(f0.a1, f0.a3, f1.a1, f1.a3);
-              *reinterpret_cast<uint4*>(q + 1024 + c1) = make_uint4(f2.a1, f2.a3, f3.a1, f3.a3);
-            }
-          }
-          __syncwarp();  // every lane has read this stage: hand its slot back to the copy engine
-          size_t un;
-          if (unit_of(cr, un)) {
-            if (lane == 0 && ok) fill_w(un, slot);
-            cur_next(cr);
-            cur_next(cr);
-          }
-          if (++slot == kTcStages) { slot = 0; phase ^= 1; }
-        }
-        async_proxy_fence();  // the stores above become visible to the tensor core's reads
-      }
-      tc_fence_before();  // this thread's tensor-memory loads are ordered before the arrival
-      __syncwarp();
-      if (lane == 0) bar_arrive(&a_full[s3]);
-      if (++s3 == kTcDepth) s3 = 0;
-      if ((z & 1) == par) {
-        // The activations of the next own step: requested after the proxy fence above (which
-        // would wait for them), two steps ahead of their use.
-        Cur c = cz;
-        cur_next(c);
-        cur_next(c);
-        if (c.j < nj) load_x(c.g);
-      }
-      if (since >= 2) drain(z - 2);
-      if (cz.g + 1 == cz.gend) {
-        // last group of the job: two or three more drains complete its sums
-        if (since >= 1) drain(z - 1);
-        drain(z);
-        since = 0;
-        if (KP == 1) {
-          store_out(cz.tile0);
-        } else {
-          // A super-tile split along K: every part leaves its fp32 sums in the workspace; the
-          // CTA that delivers the last part adds them in ascending order of the parts (so the
-          // result does not depend on who was last) and stores the tile.
-          float* wsj = a.ws + (size_t)cz.jidx * (64 * 128);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) __stcg(wsj + (col0 + k) * 128 + m, acc[k]);
-          __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(kTcWarps * 32) : "memory");
-          const int st = cz.tile0 >> 3;
-          if (tid == 0) {
-            cuda::atomic_ref<int, cuda::thread_scope_device> arrivals(a.counters[st]);
-            const int last = arrivals.fetch_add(1, cuda::memory_order_acq_rel) == KP - 1;
-            if (last) a.counters[st] = 0;
-            s_last = last;
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(kTcWarps * 32) : "memory");
-          const int last = s_last;
-          asm volatile("bar.sync 1, %0;" ::"n"(kTcWarps * 32) : "memory");  // s_last may be rewritten
-          if (last) {
-            __threadfence();
-#pragma unroll
-            for (int k = 0; k < 16; ++k) acc[k] = 0.f;
-            for (int p2 = 0; p2 < KP; ++p2) {
-              const float* wp = a.ws + (size_t)(st * KP + p2) * (64 * 128);
-#pragma unroll
-              for (int k = 0; k < 16; ++k) acc[k] += __ldcg(wp + (col0 + k) * 128 + m);
-            }
-            store_out(cz.tile0);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+    for (int j = 0; j < nj; j += 2) {
+      const bool pair = j + 1 < nj;
+      if (pair) drain(std::true_type{});
+      else drain(std::false_type{});
+      // read again after the loops: kept over them, the output's description takes the sums' registers
+      const GemmArgs* late = &a;
+      asm volatile("" : "+l"(late));
+      if (pair) {
+        sync_group();
+        if (ok)
+          tc_store(late->o, tile0_of(j + grp), (tid - 32) & 127, 128,
+                   [&](int n, int m0) { return *reinterpret_cast<const float4*>(mine + n * kTcPitch + m0); });
+        sync_group();  // the staging may be rewritten
       } else {
-        ++since;
+        auto sum = [&](int n, int m0) { return *reinterpret_cast<const float4*>(stage + n * kTcPitch + m0); };
+        sync_all();
+        if (KP == 1 && ok) tc_store(late->o, tile0_of(j), tid - 32, 256, sum);
       }
-      cur_next(cz);
+      vb += (pair ? 2 : 1) * per_job;
+      zb += walk;
     }
-    if (!ok) {  // give the copies that are still in flight a bounded chance to land
-      __syncwarp();
-      for (int s = 0; s < kTcStages; ++s) bar_wait(&full_w[warp][s], 0, 1 << 10), bar_wait(&full_w[warp][s], 1, 1 << 10);
+    if (KP > 1 && nj > 0) {
+      // A super-tile split along K (every CTA has one job at most): every part leaves its fp32 sums in
+      // the workspace; the CTA that delivers the last part adds them in ascending order of the parts
+      // (so the result does not depend on who was last) and stores the tile.
+      const GemmArgs* late = &a;
+      asm volatile("" : "+l"(late));
+      const int ti = tid - 32, st = cta / KP;
+      float4* wsj = reinterpret_cast<float4*>(late->ws + (size_t)cta * (64 * 128));
+#pragma unroll 4
+      for (int e = ti; e < late->o.N * 32; e += 256)
+        __stcg(wsj + e, *reinterpret_cast<const float4*>(stage + (e >> 5) * kTcPitch + (e & 31) * 4));
+      __threadfence();
+      sync_all();
+      if (ti == 0) {
+        cuda::atomic_ref<int, cuda::thread_scope_device> arrivals(late->counters[st]);
+        const int last = arrivals.fetch_add(1, cuda::memory_order_acq_rel) == KP - 1;
+        if (last) late->counters[st] = 0;
+        s_last = last;
+      }
+      sync_all();
+      if (s_last && ok) tc_add_parts(*late, st, ti);
     }
+    if (!kTma) asm volatile("cp.async.wait_all;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == kTcWarps) {
+  if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
 }
 
@@ -692,6 +853,26 @@ int gemm_kparts(int tiles, int G, int epilogue) {
   const int ST = (tiles + 7) / 8, sms = qe_sm_count();
   if (epilogue != QE_EPI_NONE || ST * 2 > sms) return 1;
   return std::max(1, std::min({sms / ST, G / 8, 16}));
+}
+
+// Tensor map over the rows of x as (64 k, rows, 64-k chunks): boxes of four chunks of 64 rows in the
+// 128-byte swizzle, rows and chunks beyond the end read as zero. False where a map cannot describe them (rows that overlap, as in an expanded row).
+bool map_rows(const qe_w4_params* p, CUtensorMap* map) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
+    return reinterpret_cast<Encode>(e == cudaSuccess && found == cudaDriverEntryPointSuccess ? fn : nullptr);
+  }();
+  if (!encode || p->ldx < p->K) return false;
+  const cuuint64_t dim[3] = {64, (cuuint64_t)p->N, (cuuint64_t)p->K / 64}, stride[2] = {(cuuint64_t)p->ldx * 2, 128};
+  const cuuint32_t box[3] = {64, 64, 4}, step[3] = {1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p->x), dim, stride, box, step,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // The opt-in limit of dynamic shared memory is a per-device, per-function setting: raised once.
@@ -754,7 +935,9 @@ extern "C" int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* str
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     if (!allowed[dev]) {
-      e = cudaFuncSetAttribute(w4_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+      e = cudaFuncSetAttribute(w4_gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(w4_gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
       if (e != cudaSuccess) return (int)e;
       allowed[dev] = true;
     }
@@ -777,7 +960,9 @@ extern "C" int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* str
     a.counters = p->counters;
     a.nctas = std::min(qe_sm_count(), ((a.tiles + 7) / 8) * a.kparts);
     const bool pdl = cfg->pdl && pdl_launch_enabled() && pdl_trigger_enabled();
-    return (int)launch(w4_gemm_tc_kernel, dim3(a.nctas), dim3(kTcThreads), kTcSmem, (cudaStream_t)stream, pdl, a);
+    CUtensorMap map{};
+    const auto kernel = map_rows(p, &map) ? w4_gemm_tc_kernel<true> : w4_gemm_tc_kernel<false>;
+    return (int)launch(kernel, dim3(a.nctas), dim3(kTcThreads), kTcSmem, (cudaStream_t)stream, pdl, a, map);
   }
   int which;
   if (p->N <= 32 && G % 4 == 0) which = 0;

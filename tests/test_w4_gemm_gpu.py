@@ -122,6 +122,38 @@ def test_odd_group_counts(api, M, K):
         check(api["gemm"](x[:N].contiguous(), p), x[:N], Wd, f"{M}x{K} N={N}")
 
 
+@pytest.mark.parametrize("M,K", [(148 * 128 * 3 + 300, 128), (148 * 128 * 4 + 77, 384), (148 * 128 * 2, 640),
+                                 (148 * 128 + 5, 29 * 128), (128, 57 * 128), (148 * 128 * 5 + 200, 128)])
+def test_walks_over_several_super_tiles(api, M, K):
+    """The tensor-memory kernel walks a CTA's super-tiles two at a time and a last odd one alone: one to
+    six super-tiles per CTA, odd and even numbers of 128-k groups, more groups than one request of
+    scales (28); rows that a tensor map describes (plain and strided) and rows that overlap, for
+    which the activations are copied by the warps: the same values give the same bits."""
+    p = api["q"](rand_w(M, K, seed=25))
+    Wd = api["deq"](p)
+    base = rand_x(1, 64 * 8 + K, seed=26)[0]
+    for x in (base.as_strided((64, K), (8, 1)), base.as_strided((17, K), (8, 1)), base[:K].expand(33, K)):
+        out, flat = (torch.empty(x.size(0), M, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        api["w4"].gemm(x, p.qw, p.scales, out, M)
+        api["w4"].gemm(x.contiguous(), p.qw, p.scales, flat, M)
+        assert torch.equal(bits(out), bits(flat))
+        check(flat, x, Wd, f"{M}x{K} N={x.size(0)}")
+
+
+@pytest.mark.parametrize("M,ldo,first", [(5120, 5121, 0), (5120, 5120 + 8, 1), (5117, 5120, 0), (200, 203, 3)])
+def test_output_rows_of_any_alignment(api, M, ldo, first):
+    """The tensor-memory kernel stores four rows at a time where the output allows it (8-byte aligned,
+    row stride a multiple of 4, four rows left), else one by one; split along K and not."""
+    p = api["q"](rand_w(M, 1024, seed=27))
+    x = rand_x(19, 1024, seed=28)
+    want = api["gemm"](x, p)
+    out = torch.full((19, ldo + first), 7.0, dtype=torch.bfloat16, device=DEV)
+    view = out.as_strided((19, M), (ldo + first, 1), first)
+    api["w4"].gemm(x, p.qw, p.scales, view, M)
+    assert torch.equal(bits(view), bits(want))
+    assert (out[:, :first] == 7).all() and (out[:, first + M:] == 7).all()
+
+
 def test_fp32_sums_and_strided_rows(api, variant):
     p = api["q"](rand_w(H, 6144, seed=31))
     Wd = api["deq"](p)
