@@ -163,6 +163,16 @@ int qe_gdn_step_n(const void* qkv, const void* z, const void* b, const void* a, 
                   const int* ctl, void* out, long ldo, int n, int Hk, int Hv, int D, float eps,
                   int q, void* stream);
 
+/* n = 8, 16 .. 64 consecutive rows of a prompt, all kept: what n / 8 calls of qe_gdn_step_n with
+ * ctl advanced by 8 rows each do (state, checkpoints of the last 8 rows, conv ring, outputs), with
+ * the state read and written once, bit for bit. ctl as for the first of those calls; the caller sets ctl[0] += n, ctl[1] = 8. No counterpart in the
+ * reference, which prefills at most 8 rows per pass. */
+int qe_gdn_prefill(const void* qkv, const void* z, const void* b, const void* a, long ldp,
+                   void* ring, const void* conv_w, const void* A_log, const void* dt_bias,
+                   const void* norm_w, float* S, float* st_k, float* st_v, float* st_g,
+                   const int* ctl, void* out, long ldo, int n, int Hk, int Hv, int D, float eps,
+                   void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Gated GQA attention for n rows at positions pos[0] + t (csrc/ops.h:25-30, csrc/attn.cu).
  * hd = head dim (64, 128 or 256; the reference fixes 256, csrc/bindings.cpp:155).
@@ -183,6 +193,16 @@ int qe_attn_prep(const void* qg, const void* k, const void* v, long ldp, const v
 int qe_attn_decode(const void* q, const void* kc, const void* vc, const int* pos, const void* qg,
                    long ldp, float* part_o, float* part_ml, void* out, long ldo, int n, int Hq,
                    int Hkv, int hd, int max_len, int NS, float scale, void* stream);
+/* The two calls above for up to 64 rows of a prompt, row for row the same bits. decode: only where NS
+ * does not select the tensor-core split kernel (hd == 256 and NS a multiple of 6: QE_ERR_ARG), whose
+ * passes are 8 rows. No counterpart in the reference. */
+int qe_attn_prep_rows(const void* qg, const void* k, const void* v, long ldp, const void* qnw,
+                      const void* knw, const float* inv_freq, const int* pos, void* q_out, void* kc,
+                      void* vc, int n, int Hq, int Hkv, int hd, int max_len, int rd, float eps,
+                      void* stream);
+int qe_attn_decode_rows(const void* q, const void* kc, const void* vc, const int* pos, const void* qg,
+                        long ldp, float* part_o, float* part_ml, void* out, long ldo, int n, int Hq,
+                        int Hkv, int hd, int max_len, int NS, float scale, void* stream);
 /* Sticky error word of the attention ring waits (0 = none, 1 producer, 2 consumer wait ran out);
  * synchronises. No counterpart in the reference. */
 int qe_attn_error(void);

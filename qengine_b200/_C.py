@@ -208,10 +208,8 @@ def force_drafts(in_tok, ctl, truth, a, k, vocab):
                               int(k), int(vocab), _stream()), "force_drafts")
 
 
-def gdn_step_n(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g, ctl, out,
-               Hk, eps, q=2):
-    """Gated DeltaNet n-row step with lazy rollback; qkv/z/b/a are row views of one projection
-    buffer. `q` is accepted for compatibility and ignored."""
+def _gdn_check(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g, ctl, out, Hk, rows, what):
+    """Everything about a DeltaNet call but the launch: (n, Hk, Hv, D, row strides of qkv and out)."""
     qn, qw, qld = _rows(qkv, BF, "qkv")
     zn, zw, zld = _rows(z, BF, "z")
     bn, bw, bld = _rows(b, BF, "b")
@@ -224,7 +222,7 @@ def gdn_step_n(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v
         _chk(t, F32, nm)
     _chk(ctl, I32, "ctl")
     n, Hv, Hk = qn, S.size(0), int(Hk)
-    _req(1 <= n <= 8 and zn == n and bn == n and an == n and on == n, "1..8 rows, equal row counts")
+    _req(n in rows and zn == n and bn == n and an == n and on == n, what + ", equal row counts")
     _req(S.dim() == 3 and S.size(1) == S.size(2) and S.size(1) in (64, 128), "dk = dv in {64, 128}")
     D = S.size(1)
     _req(Hk >= 1 and Hv % Hk == 0, "Hv must be a multiple of Hk")
@@ -235,6 +233,15 @@ def gdn_step_n(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v
     _req(st_k.numel() == 8 * Hv * D and st_v.numel() == 8 * Hv * D and st_g.numel() == 8 * Hv * 2,
          "staging buffers must hold 8 rows")
     _req(ctl.numel() >= 2, "ctl too small")
+    return n, Hk, Hv, D, qld, old
+
+
+def gdn_step_n(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g, ctl, out,
+               Hk, eps, q=2):
+    """Gated DeltaNet n-row step with lazy rollback; qkv/z/b/a are row views of one projection
+    buffer. `q` is accepted for compatibility and ignored."""
+    n, Hk, Hv, D, qld, old = _gdn_check(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g,
+                                        ctl, out, Hk, range(1, 9), "1..8 rows")
     check(lib.qe_gdn_step_n(qkv.data_ptr(), z.data_ptr(), b.data_ptr(), a.data_ptr(), qld,
                             ring.data_ptr(), conv_w.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
                             norm_w.data_ptr(), S.data_ptr(), st_k.data_ptr(), st_v.data_ptr(),
@@ -242,8 +249,19 @@ def gdn_step_n(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v
                             float(eps), int(q), _stream()), "gdn_step_n")
 
 
-def attn_prep(qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
-    """pos: int32 tensor whose element 0 is the position of row 0."""
+def gdn_prefill(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g, ctl, out, Hk, eps):
+    """What n / 8 calls of `gdn_step_n` on consecutive rows do (n = 8, 16 .. 64, all rows kept), in one
+    pass over the state, bit for bit. The last 8 rows are left pending. Not in the reference."""
+    n, Hk, Hv, D, qld, old = _gdn_check(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g,
+                                        ctl, out, Hk, range(8, 65, 8), "8, 16 .. 64 rows")
+    check(lib.qe_gdn_prefill(qkv.data_ptr(), z.data_ptr(), b.data_ptr(), a.data_ptr(), qld,
+                             ring.data_ptr(), conv_w.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
+                             norm_w.data_ptr(), S.data_ptr(), st_k.data_ptr(), st_v.data_ptr(),
+                             st_g.data_ptr(), ctl.data_ptr(), out.data_ptr(), old, n, Hk, Hv, D,
+                             float(eps), _stream()), "gdn_prefill", kernels=2)
+
+
+def _attn_prep(fn, rows, qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
     gn, gw, gld = _rows(qg, BF, "qg")
     kn, kw, kld = _rows(k, BF, "k")
     vn, vw, vld = _rows(v, BF, "v")
@@ -256,20 +274,27 @@ def attn_prep(qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
     _req(kc.dim() == 3 and kc.size(2) in (64, 128, 256), "head_dim in {64, 128, 256}")
     hd = kc.size(2)
     n, Hkv, max_len, Hq = gn, kc.size(0), kc.size(1), ow // hd
-    _req(1 <= n <= 8 and kn == n and vn == n and on == n and old == ow, "row counts / contiguous q_out")
+    _req(1 <= n <= rows and kn == n and vn == n and on == n and old == ow, "row counts / contiguous q_out")
     _req(gw == Hq * 2 * hd and kw == Hkv * hd and vw == Hkv * hd, "projection widths")
     _req(vc.shape == kc.shape and qnw.numel() == hd and knw.numel() == hd, "cache / norm shapes")
     rd = inv_freq.numel() * 2
     _req(rd <= hd, "rotary dim")
-    check(lib.qe_attn_prep(qg.data_ptr(), k.data_ptr(), v.data_ptr(), gld, qnw.data_ptr(),
-                           knw.data_ptr(), inv_freq.data_ptr(), pos.data_ptr(), q_out.data_ptr(),
-                           kc.data_ptr(), vc.data_ptr(), n, Hq, Hkv, hd, max_len, rd, float(eps),
-                           _stream()), "attn_prep")
+    check(fn(qg.data_ptr(), k.data_ptr(), v.data_ptr(), gld, qnw.data_ptr(), knw.data_ptr(), inv_freq.data_ptr(),
+             pos.data_ptr(), q_out.data_ptr(), kc.data_ptr(), vc.data_ptr(), n, Hq, Hkv, hd, max_len, rd, float(eps),
+             _stream()), "attn_prep")
 
 
-def attn_decode(q, kc, vc, pos, qg, part_o, part_ml, out):
-    """q: [n, Hq*hd] contiguous; part_o: fp32 [>=n, Hq, NS, hd]; part_ml [>=n, Hq, NS, 2];
-    out: [n, Hq*hd] (gated by sigmoid of the gate half of the qg rows)."""
+def attn_prep(qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
+    """pos: int32 tensor whose element 0 is the position of row 0."""
+    _attn_prep(lib.qe_attn_prep, 8, qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps)
+
+
+def attn_prep_rows(qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
+    """`attn_prep` for up to 64 rows (a prefill pass); same bits per row. Not in the reference."""
+    _attn_prep(lib.qe_attn_prep_rows, 64, qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps)
+
+
+def _attn_decode(fn, rows, q, kc, vc, pos, qg, part_o, part_ml, out):
     qn, qw, qld = _rows(q, BF, "q")
     gn, gw, gld = _rows(qg, BF, "qg")
     on, ow, old = _rows(out, BF, "out")
@@ -279,15 +304,27 @@ def attn_decode(q, kc, vc, pos, qg, part_o, part_ml, out):
     hd = kc.size(2)
     _chk16(q, qld, "q"); _chk16(kc, hd, "kc"); _chk16(vc, hd, "vc")
     n, Hq, Hkv, max_len = qn, qw // hd, kc.size(0), kc.size(1)
-    _req(qld == qw and gn == n and on == n and Hq % Hkv == 0, "row counts / contiguous q")
+    _req(n <= rows and qld == qw and gn == n and on == n and Hq % Hkv == 0, "row counts / contiguous q")
     _req(part_o.dim() == 4 and part_o.size(0) >= n and part_o.size(1) == Hq and part_o.size(3) == hd,
          "part_o shape")
     NS = part_o.size(2)
     _req(part_ml.numel() == part_o.size(0) * Hq * NS * 2 and ow == Hq * hd and gw == Hq * 2 * hd,
          "part_ml / out / qg shapes")
-    check(lib.qe_attn_decode(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(), qg.data_ptr(),
-                             gld, part_o.data_ptr(), part_ml.data_ptr(), out.data_ptr(), old, n, Hq,
-                             Hkv, hd, max_len, NS, float(hd) ** -0.5, _stream()), "attn_decode", kernels=2)
+    check(fn(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(), qg.data_ptr(), gld, part_o.data_ptr(),
+             part_ml.data_ptr(), out.data_ptr(), old, n, Hq, Hkv, hd, max_len, NS, float(hd) ** -0.5, _stream()),
+          "attn_decode", kernels=2)
+
+
+def attn_decode(q, kc, vc, pos, qg, part_o, part_ml, out):
+    """q: [n, Hq*hd] contiguous; part_o: fp32 [>=n, Hq, NS, hd]; part_ml [>=n, Hq, NS, 2];
+    out: [n, Hq*hd] (gated by sigmoid of the gate half of the qg rows)."""
+    _attn_decode(lib.qe_attn_decode, 8, q, kc, vc, pos, qg, part_o, part_ml, out)
+
+
+def attn_decode_rows(q, kc, vc, pos, qg, part_o, part_ml, out):
+    """`attn_decode` for up to 64 rows (a prefill pass) where the number of splits does not select the
+    tensor-core kernel (hd 256 and a multiple of 6); same bits per row. Not in the reference."""
+    _attn_decode(lib.qe_attn_decode_rows, 64, q, kc, vc, pos, qg, part_o, part_ml, out)
 
 
 def l2_persist_limit(nbytes):

@@ -73,6 +73,12 @@ SIGNATURES = {
     "qe_force_drafts": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P]),
     "qe_gdn_step_n": (c_int, [P, P, P, P, c_long, P, P, P, P, P, P, P, P, P, P, P, c_long, c_int,
                               c_int, c_int, c_int, c_float, c_int, P]),
+    "qe_gdn_prefill": (c_int, [P, P, P, P, c_long, P, P, P, P, P, P, P, P, P, P, P, c_long, c_int,
+                               c_int, c_int, c_int, c_float, P]),
+    "qe_attn_prep_rows": (c_int, [P, P, P, c_long, P, P, P, P, P, P, P, c_int, c_int, c_int, c_int,
+                                  c_int, c_int, c_float, P]),
+    "qe_attn_decode_rows": (c_int, [P, P, P, P, P, c_long, P, P, P, c_long, c_int, c_int, c_int, c_int,
+                                    c_int, c_int, c_float, P]),
     "qe_attn_prep": (c_int, [P, P, P, c_long, P, P, P, P, P, P, P, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_float, P]),
     "qe_attn_decode": (c_int, [P, P, P, P, P, c_long, P, P, P, c_long, c_int, c_int, c_int, c_int,

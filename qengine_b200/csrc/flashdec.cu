@@ -818,7 +818,15 @@ extern "C" int qe_attn_prep(const void* qg, const void* k, const void* v, long l
                             const void* knw, const float* inv_freq, const int* pos, void* q_out,
                             void* kc, void* vc, int n, int Hq, int Hkv, int hd, int max_len, int rd,
                             float eps, void* stream) {
-  if (n < 1 || n > QE_MAX_ROWS || Hq < 1 || Hkv < 1 || rd < 0 || rd > hd || (rd & 1)) return QE_ERR_ARG;
+  if (n > QE_MAX_ROWS) return QE_ERR_ARG;
+  return qe_attn_prep_rows(qg, k, v, ldp, qnw, knw, inv_freq, pos, q_out, kc, vc, n, Hq, Hkv, hd, max_len, rd, eps, stream);
+}
+
+extern "C" int qe_attn_prep_rows(const void* qg, const void* k, const void* v, long ldp, const void* qnw,
+                                 const void* knw, const float* inv_freq, const int* pos, void* q_out,
+                                 void* kc, void* vc, int n, int Hq, int Hkv, int hd, int max_len, int rd,
+                                 float eps, void* stream) {
+  if (n < 1 || n > QE_MAX_GEMM_ROWS || Hq < 1 || Hkv < 1 || rd < 0 || rd > hd || (rd & 1)) return QE_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const dim3 grid(Hq + Hkv, n);
 #define QB_PREP(HD)                                                                              \
@@ -839,11 +847,32 @@ extern "C" int qe_attn_error(void) {
   return h;
 }
 
+static int attn_decode(const void* q, const void* kc, const void* vc, const int* pos,
+                       const void* qg, long ldp, float* part_o, float* part_ml, void* out,
+                       long ldo, int n, int Hq, int Hkv, int hd, int max_len, int NS,
+                       float scale, void* stream);
+
 extern "C" int qe_attn_decode(const void* q, const void* kc, const void* vc, const int* pos,
                               const void* qg, long ldp, float* part_o, float* part_ml, void* out,
                               long ldo, int n, int Hq, int Hkv, int hd, int max_len, int NS,
                               float scale, void* stream) {
-  if (n < 1 || n > QE_MAX_ROWS || Hq < 1 || Hkv < 1 || Hq % Hkv || NS < 1 || NS > kMergeMaxSplits) return QE_ERR_ARG;
+  if (n > QE_MAX_ROWS) return QE_ERR_ARG;
+  return attn_decode(q, kc, vc, pos, qg, ldp, part_o, part_ml, out, ldo, n, Hq, Hkv, hd, max_len, NS, scale, stream);
+}
+
+extern "C" int qe_attn_decode_rows(const void* q, const void* kc, const void* vc, const int* pos,
+                                   const void* qg, long ldp, float* part_o, float* part_ml, void* out,
+                                   long ldo, int n, int Hq, int Hkv, int hd, int max_len, int NS,
+                                   float scale, void* stream) {
+  if (n > QE_MAX_GEMM_ROWS || (hd == 256 && NS % 6 == 0)) return QE_ERR_ARG;
+  return attn_decode(q, kc, vc, pos, qg, ldp, part_o, part_ml, out, ldo, n, Hq, Hkv, hd, max_len, NS, scale, stream);
+}
+
+static int attn_decode(const void* q, const void* kc, const void* vc, const int* pos,
+                       const void* qg, long ldp, float* part_o, float* part_ml, void* out,
+                       long ldo, int n, int Hq, int Hkv, int hd, int max_len, int NS,
+                       float scale, void* stream) {
+  if (n < 1 || Hq < 1 || Hkv < 1 || Hq % Hkv || NS < 1 || NS > kMergeMaxSplits) return QE_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const dim3 grid(Hq, NS, n);
   const int gq = Hq / Hkv;

@@ -754,52 +754,56 @@ class Engine:
         B.mix = buf(W, max(c.value_dim, c.hq * c.head_dim))
         B.act = buf(W, c.inter)
         B.q = buf(W, c.hq * c.head_dim)
+        B.part_o = B.part_ml = None  # partial results of the attention over all rows, where it takes them
+        if c.head_dim != 256 or self.ATTN_SPLITS % 6:
+            B.part_o = buf(W, c.hq, self.ATTN_SPLITS, c.head_dim, dt=F32)
+            B.part_ml = buf(W, c.hq, self.ATTN_SPLITS, 2, dt=F32)
         if self.has_mtp:
             B.cat, B.mh = buf(W, 2 * H), buf(W, H)
         self.wb = B
 
     def _wide_mixer(self, L, n, kv_only=False):
-        """Token mixing of a wide pass: the mixers take 8 rows, so the rows go through them in
-        sub-passes of 8, each with its own control words (position, and the 8 DeltaNet rows the
-        sub-pass before it staged). kv_only: just write K and V (a draft layer during prefill:
-        nothing else of it is kept)."""
+        """Token mixing of a wide pass. DeltaNet and the attention over caches up to 8K positions take
+        all rows in one launch; the tensor-core attention of longer caches takes 8 rows, so there the
+        rows go through in sub-passes, each with its own control words (position). kv_only: just
+        write K and V (a draft layer during prefill: nothing else of it is kept)."""
         c, B = self.cfg, self.wb
-        for j in range(n // NMAX):
-            rows = slice(j * NMAX, (j + 1) * NMAX)
-            ctl = B.ctl[j]
-            if L["type"] == "linear_attention":
-                pr = B.proj[rows, :c.gdn_proj_rows]
-                a0, a1 = c.conv_dim, c.conv_dim + c.value_dim
-                _C.gdn_step_n(pr[:, :a0], pr[:, a0:a1], pr[:, a1:a1 + c.hv], pr[:, a1 + c.hv:], L["ring"],
-                              L["conv_w"], L["A_log"], L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"],
-                              L["st_g"], ctl, B.mix[rows, :c.value_dim], c.hk, c.eps, q=self.GDN_Q)
-            else:
-                pr = B.proj[rows, :c.attn_proj_rows]
-                nq = c.hq * 2 * c.head_dim
-                nk = nq + c.hkv * c.head_dim
-                _C.attn_prep(pr[:, :nq], pr[:, nq:nk], pr[:, nk:], L["q_norm"], L["k_norm"], self.inv_freq, ctl,
-                             B.q[rows], L["kc"], L["vc"], c.eps)
-                if not kv_only:
-                    _C.attn_decode(B.q[rows], L["kc"], L["vc"], ctl, pr[:, :nq], self.part_o, self.part_ml,
-                                   B.mix[rows, :c.hq * c.head_dim])
-        width = c.value_dim if L["type"] == "linear_attention" else c.hq * c.head_dim
-        return B.mix[:n, :width]
+        if L["type"] == "linear_attention":
+            pr = B.proj[:n, :c.gdn_proj_rows]
+            a0, a1 = c.conv_dim, c.conv_dim + c.value_dim
+            out = B.mix[:n, :c.value_dim]
+            _C.gdn_prefill(pr[:, :a0], pr[:, a0:a1], pr[:, a1:a1 + c.hv], pr[:, a1 + c.hv:], L["ring"], L["conv_w"],
+                           L["A_log"], L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"], L["st_g"], self.ctl, out,
+                           c.hk, c.eps)
+            return out
+        pr = B.proj[:n, :c.attn_proj_rows]
+        nq = c.hq * 2 * c.head_dim
+        nk = nq + c.hkv * c.head_dim
+        out = B.mix[:n, :c.hq * c.head_dim]
+        _C.attn_prep_rows(pr[:, :nq], pr[:, nq:nk], pr[:, nk:], L["q_norm"], L["k_norm"], self.inv_freq, self.ctl,
+                          B.q[:n], L["kc"], L["vc"], c.eps)
+        if kv_only:
+            return out
+        if B.part_o is not None:
+            _C.attn_decode_rows(B.q[:n], L["kc"], L["vc"], self.ctl, pr[:, :nq], B.part_o, B.part_ml, out)
+        else:
+            for j in range(n // NMAX):
+                rows = slice(j * NMAX, (j + 1) * NMAX)
+                _C.attn_decode(B.q[rows], L["kc"], L["vc"], B.ctl[j], pr[rows, :nq], self.part_o, self.part_ml, out[rows])
+        return out
 
     def _wide_pass(self, n, mtp):
         """One prefill pass over n rows (a multiple of 8, at most WIDE) of wb.tok: what n / 8
         ordinary prefill passes do to the K/V caches, the DeltaNet state and the position, with
         every matrix streamed once (`_w4.gemm`). No logits: the pass that follows emits them.
         Follows python/qengine/engine.py:434-477 (layer, main) and :479-496 (draft layer) of the
-        reference with 8-row sub-passes for the mixers."""
+        reference."""
         c, B, lin, eps = self.cfg, self.wb, self.linear, self.cfg.eps
         nb = n // NMAX
         self._flush()
-        # control words of the sub-passes: positions 8 apart; every sub-pass but the first finds the
-        # 8 DeltaNet rows of the one before it pending
-        B.ctl[:nb].copy_(self.ctl.expand(nb, -1))
-        B.ctl[:nb, self.POS].add_(B.off[:nb])
-        if nb > 1:
-            B.ctl[1:nb, self.PENDING].fill_(NMAX)
+        if B.part_o is None:  # control words of the attention's sub-passes: positions 8 apart
+            B.ctl[:nb].copy_(self.ctl.expand(nb, -1))
+            B.ctl[:nb, self.POS].add_(B.off[:nb])
         h, xn, mo = B.h[:n], B.xn[:n], B.mo[:n]
 
         def mm(x, p, out):
