@@ -314,6 +314,12 @@ int qe_w4_plan_gemv(const qe_w4_params* p, const qe_w4_cfg* cfg, qe_w4_plan* pla
 int qe_w4_auto_ksplit(int Mp, int Kp, int N, int warps);
 /* Replaces launch_gemv_w4 (gemv_w4.h:56). */
 int qe_w4_gemv(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream);
+/* qe_w4_plan_gemv and qe_w4_gemv with default options in one call, arguments instead of structs: bf16
+ * in and out. ws / counters as in qe_w4_params with their sizes; QE_ERR_SCRATCH when the plan needs
+ * more (nothing is launched). No counterpart in the reference. */
+int qe_w4_gemv_call(const void* qw, const void* scales, const void* x, void* out, float* ws,
+                    long ws_floats, int* counters, long n_counters, int M, int K, int Mp, int Kp, int N,
+                    long ldx, long ldo, int epilogue, void* stream);
 /* qe_w4_gemv with the fused prologue described at qe_w4_norm (nrm may be NULL). */
 int qe_w4_gemv_ex(const qe_w4_params* p, const qe_w4_norm* nrm, const qe_w4_cfg* cfg, void* stream);
 /* The prologue of qe_w4_gemv_ex as a launch of its own: xn_out[r] = RMSNorm1p(h_in[r] + delta[r]) *

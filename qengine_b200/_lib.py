@@ -94,6 +94,8 @@ SIGNATURES = {
     "qe_w4_plan_gemv": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), C.POINTER(W4Plan)]),
     "qe_w4_auto_ksplit": (c_int, [c_int, c_int, c_int, c_int]),
     "qe_w4_gemv": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), P]),
+    "qe_w4_gemv_call": (c_int, [P, P, P, P, P, c_long, P, c_long, c_int, c_int, c_int, c_int, c_int, c_long, c_long,
+                                c_int, P]),
     "qe_w4_gemv_ex": (c_int, [C.POINTER(W4Params), C.POINTER(W4Norm), C.POINTER(W4Cfg), P]),
     "qe_w4_norm_rows": (c_int, [C.POINTER(W4Norm), c_int, c_int, C.POINTER(W4Cfg), P]),
     "qe_w4_gemv_chain": (c_int, [C.POINTER(C.POINTER(W4Params)), C.POINTER(C.POINTER(W4Norm)), c_int,

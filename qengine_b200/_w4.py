@@ -215,18 +215,54 @@ def gemv_chain(jobs, warps=0, unroll=0, ksplit=0, pdl=True, variant=0, mode=-1, 
     _launch(jobs, _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units), "gemv_w4 chain")
 
 
+_DEFAULTS = (0, 0, 0, True, 0, -1, 0, 4)
+
+
+def _call(x, qw, scales, out, M, epilogue, opts):
+    """One GEMV called by itself. What `job` checks, in one expression over plain numbers, then plan and
+    launch in one library call: for a small matrix the call is all the time there is (18 us through
+    `job` and `_launch` on the host of a B200). Whatever does not pass goes through those, which know
+    what to complain about."""
+    T = torch.Tensor
+    if type(x) is T and type(qw) is T and type(scales) is T and type(out) is T and opts == _DEFAULTS:
+        xs, qs, ss, os = x.shape, qw.shape, scales.shape, out.shape
+        if len(xs) == 2 and len(os) == 2 and len(qs) == 4 and len(ss) == 3:
+            N, K = xs
+            Mp, Kp = qs[0] * 16, qs[1] * 64
+            ldx, kx = x.stride()
+            ldo, ko = out.stride()
+            rows = Mp // 2 - 8 < M <= Mp // 2 if epilogue else Mp - 16 < M <= Mp
+            xp, qp, sp, op = x.data_ptr(), qw.data_ptr(), scales.data_ptr(), out.data_ptr()
+            bf, dev = torch.bfloat16, x.get_device()
+            W = _per_device.get(dev)
+            if (x.is_cuda and qw.is_cuda and scales.is_cuda and out.is_cuda and x.dtype is bf and out.dtype is bf and
+                    qw.dtype is torch.int32 and scales.dtype is torch.float16 and type(M) is int and 1 <= N <= 8 and
+                    os[0] == N and os[1] == M and rows and Kp - 128 < K <= Kp and kx == 1 and ko == 1 and
+                    qs[2] == 32 and qs[3] == 4 and ss[2] == 16 and ss[0] == qs[0] and ss[1] * 128 == Kp and
+                    (qp | sp) % 16 == 0 and xp != op and qw.is_contiguous() and scales.is_contiguous() and
+                    W is not None and W.ws is not None and W.counters is not None):
+                stream = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+                code = lib.qe_w4_gemv_call(qp, sp, xp, op, W.ws.data_ptr(), W.ws.numel(), W.counters.data_ptr(),
+                                           W.counters.numel(), M, K, Mp, Kp, N, ldx, ldo, epilogue, stream)
+                if code == 0:
+                    launches[0] += 1
+                    return
+                if code != -28:  # anything but scratch that has to grow
+                    _req(code != -22, "gemv_w4: argument combination not supported by the kernel")
+                    _req(False, f"gemv_w4 launch failed: CUDA error {code}")
+    _launch([job(x, qw, scales, out, M, swiglu=epilogue == EPI_SWIGLU)], _cfg(*opts), "gemv_w4")
+
+
 def gemv(x, qw, scales, out, M, warps=0, unroll=0, ksplit=0, pdl=True, variant=0, mode=-1,
          blocks_per_sm=0, min_units=4):
     """out[N, M] = x[N, K] @ W~^T (W packed by quant.quantize_w4)."""
-    _launch([job(x, qw, scales, out, M)],
-            _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units), "gemv_w4")
+    _call(x, qw, scales, out, M, EPI_NONE, (warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units))
 
 
 def gemv_swiglu(x, qw, scales, out, I, warps=0, unroll=0, ksplit=0, pdl=True, variant=0, mode=-1,
                 blocks_per_sm=0, min_units=4):
     """out[N, I] = silu(x @ Wg^T) * (x @ Wu^T) (packed by quant.quantize_w4_gate_up)."""
-    _launch([job(x, qw, scales, out, I, swiglu=True)],
-            _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units), "gemv_w4")
+    _call(x, qw, scales, out, I, EPI_SWIGLU, (warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units))
 
 
 def gemv_partial(x, qw, scales, out32, M, warps=0, unroll=0, ksplit=0, pdl=True, variant=0, mode=-1,

@@ -944,6 +944,19 @@ extern "C" int qe_w4_gemv(const qe_w4_params* p, const qe_w4_cfg* cfg, void* str
   return launch_chain(&p, nullptr, 1, cfg, nullptr, (cudaStream_t)stream);
 }
 
+extern "C" int qe_w4_gemv_call(const void* qw, const void* scales, const void* x, void* out, float* ws,
+                               long ws_floats, int* counters, long n_counters, int M, int K, int Mp, int Kp, int N,
+                               long ldx, long ldo, int epilogue, void* stream) {
+  qe_w4_params p{qw, scales, x, out, ws, counters, M, K, Mp, Kp, N, ldx, ldo, epilogue, 0, 0};
+  qe_w4_cfg cfg;
+  qe_w4_cfg_default(&cfg);
+  qe_w4_plan plan;
+  const int e = qe_w4_plan_gemv(&p, &cfg, &plan);
+  if (e) return e;
+  if (plan.ws_floats > ws_floats || plan.counters > n_counters) return QE_ERR_SCRATCH;
+  return qe_w4_gemv(&p, &cfg, stream);
+}
+
 extern "C" int qe_w4_gemv_ex(const qe_w4_params* p, const qe_w4_norm* nrm, const qe_w4_cfg* cfg, void* stream) {
   return launch_chain(&p, &nrm, 1, cfg, nullptr, (cudaStream_t)stream);
 }
