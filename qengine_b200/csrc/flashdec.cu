@@ -799,6 +799,36 @@ attn_merge_kernel(const float* part_o, const float* part_ml, const bf16* qg, lon
   }
 }
 
+// The same for at most 16 splits (caches up to 8K positions): there every warp of the kernel above has one
+// split at most, so a thread per output dim that adds the splits in ascending order gives the same
+// bits, with all loads in flight at once, no shared memory and no barrier.
+constexpr int kMergeSmall = 16;
+template <int HD>
+__global__ void __launch_bounds__(HD)
+attn_merge_small_kernel(const float* part_o, const float* part_ml, const bf16* qg, long ldp, bf16* out, long ldo,
+                        int Hq, int NS) {
+  dep_release();
+  dep_wait();
+  const int h = blockIdx.x, t = blockIdx.y, c = threadIdx.x, lane = c & 31;
+  const size_t base = ((size_t)t * Hq + h) * NS;
+  float v[kMergeSmall];
+#pragma unroll
+  for (int s = 0; s < kMergeSmall; ++s) v[s] = s < NS ? part_o[(base + s) * HD + c] : 0.f;
+  const float gate = tofloat(qg[(long)t * ldp + (size_t)h * 2 * HD + HD + c]);
+  const float2 ml = lane < NS ? reinterpret_cast<const float2*>(part_ml)[base + lane] : make_float2(-INFINITY, 0.f);
+  float M = ml.x;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  const float f = ml.x == -INFINITY ? 0.f : expf(ml.x - M);
+  const float L = warp_allsum(lane < NS ? ml.y * f : 0.f);
+  float O = 0.f;
+#pragma unroll
+  for (int s = 0; s < kMergeSmall; ++s)
+    if (s < NS) O += fmaf(v[s], __shfl_sync(0xffffffffu, f, s), 0.f);
+  const float ob = rnd(O / L);
+  out[(long)t * ldo + (size_t)h * HD + c] = tobf16(ob * rnd(sigmoid_acc(gate)));
+}
+
 inline bool pdl_on() { return pdl_launch_enabled() && pdl_trigger_enabled(); }
 
 template <int HD, int GQ>
@@ -892,6 +922,10 @@ static int attn_decode(const void* q, const void* kc, const void* vc, const int*
                       (const bf16*)q, (const bf16*)kc, (const bf16*)vc, pos, part_o, part_ml,     \
                       Hq, Hkv, max_len, scale);                                                   \
     if (e) return e;                                                                              \
+    if (NS <= kMergeSmall)                                                                        \
+      return (int)launch(attn_merge_small_kernel<HD>, dim3(Hq, n), dim3(HD), 0, s, pdl_on(),      \
+                         (const float*)part_o, (const float*)part_ml, (const bf16*)qg, ldp,       \
+                         (bf16*)out, ldo, Hq, NS);                                                \
     return (int)launch(attn_merge_kernel<HD>, dim3(Hq, n), dim3(kMergeWarps * 32), 0, s, pdl_on(), \
                        (const float*)part_o, (const float*)part_ml, (const bf16*)qg, ldp,         \
                        (bf16*)out, ldo, Hq, NS, pos, max_len, 0);                                 \
