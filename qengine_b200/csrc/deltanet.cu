@@ -367,7 +367,6 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gdn_prefill_kernel(const GdnAr
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
 
-  cluster.barrier_arrive();  // waited for before the first store into another CTA's shared memory
   const int j = blockIdx.y, cs = blockIdx.x, c0 = cs * kCols;
   const int rep = a.Hv / a.Hk, i_qk = j / rep;
   const int C = 2 * a.Hk * D + a.Hv * D;
@@ -445,26 +444,36 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gdn_prefill_kernel(const GdnAr
   if (lane < 2) sh.gate[warp][lane] = a.st_g[(warp * a.Hv + j) * 2 + lane];
   __syncthreads();
   for (int t = 0; t < pend; ++t) row_update(t, false);
-  __syncthreads();  // k, v, gate are about to be overwritten
+  cluster.sync();  // k, v, gate are about to be overwritten, k and q by the other CTAs, too
 
-  // ---- causal convolution + SiLU: tasks of 32 channels x 8 rows (q and k: all D channels of the
-  // head's q/k head; v: own columns), dealt out over the warps, each one's loads in flight together ----
-  const int tasks = (2 * D + kCols) / 32 * (n / 8);
-  for (int task = warp; task < tasks; task += kWarps) {
-    const int cb = task / (n / 8), t0 = (task - cb * (n / 8)) * 8;
-    const int idx = cb * 32 + lane;
+  // ---- causal convolution + SiLU: tasks of 32 channels x 8 rows, dealt out over the warps, a task's
+  // loads in flight together. v: own columns, all rows. q and k are the same in all CTAs of the
+  // cluster: each takes every NCTA-th block of 8 rows and hands the normalised rows to the others ----
+  constexpr int kQk = 2 * D / 32;
+  const int nb = n / 8, mine = (nb - cs + NCTA - 1) / NCTA;
+  for (int task = warp; task < kQk * mine + nb; task += kWarps) {
+    const bool is_v = task >= kQk * mine;
+    const int idx = is_v ? 2 * D + lane : task % kQk * 32 + lane;
+    const int t0 = 8 * (is_v ? task - kQk * mine : cs + task / kQk * NCTA);
     const int part_id = idx < D ? 0 : idx < 2 * D ? 1 : 2;
     const int c = part_id == 0 ? idx : part_id == 1 ? idx - D : idx - 2 * D;
     const int ch = part_id == 0 ? i_qk * D + c : part_id == 1 ? a.Hk * D + i_qk * D + c : 2 * a.Hk * D + j * D + c0 + c;
-    float x[11], w[4];
+    const bf16* src = a.qkv + (long)t0 * a.ldp + ch;
+    bf16 raw[11];
 #pragma unroll
-    for (int u = 0; u < 11; ++u) {
-      const int t = t0 - 3 + u, p = P + t;
-      x[u] = t >= 0 ? tofloat(a.qkv[(long)t * a.ldp + ch])
-                    : p >= 0 ? tofloat(a.ring[(size_t)(p & (kRing - 1)) * C + ch]) : 0.f;
+    for (int u = 0; u < 3; ++u) {  // the three rows before: of this pass, or from the ring
+      const int p = P + t0 - 3 + u;
+      const bf16* from = t0 ? src + (long)(u - 3) * a.ldp : a.ring + (size_t)(p & (kRing - 1)) * C + ch;
+      raw[u] = *from;
+      if (p < 0) raw[u] = tobf16(0.f);
     }
 #pragma unroll
+    for (int u = 3; u < 11; ++u) raw[u] = src[(long)(u - 3) * a.ldp];
+    float x[11], w[4];
+#pragma unroll
     for (int u = 0; u < 4; ++u) w[u] = tofloat(a.conv_w[ch * 4 + u]);
+#pragma unroll
+    for (int u = 0; u < 11; ++u) x[u] = tofloat(raw[u]);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       float acc = w[0] * x[u];
@@ -486,8 +495,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gdn_prefill_kernel(const GdnAr
   }
   __syncthreads();
 
-  // ---- l2norm of q and k of every row and k . q: one warp per row ----
-  for (int t = warp; t < n; t += kWarps) {
+  // ---- l2norm of q and k and k . q of this CTA's rows, one warp per row, into all CTAs ----
+  for (int u8 = warp; u8 < 8 * mine; u8 += kWarps) {
+    const int t = 8 * (cs + u8 / 8 * NCTA) + (u8 & 7);
     float eq[NI], ek[NI], sq = 0.f, sk = 0.f;
 #pragma unroll
     for (int u = 0; u < NI; ++u) {
@@ -505,15 +515,28 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gdn_prefill_kernel(const GdnAr
     float dot = 0.f;
 #pragma unroll
     for (int u = 0; u < NI; ++u) {
-      const float qn = (eq[u] * iq) / sqrtf((float)D), kn = ek[u] * ik;
-      sh.q[t][Shared::at(lane + 32 * u)] = qn;
-      sh.k[t][Shared::at(lane + 32 * u)] = kn;
-      dot = fmaf(qn, kn, dot);
+      eq[u] = (eq[u] * iq) / sqrtf((float)D), ek[u] = ek[u] * ik;
+      dot = fmaf(eq[u], ek[u], dot);
     }
     dot = warp_allsum(dot);
-    if (lane == 0) sh.kq[t] = dot;
+#pragma unroll
+    for (int rk = 0; rk < NCTA; ++rk) {
+      Shared& to = *cluster.map_shared_rank(&sh, rk);
+#pragma unroll
+      for (int u = 0; u < NI; ++u) {
+        to.q[t][Shared::at(lane + 32 * u)] = eq[u];
+        to.k[t][Shared::at(lane + 32 * u)] = ek[u];
+      }
+      if (lane == 0) to.kq[t] = dot;
+    }
   }
-  __syncthreads();
+  // gate inputs of this warp's rows, needed at the very end
+  constexpr int kRowsPerWarp = kWideRows / kWarps;
+  float zz[kRowsPerWarp];
+#pragma unroll
+  for (int u = 0; u < kRowsPerWarp; ++u)
+    zz[u] = warp + kWarps * u < n ? tofloat(a.z[(long)(warp + kWarps * u) * a.ldp + j * D + c0 + lane]) : 0.f;
+  cluster.sync();
 
   // ---- the recurrence; S is written as it stands before the last 8 rows, which stay pending ----
   for (int t = 0; t < n; ++t) {
@@ -524,22 +547,26 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gdn_prefill_kernel(const GdnAr
   __syncthreads();
 
   // ---- gated RMSNorm over the head's D outputs, as in the step kernel ----
-  cluster.barrier_wait();
-  for (int t = warp; t < n; t += kWarps) {
-    const float ob = sh.o[t][lane];
-    const float ssum = warp_allsum(ob * ob);
-    if (lane < NCTA) *cluster.map_shared_rank(&sh.ss[cs][t], lane) = ssum;
+  float ob[kRowsPerWarp];
+#pragma unroll
+  for (int u = 0; u < kRowsPerWarp; ++u) {
+    const int t = warp + kWarps * u;
+    ob[u] = t < n ? sh.o[t][lane] : 0.f;
+    const float ssum = warp_allsum(ob[u] * ob[u]);
+    if (t < n && lane < NCTA) *cluster.map_shared_rank(&sh.ss[cs][t], lane) = ssum;
   }
-  cluster.sync();
   const float nw = tofloat(a.norm_w[c0 + lane]);
-  for (int t = warp; t < n; t += kWarps) {
+  cluster.sync();
+#pragma unroll
+  for (int u = 0; u < kRowsPerWarp; ++u) {
+    const int t = warp + kWarps * u;
+    if (t >= n) break;
     float total = 0.f;
 #pragma unroll
     for (int rk = 0; rk < NCTA; ++rk) total += sh.ss[rk][t];
-    const float nn = rnd(sh.o[t][lane] * rsqrtf(total / (float)D + a.eps));
+    const float nn = rnd(ob[u] * rsqrtf(total / (float)D + a.eps));
     const float y = rnd(nw * nn);
-    const float zz = tofloat(a.z[(long)t * a.ldp + j * D + c0 + lane]);
-    a.out[(long)t * a.ldo + j * D + c0 + lane] = tobf16(y * silu_acc(zz));
+    a.out[(long)t * a.ldo + j * D + c0 + lane] = tobf16(y * silu_acc(zz[u]));
   }
   // ---- checkpoints of the last 8 rows; the cluster barrier lies between them and the replay of the
   // CTAs that read the old ones ----
