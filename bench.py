@@ -617,7 +617,7 @@ def run_ours(a):
         prefill.update(prompt_tokens=a.prefill_tokens, speedup=prefill["rows64"]["tok_s"] / prefill["rows8"]["tok_s"],
                        first_token_equal=firsts["rows8"] == firsts["rows64"],
                        what="host feed + graph replays of a whole prompt; rows64 = passes of 64 rows through "
-                            "qe_w4_gemm (tcgen05), the mixers in sub-passes of 8 rows")
+                            "qe_w4_gemm (tcgen05), the mixers in one launch per layer")
         del eng_f
         gc.collect()
         torch.cuda.empty_cache()
