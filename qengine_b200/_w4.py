@@ -38,6 +38,11 @@ class _Workspace:
 _per_device: dict[int, _Workspace] = {}
 
 
+def _stream() -> int:
+    """The current stream of the current device, without building a Stream object."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _req(cond, msg):
     if not cond:
         raise RuntimeError(msg)
@@ -112,7 +117,7 @@ def _launch(jobs, cfg, what):
     W = _workspace(dev, ws_floats, counters)
     for j in jobs:
         j.p.ws, j.p.counters = W.ws.data_ptr(), W.counters.data_ptr()
-    stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream()
     n = len(jobs)
     if n == 1 and jobs[0].nrm is None:
         code = lib.qe_w4_gemv(C.byref(jobs[0].p), C.byref(cfg), stream)
@@ -241,9 +246,8 @@ def _call(x, qw, scales, out, M, epilogue, opts):
                     qs[2] == 32 and qs[3] == 4 and ss[2] == 16 and ss[0] == qs[0] and ss[1] * 128 == Kp and
                     (qp | sp) % 16 == 0 and xp != op and qw.is_contiguous() and scales.is_contiguous() and
                     W is not None and W.ws is not None and W.counters is not None):
-                stream = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
                 code = lib.qe_w4_gemv_call(qp, sp, xp, op, W.ws.data_ptr(), W.ws.numel(), W.counters.data_ptr(),
-                                           W.counters.numel(), M, K, Mp, Kp, N, ldx, ldo, epilogue, stream)
+                                           W.counters.numel(), M, K, Mp, Kp, N, ldx, ldo, epilogue, _stream())
                 if code == 0:
                     launches[0] += 1
                     return
@@ -321,7 +325,7 @@ def norm_rows(h_in, delta, norm_w, eps, xn_out, h_out=None, tok=None, xn16_out=N
              xn16_out.stride(1) == 1, "xn16_out fp16 [N, K]")
         nrm.xn16_out, nrm.ldx16 = xn16_out.data_ptr(), xn16_out.stride(0)
     cfg = _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units)
-    check(lib.qe_w4_norm_rows(C.byref(nrm), N, K, C.byref(cfg), torch.cuda.current_stream().cuda_stream), "norm_rows")
+    check(lib.qe_w4_norm_rows(C.byref(nrm), N, K, C.byref(cfg), _stream()), "norm_rows")
 
 
 MAX_GEMM_ROWS = 64
@@ -363,7 +367,7 @@ def gemm(x, qw, scales, out, M, swiglu=False, pdl=True, variant=0):
                  torch.zeros(max(plan.counters, 1 << 10), dtype=torch.int32, device=x.device), W)  # old ones stay alive
             _gemm_scratch[dev] = W
         p.ws, p.counters = W[0].data_ptr(), W[1].data_ptr()
-    code = lib.qe_w4_gemm(C.byref(p), C.byref(cfg), torch.cuda.current_stream().cuda_stream)
+    code = lib.qe_w4_gemm(C.byref(p), C.byref(cfg), _stream())
     _req(code != -22, "gemm: argument combination not supported by the kernel")
     _req(code == 0, f"gemm launch failed: CUDA error {code}")
     launches[0] += 1
@@ -406,7 +410,7 @@ def gemv_static(x, qw, scales, out, M, swiglu=False, warps=0, unroll=0, ksplit=0
     p = W4Params(qw.data_ptr(), scales.data_ptr(), x.data_ptr(), out.data_ptr(), None, None, M, K, Mp, Kp, N,
                  x.stride(0), out.stride(0), EPI_SWIGLU if swiglu else EPI_NONE, 0, 0)
     cfg = W4Cfg(int(warps), int(unroll), int(ksplit), 0, int(variant), int(mode), int(blocks_per_sm), int(min_units))
-    code = lib.qe_w4_gemv_static(C.byref(p), C.byref(cfg), torch.cuda.current_stream().cuda_stream)
+    code = lib.qe_w4_gemv_static(C.byref(p), C.byref(cfg), _stream())
     _req(code != -28, "gemv_static: this shape needs more scratch than the library's fixed array "
                       "(1 Mi partial-sum floats, 16 Ki tile counters); use gemv with caller scratch")
     _req(code == 0, f"gemv_static failed: error {code}")
