@@ -122,55 +122,48 @@ rmsnorm1p_any_kernel(bf16* x, const bf16* delta,
 // gemv_bf16_kernel (reference csrc/basic.cu:99-155). A lane always walks k in the same order
 // whatever NR and WR are, so neither shows in the result.
 // Bound by HBM (2 bytes per weight) for one row; with more rows by issue slots, since every 16 bytes of
-// weights cost the load and the widening of NR x 16 bytes of activations and 8 NR multiply-adds. Two
-// weight rows per warp share the activations, the multiply-adds are done in pairs (even and odd k) and
-// weights leave no L1 lines. 62,080 x 5,120, us before (one row per warp) -> now: 1 row 90 -> 89, 3 rows
-// 143 -> 101 (6.3 TB/s), 5 rows 170 -> 130, 8 rows 270 -> 197. Four rows per warp: the same at this size,
-// 36 % slower at 1,000 rows x 3; one row per warp with pairs: 3 rows 106, 8 rows 265.
+// weights cost the load and the widening of NR x 16 bytes of activations. Two weight rows per warp share
+// them, and weights leave no L1 lines. 62,080 x 5,120, us before (one row per warp) -> now:
+// 1 row 90 -> 90, 3 rows 121 -> 99 (6.4 TB/s; 137 -> 102 called on its own), 5 rows 170 -> 134, 8 rows 270 -> 206.
+// Four rows per warp: the same at this size, 20 % slower at 1,000 rows x 3. Multiply-adds in pairs (even
+// and odd k, fma.rn.f32x2) take another 4 % (3 rows) to 12 % (8 rows) off, but the second accumulator costs
+// a single row 2 to 9 % where K is some hundreds, and rows must not depend on how many there are.
 // ---------------------------------------------------------------------------------------------
-constexpr int kGemvWarps = 4;
+constexpr int kGemvRows = 8;  // weight rows per block: fewer make short rows (K of some hundreds) pay for the blocks
 
 __device__ __forceinline__ uint4 ld_once(const uint4* p) {  // constant and read once: no L1 line, x stays there
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 
-// c += (a0, a1) * (b0, b1): two fp32 fused multiply-adds in one instruction.
-__device__ __forceinline__ void fma2(float2& c, float a0, float a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
-      "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
-      : "+f"(c.x), "+f"(c.y) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-
 template <int NR, int WR>
-__global__ void __launch_bounds__(kGemvWarps * 32)
+__global__ void __launch_bounds__(kGemvRows / WR * 32)
 gemv_bf16_rows_kernel(const bf16* W, const bf16* x,
                       bf16* out, int N, int K, long ldx, long ldo) {
   constexpr int U = 4;  // packets of a row in flight
   dep_release();
   const int lane = threadIdx.x & 31;
-  const int j = (blockIdx.x * kGemvWarps + (threadIdx.x >> 5)) * WR;
+  const int j = blockIdx.x * kGemvRows + (threadIdx.x >> 5) * WR;
   if (j >= N) { dep_wait(); return; }
   const int npk = K >> 3;
   const uint4* wr[WR];  // rows beyond the last one repeat it and are not stored
 #pragma unroll
-  for (int i = 0; i < WR; ++i) wr[i] = reinterpret_cast<const uint4*>(W + (size_t)min(j + i, N - 1) * K);
-  float2 acc[WR][NR];  // sums over the even and the odd k of the lane
+  for (int i = 0; i < WR; ++i) wr[i] = reinterpret_cast<const uint4*>(W + (size_t)(WR == 1 ? j : min(j + i, N - 1)) * K);
+  float acc[WR][NR];
 #pragma unroll
   for (int i = 0; i < WR; ++i)
 #pragma unroll
-    for (int r = 0; r < NR; ++r) acc[i][r] = make_float2(0.f, 0.f);
+    for (int r = 0; r < NR; ++r) acc[i][r] = 0.f;
   bool waited = false;
-#pragma unroll 1
   for (int p0 = lane; p0 < npk; p0 += 32 * U) {
     uint4 wq[U][WR];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int i = 0; i < WR; ++i)
-        if (p0 + 32 * u < npk) wq[u][i] = ld_once(wr[i] + p0 + 32 * u);
+        if (p0 + 32 * u < npk) wq[u][i] = NR == 1 ? __ldg(wr[i] + p0 + 32 * u) : ld_once(wr[i] + p0 + 32 * u);
     if (!waited) { dep_wait(); waited = true; }  // weights are constants; x is produced upstream
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -183,9 +176,9 @@ gemv_bf16_rows_kernel(const bf16* W, const bf16* x,
           float xf[8];
           widen8(reinterpret_cast<const uint4*>(x + (long)r * ldx)[p0 + 32 * u], xf);
 #pragma unroll
-          for (int e = 0; e < 8; e += 2)
+          for (int e = 0; e < 8; ++e)
 #pragma unroll
-            for (int i = 0; i < WR; ++i) fma2(acc[i][r], wf[i][e], wf[i][e + 1], xf[e], xf[e + 1]);
+            for (int i = 0; i < WR; ++i) acc[i][r] = fmaf(wf[i][e], xf[e], acc[i][r]);
         }
       }
     }
@@ -195,7 +188,7 @@ gemv_bf16_rows_kernel(const bf16* W, const bf16* x,
   for (int i = 0; i < WR; ++i) {
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-      const float s = warp_allsum(acc[i][r].x + acc[i][r].y);
+      const float s = warp_allsum(acc[i][r]);
       if (lane == 0 && j + i < N) out[(long)r * ldo + j + i] = tobf16(s);
     }
   }
@@ -362,15 +355,17 @@ extern "C" int qe_gemv_bf16(const void* W, const void* x, void* out, int nr, int
                             long ldo, void* stream) {
   if (nr < 1 || nr > QE_MAX_ROWS || K % 8 || N < 1) return QE_ERR_ARG;
   if (!aligned16(W) || !aligned16(x) || ldx % 8) return QE_ERR_ARG;
-  // one weight row per warp for a single activation row (nothing to share), two for more
-  const int per_block = kGemvWarps * (nr == 1 ? 1 : 2);
-  const dim3 grid((N + per_block - 1) / per_block), block(kGemvWarps * 32);
+  // One weight row per warp for a single activation row (nothing to share), and for up to four where half
+  // the warps would not fill the chip (one against two rows per warp, us: 3,000 x 4,096, 4 rows 11.9 / 14.1;
+  // 20,000 x 2,000 24.3 / 20.9).
+  const int wr = nr == 1 || (nr <= 4 && N < 8192) ? 1 : 2;
+  const dim3 grid((N + kGemvRows - 1) / kGemvRows), block(kGemvRows / wr * 32);
   cudaStream_t s = (cudaStream_t)stream;
   const bf16 *w = (const bf16*)W, *xx = (const bf16*)x;
   bf16* o = (bf16*)out;
   switch (nr) {
 #define QB_ROWS(R) \
-  case R: return (int)launch(gemv_bf16_rows_kernel<R, R == 1 ? 1 : 2>, grid, block, 0, s, pdl_on(), w, xx, o, N, K, ldx, ldo);
+  case R: return (int)launch(wr == 1 ? gemv_bf16_rows_kernel<R, R <= 4 ? 1 : 2> : gemv_bf16_rows_kernel<R, R == 1 ? 1 : 2>, grid, block, 0, s, pdl_on(), w, xx, o, N, K, ldx, ldo);
     QB_ROWS(1) QB_ROWS(2) QB_ROWS(3) QB_ROWS(4) QB_ROWS(5) QB_ROWS(6) QB_ROWS(7) QB_ROWS(8)
 #undef QB_ROWS
   }
