@@ -376,6 +376,10 @@ int qe_w4_gemv_static(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream)
 #define QE_MAX_GEMM_ROWS 64
 int qe_w4_plan_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, qe_w4_plan* plan);
 int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream);
+/* qe_w4_gemm whose default kernel gives a wait up after wait_limit polls of its barrier instead of the
+ * usual 2^20: out is then incomplete, qe_w4_ring_error reports it, and everything else is usable as
+ * before. For callers that want to hear of a stalled GPU sooner, and for testing that way out. */
+int qe_w4_gemm_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wait_limit, void* stream);
 
 /* Packs W [M, K] (row stride ld0; dtype 0 bf16, 1 fp16, 2 fp32) into the wire format on the GPU: qw
  * int32 [Mp/16, Kp/64, 32, 4] (16-byte aligned), scales fp16 [Mp/16, Kp/128, 16]. With w1 != NULL w0 / w1

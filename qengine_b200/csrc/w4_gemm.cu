@@ -32,8 +32,10 @@
 // atomics, results are bit-identical run to run.
 //
 // Every mbarrier wait of both kernels is bounded; on expiry the warp records the error word
-// (reported by qe_w4_ring_error), stops working, keeps arriving where others wait for it, and the
-// CTA frees its tensor memory and leaves.
+// (reported by qe_w4_ring_error), requests nothing more and waits, bounded as well, for the copies and
+// products it still has in flight. In w4_gemm_kernel the other warps stop at their next wait for it; the
+// warps of w4_gemm_tc_kernel each run into their own limit at the latest. Then the CTA frees its tensor
+// memory and leaves.
 #include <cuda.h>  // CUtensorMap (types only: the encoder is looked up at run time)
 
 #include <cuda/atomic>
@@ -58,6 +60,7 @@ struct GemmArgs {
   int kparts;      // tensor-memory kernel: parts of K a super-tile is split into
   float* ws;       // ... their fp32 sums, [super-tile][part][64][128]
   int* counters;   // ... and one arrival counter per super-tile, zero between launches
+  int wait_limit;  // tensor-memory kernel: polls after which a wait gives up
 };
 
 __device__ int g_gemm_error = 0;
@@ -65,8 +68,8 @@ __device__ int g_gemm_error = 0;
 constexpr int kGemmWaitLimit = 1 << 20;
 
 // A bounded wait whose verdict is the same in every lane of the (converged) warp.
-__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity) {
-  return __all_sync(0xffffffffu, bar_wait(b, parity, kGemmWaitLimit));
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, int limit = kGemmWaitLimit) {
+  return __all_sync(0xffffffffu, bar_wait(b, parity, limit));
 }
 __device__ __forceinline__ void bar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sa(b)) : "memory");
@@ -568,7 +571,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((128u >> 4) << 24);
     const uint64_t db0 = tc_desc(sa(Bbase));
     if (elect_one()) {
-      int v = 0, z = 0;
+      int v = 0, z = 0;  // micro-steps issued, step
       bool ok = true;
 #pragma unroll 1
       for (int j = 0; j < nj && ok; j += 2) {
@@ -577,15 +580,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int i = 0; i < per_job && ok; ++i, ++z) {
           const uint64_t db = db0 + (uint64_t)((z & (kTcB - 1)) * (kTcBStage >> 4));
           if (!(i & 1)) {
-            ok = bar_wait(&b_full[(z >> 1) & (kTcB / 2 - 1)], (z / kTcB) & 1, kGemmWaitLimit);
+            ok = bar_wait(&b_full[(z >> 1) & (kTcB / 2 - 1)], (z / kTcB) & 1, a.wait_limit);
             // Copies made by other threads: the fence that shows them to the tensor core is here because
             // it waits for its thread's own outstanding memory operations, of which this one has none.
             if (!kTma) async_proxy_fence();
           }
 #pragma unroll 1
-          for (int h = 0; h < (pair ? 2 : 1) && ok; ++h, ++v) {
+          for (int h = 0; h < (pair ? 2 : 1) && ok; ++h) {
             const int s = v & 3;
-            ok = bar_wait(&ready[s], (v >> 2) & 1, kGemmWaitLimit);
+            ok = bar_wait(&ready[s], (v >> 2) & 1, a.wait_limit);
             tc_fence_after();
             const uint32_t d = tmem + s * 64, ac = tmem + kTcACol + s * 64;
             if (ok) {
@@ -593,12 +596,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
               for (int k = 0; k < 8; ++k)
                 tc_mma(d, ac + 8 * k, db + (uint64_t)((k >> 2) * (8192 >> 4) + (k & 3) * 2), idesc, k ? 1u : 0u);
               tc_commit(&d_full[s]);
+              ++v;
             }
           }
         }
         if (per_job & 1) ++z;
       }
       if (!ok) atomicExch(&g_gemm_error, 2);
+      // The products in flight, which drain warps that gave up have not waited for.
+      if (v > 0) bar_wait(&d_full[(v - 1) & 3], ((v - 1) >> 2) & 1, kGemmWaitLimit);
     }
     __syncwarp();
   } else if (warp > 8) {
@@ -611,7 +617,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int i = 0; i < kTcAhead; ++i) {
         const int v = v0 + 2 * i, s = v & 3;
         if (v >= V || !ok) break;
-        if (v >= 4 && !warp_wait(&d_full[s], ((v >> 2) - 1) & 1)) {
+        if (v >= 4 && !warp_wait(&d_full[s], ((v >> 2) - 1) & 1, a.wait_limit)) {
           ok = false;
           atomicExch(&g_gemm_error, 1);
           break;
@@ -725,9 +731,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       int i = 0, v = vb + (kPair ? grp : 0);
 #pragma unroll 1
       for (int c0 = 0; c0 < per_job; c0 += kTcChunk, ++chunk) {
-        if (ok && !warp_wait(&s_full[wd][chunk & 1], (chunk >> 1) & 1)) {
+        if (!ok) break;
+        if (!warp_wait(&s_full[wd][chunk & 1], (chunk >> 1) & 1, a.wait_limit)) {
           ok = false;
           if (lane == 0) atomicExch(&g_gemm_error, 8);
+          break;
         }
         const __half* const sc = reinterpret_cast<const __half*>(scales + ((chunk & 1) * 2 + (lane >> 4)) * kTcScaleBytes) +
                                  (lane & 15) - c0 * 16;
@@ -736,7 +744,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (; i < end && ok; ++i, v += kPair ? 2 : 1) {
           const int s = v & 3;
           const float scale = __half2float(sc[i * 16]);
-          if (!warp_wait(&d_full[s], (v >> 2) & 1)) {
+          if (!warp_wait(&d_full[s], (v >> 2) & 1, a.wait_limit)) {
             ok = false;
             if (lane == 0) atomicExch(&g_gemm_error, 4);
             break;
@@ -764,6 +772,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (; loaded < min(steps, zb + i + kTcB); ++loaded) load_b(loaded);
           }
         }
+        if (!ok) break;
         __syncwarp();  // every lane has read its scales
         request_scales();
       }
@@ -817,6 +826,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       sync_all();
       if (s_last && ok) tc_add_parts(*late, st, ti);
+    }
+    if (!ok) {
+      // Shared memory may not be left with copies on their way: the last request of scales per slot and
+      // this warp's last request of activations (those before it have been waited for; its barrier
+      // may be a phase further, never one behind, for a warp requests when the products of the unit's
+      // predecessor in the stage are complete).
+      for (int r = max(snext - 2, 0); r < snext; ++r) bar_wait(&s_full[wd][r & 1], (r >> 1) & 1, kGemmWaitLimit);
+      const int u = unit - 8;
+      if (kTma && u >= 0 && 2 * u < steps) bar_wait(&b_full[u & (kTcB / 2 - 1)], (u / (kTcB / 2)) & 1, kGemmWaitLimit);
     }
     if (!kTma) asm volatile("cp.async.wait_all;" ::: "memory");
   }
@@ -919,7 +937,11 @@ extern "C" int qe_w4_plan_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, qe_w
 }
 
 extern "C" int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream) {
-  if (!p || !cfg) return QE_ERR_ARG;
+  return qe_w4_gemm_bounded(p, cfg, kGemmWaitLimit, stream);
+}
+
+extern "C" int qe_w4_gemm_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wait_limit, void* stream) {
+  if (!p || !cfg || wait_limit < 0) return QE_ERR_ARG;
   if (p->N < 1 || p->N > QE_MAX_GEMM_ROWS || p->Mp % 16 || p->Kp % 128 || p->Mp <= 0 || p->Kp <= 0) return QE_ERR_ARG;
   if (p->K != p->Kp || p->M <= 0 || p->x_f16 || !p->x || !p->out) return QE_ERR_ARG;
   if (p->epilogue == QE_EPI_SWIGLU ? p->M > p->Mp / 2 : p->M > p->Mp) return QE_ERR_ARG;
@@ -954,6 +976,7 @@ extern "C" int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* str
     a.o.out_f32 = (p->out_f32 && p->epilogue == QE_EPI_NONE) ? 1 : 0;
     a.G = G;
     a.tiles = p->Mp / 16;
+    a.wait_limit = wait_limit;
     a.kparts = gemm_kparts(a.tiles, G, p->epilogue);
     if (a.kparts > 1 && (!p->ws || !p->counters)) a.kparts = 1;  // no scratch: whole K per job
     a.ws = p->ws;

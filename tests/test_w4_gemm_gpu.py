@@ -181,3 +181,36 @@ def test_unsupported_arguments_are_refused(api):
     with pytest.raises(RuntimeError):
         api["gemm"](rand_x(16, 500), api["q"](rand_w(64, 500, seed=43)))  # K != Kp
     assert api["w4"].ring_error() == 0
+
+
+@pytest.mark.parametrize("limit", [0, 1, 2, 5, 20, 100])
+@pytest.mark.parametrize("M,K,swiglu", [(148 * 128 * 2 + 77, 640, True), (148 * 128, 57 * 128, False), (5120, 6144, False)])
+def test_waits_that_run_out(api, M, K, swiglu, limit):
+    """The tensor-memory kernel with few polls per wait (a walk of a pair and a lone super-tile, more scales
+    than two requests, K split): the launch ends, says so, and leaves scratch and device as before."""
+    import ctypes as C
+
+    from qengine_b200._lib import W4Cfg, W4Params, W4Plan, lib
+    w4 = api["w4"]
+    p = api["qgu"](rand_w(M // 2, K, seed=51), rand_w(M // 2, K, seed=52)) if swiglu else api["q"](rand_w(M, K, seed=51))
+    base = rand_x(1, 64 * 8 + K, seed=53)[0]
+    for x in (rand_x(40, K, seed=54), base.as_strided((40, K), (8, 1))):  # by tensor map; copied by the warps
+        want, got = (torch.empty(40, p.M, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        w4.gemm(x, p.qw, p.scales, want, p.M, swiglu=swiglu)
+        a = W4Params(p.qw.data_ptr(), p.scales.data_ptr(), x.data_ptr(), got.data_ptr(), None, None, p.M, K,
+                     16 * p.qw.size(0), 64 * p.qw.size(1), 40, x.stride(0), got.stride(0), int(swiglu), 0, 0)
+        cfg, plan = W4Cfg(0, 0, 0, 1, 0, -1, 0, 4), W4Plan()
+        assert lib.qe_w4_plan_gemm(C.byref(a), C.byref(cfg), C.byref(plan)) == 0
+        ws = torch.zeros(max(plan.ws_floats, 4), device=DEV)
+        counters = torch.zeros(max(plan.counters, 1), dtype=torch.int32, device=DEV)
+        a.ws, a.counters = ws.data_ptr(), counters.data_ptr()
+        stream = torch.cuda.current_stream().cuda_stream
+        assert lib.qe_w4_gemm_bounded(C.byref(a), C.byref(cfg), -1, stream) == -22
+        assert lib.qe_w4_gemm_bounded(C.byref(a), C.byref(cfg), limit, stream) == 0
+        error = w4.ring_error()
+        assert error > 0 if limit == 0 else error >= 0
+        if error == 0:
+            assert torch.equal(bits(got), bits(want))
+        assert lib.qe_w4_clear_error() == 0 and not counters.any()
+        assert lib.qe_w4_gemm(C.byref(a), C.byref(cfg), stream) == 0
+        assert w4.ring_error() == 0 and torch.equal(bits(got), bits(want)) and not counters.any()
