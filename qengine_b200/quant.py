@@ -17,6 +17,7 @@ The packer below builds the words with a reshape of the code matrix to
 from __future__ import annotations
 
 from dataclasses import dataclass
+from pathlib import Path
 
 import torch
 
@@ -116,11 +117,20 @@ def _quantize_pack(W: torch.Tensor, M: int, K: int, gate_up: bool, rows_per_step
 _PACK_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
+_LIBRARY = Path(__file__).resolve().with_name("libqengine_b200.so")
+
+
+def _packer_runs_on(device: torch.device) -> bool:
+    """The library is compiled for sm_100a, which only devices of capability 10.0 run. Packing needs no more
+    than torch, so other devices, and a checkout whose library is not built, go on with that."""
+    return torch.cuda.get_device_capability(device) == (10, 0) and _LIBRARY.exists()
+
+
 def _on_gpu(*mats: torch.Tensor) -> bool:
     """Matrices the GPU packer takes: same CUDA device and type, unit stride along K, not empty."""
     a = mats[0]
     return all(m.is_cuda and m.device == a.device and m.dtype == a.dtype and m.dtype in _PACK_DTYPE and m.numel() > 0 and
-               m.stride(1) == 1 and m.stride(0) >= m.shape[1] for m in mats)
+               m.stride(1) == 1 and m.stride(0) >= m.shape[1] for m in mats) and _packer_runs_on(a.device)
 
 
 def _pack_on_gpu(*mats: torch.Tensor) -> W4Packed:
