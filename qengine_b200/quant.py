@@ -126,9 +126,23 @@ def _packer_runs_on(device: torch.device) -> bool:
     return torch.cuda.get_device_capability(device) == (10, 0) and _LIBRARY.exists()
 
 
+def _plain(m: torch.Tensor) -> bool:
+    """Its elements are what lies at its data pointer: no subclass (fake tensors among them), no wrapper of a
+    function transform, no negation still to be done."""
+    return type(m) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(m) and \
+        not m.is_neg()
+
+
+def _traced() -> bool:
+    """Somebody records the operators that run, or replaces them: a launch behind torch's back would be missed."""
+    return torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0
+
+
 def _on_gpu(*mats: torch.Tensor) -> bool:
     """Matrices the GPU packer takes: same CUDA device and type, unit stride along K, not empty."""
     a = mats[0]
+    if _traced() or not all(_plain(m) for m in mats):
+        return False
     return all(m.is_cuda and m.device == a.device and m.dtype == a.dtype and m.dtype in _PACK_DTYPE and m.numel() > 0 and
                m.stride(1) == 1 and m.stride(0) >= m.shape[1] for m in mats) and _packer_runs_on(a.device)
 

@@ -50,3 +50,14 @@ def test_views_and_misaligned_rows():
         _same(quant.quantize_w4(dev[rows, cols]), quant.quantize_w4(big[rows, cols]))
     _same(quant.quantize_w4(dev.T), quant.quantize_w4(big.T))                    # no unit stride along K: torch path
     _same(quant.quantize_w4(dev.double()), quant.quantize_w4(big.double()))
+
+
+def test_lazily_negated_and_traced_matrices():
+    """A lazy negation is not in memory yet, and a trace must hold the packing, not its first result."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from qengine_b200 import quant
+    a, b = (torch.randn(48, 256, generator=torch.Generator().manual_seed(s)).to(torch.bfloat16) for s in (6, 7))
+    _same(quant.quantize_w4(torch._neg_view(a.cuda())), quant.quantize_w4(-a))
+    traced = make_fx(lambda w: quant.quantize_w4(w).qw)(a.cuda())
+    assert torch.equal(traced(b.cuda()).cpu(), quant.quantize_w4(b).qw)
