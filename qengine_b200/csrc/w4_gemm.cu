@@ -570,6 +570,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t idesc =
         (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((128u >> 4) << 24);
     const uint64_t db0 = tc_desc(sa(Bbase));
+    dep_wait();  // before the first bounded wait: its limit is not for the producer of x to use up
     if (elect_one()) {
       int v = 0, z = 0;  // micro-steps issued, step
       bool ok = true;
@@ -617,10 +618,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int i = 0; i < kTcAhead; ++i) {
         const int v = v0 + 2 * i, s = v & 3;
         if (v >= V || !ok) break;
-        if (v >= 4 && !warp_wait(&d_full[s], ((v >> 2) - 1) & 1, a.wait_limit)) {
-          ok = false;
-          atomicExch(&g_gemm_error, 1);
-          break;
+        if (v >= 4) {
+          if (v < 6) dep_wait();  // before the group's first bounded wait, as in the issuing warp
+          if (!warp_wait(&d_full[s], ((v >> 2) - 1) & 1, a.wait_limit)) {
+            ok = false;
+            atomicExch(&g_gemm_error, 1);
+            break;
+          }
         }
         tc_fence_after();
         const uint32_t t0 = t_lane + s * 64;

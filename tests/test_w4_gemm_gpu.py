@@ -214,3 +214,26 @@ def test_waits_that_run_out(api, M, K, swiglu, limit):
         assert lib.qe_w4_clear_error() == 0 and not counters.any()
         assert lib.qe_w4_gemm(C.byref(a), C.byref(cfg), stream) == 0
         assert w4.ring_error() == 0 and torch.equal(bits(got), bits(want)) and not counters.any()
+
+
+def test_waits_do_not_count_the_time_of_the_kernel_before(api):
+    """With programmatic launch the GEMM's blocks may be resident long before their activations are there
+    (one block that streams 2 x 256 MB stands for it). A limit of polls that covers the product's own waits
+    must not be used up on that."""
+    import ctypes as C
+
+    from qengine_b200 import _C
+    from qengine_b200._lib import W4Cfg, W4Params, lib
+    M, K = 148 * 128, 1280
+    p, x = api["q"](rand_w(M, K, seed=71)), rand_x(64, K, seed=72)
+    want, got = api["gemm"](x, p), torch.empty(64, M, dtype=torch.bfloat16, device=DEV)
+    a = W4Params(p.qw.data_ptr(), p.scales.data_ptr(), x.data_ptr(), got.data_ptr(), None, None, M, K, 16 * p.qw.size(0),
+                 64 * p.qw.size(1), 64, K, M, 0, 0, 0)
+    cfg = W4Cfg(0, 0, 0, 1, 0, -1, 0, 4)
+    row, y = torch.ones(1, 1 << 27, dtype=torch.bfloat16, device=DEV), torch.empty(1, 1, dtype=torch.bfloat16, device=DEV)
+    torch.cuda.synchronize()
+    _C.gemv_bf16(row, row, y)
+    assert lib.qe_w4_gemm_bounded(C.byref(a), C.byref(cfg), 20000, torch.cuda.current_stream().cuda_stream) == 0
+    error = api["w4"].ring_error()
+    assert lib.qe_w4_clear_error() == 0
+    assert error == 0 and torch.equal(bits(got), bits(want))
