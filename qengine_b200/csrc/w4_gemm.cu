@@ -459,18 +459,32 @@ __device__ __forceinline__ void tc_store(const OutDesc& o, int tile0, int ti, in
       tc_put4(o, vec, e >> 5, tile0 * 16 + (e & 31) * 4, get(e >> 5, (e & 31) * 4));
   }
 }
+// Four sums of the workspace: at once where the caller's array is 16-byte aligned, which nothing asks of it.
+__device__ __forceinline__ void ws_put(float* p, const float4& f, bool vec) {
+  if (vec) {
+    __stcg(reinterpret_cast<float4*>(p), f);
+  } else {
+    __stcg(p, f.x), __stcg(p + 1, f.y), __stcg(p + 2, f.z), __stcg(p + 3, f.w);
+  }
+}
+__device__ __forceinline__ float4 ws_get(const float* p, bool vec) {
+  if (vec) return __ldcg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+}
+__device__ __forceinline__ bool ws_vec(const GemmArgs& a) { return (reinterpret_cast<uintptr_t>(a.ws) & 15) == 0; }
 // The parts of a super-tile split along K, added in ascending order.
 __device__ __forceinline__ void tc_add_parts(const GemmArgs& a, int st, int ti) {
   __threadfence();
   const int KP = a.kparts;
-  const float4* wp = reinterpret_cast<const float4*>(a.ws + (size_t)(st * KP) * (64 * 128));
+  const bool vec = ws_vec(a);
+  const float* wp = a.ws + (size_t)(st * KP) * (64 * 128);
   tc_store(a.o, st * 8, ti, 256, [&](int n, int m0) {
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int p0 = 0; p0 < KP; p0 += 4) {
       float4 x[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (p0 + k < KP) x[k] = __ldcg(wp + (size_t)(p0 + k) * (64 * 32) + n * 32 + (m0 >> 2));
+        if (p0 + k < KP) x[k] = ws_get(wp + (size_t)(p0 + k) * (64 * 128) + n * 128 + m0, vec);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (p0 + k < KP) f.x += x[k].x, f.y += x[k].y, f.z += x[k].z, f.w += x[k].w;
@@ -816,10 +830,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const GemmArgs* late = &a;
       asm volatile("" : "+l"(late));
       const int ti = tid - 32, st = cta / KP;
-      float4* wsj = reinterpret_cast<float4*>(late->ws + (size_t)cta * (64 * 128));
+      float* wsj = late->ws + (size_t)cta * (64 * 128);
+      const bool vec = ws_vec(*late);
 #pragma unroll 4
       for (int e = ti; e < late->o.N * 32; e += 256)
-        __stcg(wsj + e, *reinterpret_cast<const float4*>(stage + (e >> 5) * kTcPitch + (e & 31) * 4));
+        ws_put(wsj + 4 * e, *reinterpret_cast<const float4*>(stage + (e >> 5) * kTcPitch + (e & 31) * 4), vec);
       __threadfence();
       sync_all();
       if (ti == 0) {

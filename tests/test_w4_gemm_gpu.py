@@ -183,6 +183,27 @@ def test_unsupported_arguments_are_refused(api):
     assert api["w4"].ring_error() == 0
 
 
+@pytest.mark.parametrize("M,K", [(5120, 6144), (200, 3072)])
+@pytest.mark.parametrize("first", [1, 2, 3])
+def test_workspace_of_any_alignment(api, M, K, first):
+    """K split: the caller's partial sums need no alignment beyond a float's."""
+    import ctypes as C
+
+    from qengine_b200._lib import W4Cfg, W4Params, W4Plan, lib
+    p, x = api["q"](rand_w(M, K, seed=61)), rand_x(64, K, seed=62)
+    want, got = api["gemm"](x, p), torch.empty(64, M, dtype=torch.bfloat16, device=DEV)
+    a = W4Params(p.qw.data_ptr(), p.scales.data_ptr(), x.data_ptr(), got.data_ptr(), None, None, M, K, 16 * p.qw.size(0),
+                 64 * p.qw.size(1), 64, x.stride(0), got.stride(0), 0, 0, 0)
+    cfg, plan = W4Cfg(0, 0, 0, 1, 0, -1, 0, 4), W4Plan()
+    assert lib.qe_w4_plan_gemm(C.byref(a), C.byref(cfg), C.byref(plan)) == 0 and plan.ws_floats > 0
+    ws = torch.full((plan.ws_floats + 8,), 7.0, device=DEV)
+    counters = torch.zeros(plan.counters, dtype=torch.int32, device=DEV)
+    a.ws, a.counters = ws.data_ptr() + 4 * first, counters.data_ptr()
+    assert lib.qe_w4_gemm(C.byref(a), C.byref(cfg), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(bits(got), bits(want))
+    assert (ws[:first] == 7).all() and (ws[first + plan.ws_floats:] == 7).all() and not counters.any()
+
+
 @pytest.mark.parametrize("limit", [0, 1, 2, 5, 20, 100])
 @pytest.mark.parametrize("M,K,swiglu", [(148 * 128 * 2 + 77, 640, True), (148 * 128, 57 * 128, False), (5120, 6144, False)])
 def test_waits_that_run_out(api, M, K, swiglu, limit):
