@@ -720,6 +720,7 @@ class Engine:
 
     # -- wide prefill passes ------------------------------------------------------------------------
     WIDE, WIDE_MIN = 64, 32  # rows per wide pass; shorter prompts are not worth a second set of graphs
+    WIDE_PART_BYTES = 32 << 20  # attention partials of a wide pass beyond the 8 rows' own (27B shape, 64 rows: 25 MB)
 
     def wide_ok(self) -> bool:
         """Wide passes exist for a single GPU with every decoder matrix in the W4 wire format."""
@@ -737,6 +738,16 @@ class Engine:
         head = ((P - 1) // NMAX) * NMAX
         return head if wide and head >= self.WIDE_MIN and self.wide_ok() else 0
 
+    def _wide_attn_rows(self) -> int:
+        """Rows per attention launch of a wide pass: all of them, fewer where their partials (which grow
+        with the number of splits) would take more than WIDE_PART_BYTES, and the 8 of an ordinary pass, on
+        its buffers, where that leaves no more or the number of splits selects the tensor-core kernel."""
+        c = self.cfg
+        if c.head_dim == 256 and self.ATTN_SPLITS % 6 == 0:
+            return NMAX
+        fit = self.WIDE_PART_BYTES // (c.hq * self.ATTN_SPLITS * c.head_dim * 4)
+        return max(NMAX, min(self.WIDE, fit // NMAX * NMAX))
+
     def _make_wide_buffers(self):
         c, dev, W, H = self.cfg, self.dev, self.WIDE, self.cfg.hidden
 
@@ -747,26 +758,29 @@ class Engine:
             pass
         B = _B()
         B.tok = buf(W + 1, dt=I32)
-        B.ctl = buf(W // NMAX, 32, dt=I32)  # control words of the 8-row sub-passes
-        B.off = (torch.arange(W // NMAX, dtype=I32, device=dev) * NMAX).contiguous()
         B.h, B.xn, B.mo, B.hid = (buf(W, H) for _ in range(4))
         B.proj = buf(W, -(-max(c.gdn_proj_rows, c.attn_proj_rows) // 8) * 8)
         B.mix = buf(W, max(c.value_dim, c.hq * c.head_dim))
         B.act = buf(W, c.inter)
         B.q = buf(W, c.hq * c.head_dim)
-        B.part_o = B.part_ml = None  # partial results of the attention over all rows, where it takes them
-        if c.head_dim != 256 or self.ATTN_SPLITS % 6:
-            B.part_o = buf(W, c.hq, self.ATTN_SPLITS, c.head_dim, dt=F32)
-            B.part_ml = buf(W, c.hq, self.ATTN_SPLITS, 2, dt=F32)
+        B.attn_rows = R = self._wide_attn_rows()
+        B.part_o, B.part_ml = self.part_o, self.part_ml  # partial results of an attention launch
+        if R > NMAX:
+            B.part_o = buf(R, c.hq, self.ATTN_SPLITS, c.head_dim, dt=F32)
+            B.part_ml = buf(R, c.hq, self.ATTN_SPLITS, 2, dt=F32)
+        if R < W:  # control words of the attention's sub-passes: positions R apart
+            B.ctl = buf(-(-W // R), 32, dt=I32)
+            B.off = (torch.arange(-(-W // R), dtype=I32, device=dev) * R).contiguous()
         if self.has_mtp:
             B.cat, B.mh = buf(W, 2 * H), buf(W, H)
         self.wb = B
 
     def _wide_mixer(self, L, n, kv_only=False):
-        """Token mixing of a wide pass. DeltaNet and the attention over caches up to 8K positions take
-        all rows in one launch; the tensor-core attention of longer caches takes 8 rows, so there the
-        rows go through in sub-passes, each with its own control words (position). kv_only: just
-        write K and V (a draft layer during prefill: nothing else of it is kept)."""
+        """Token mixing of a wide pass. DeltaNet takes all rows in one launch, and so does the attention over
+        caches up to 8K positions; the tensor-core attention of longer caches takes 8 rows, and many
+        splits as many as `_wide_attn_rows` says: there the rows go through in sub-passes, each with
+        its own control words (position). kv_only: just write K and V (a draft layer during prefill:
+        nothing else of it is kept)."""
         c, B = self.cfg, self.wb
         if L["type"] == "linear_attention":
             pr = B.proj[:n, :c.gdn_proj_rows]
@@ -784,12 +798,11 @@ class Engine:
                           B.q[:n], L["kc"], L["vc"], c.eps)
         if kv_only:
             return out
-        if B.part_o is not None:
-            _C.attn_decode_rows(B.q[:n], L["kc"], L["vc"], self.ctl, pr[:, :nq], B.part_o, B.part_ml, out)
-        else:
-            for j in range(n // NMAX):
-                rows = slice(j * NMAX, (j + 1) * NMAX)
-                _C.attn_decode(B.q[rows], L["kc"], L["vc"], B.ctl[j], pr[rows, :nq], self.part_o, self.part_ml, out[rows])
+        R = B.attn_rows
+        decode = _C.attn_decode if R == NMAX else _C.attn_decode_rows
+        for j in range(-(-n // R)):
+            rows = slice(j * R, min(n, (j + 1) * R))
+            decode(B.q[rows], L["kc"], L["vc"], B.ctl[j] if j else self.ctl, pr[rows, :nq], B.part_o, B.part_ml, out[rows])
         return out
 
     def _wide_pass(self, n, mtp):
@@ -799,9 +812,9 @@ class Engine:
         Follows python/qengine/engine.py:434-477 (layer, main) and :479-496 (draft layer) of the
         reference."""
         c, B, lin, eps = self.cfg, self.wb, self.linear, self.cfg.eps
-        nb = n // NMAX
+        nb = -(-n // B.attn_rows)  # sub-passes of the attention
         self._flush()
-        if B.part_o is None:  # control words of the attention's sub-passes: positions 8 apart
+        if nb > 1:
             B.ctl[:nb].copy_(self.ctl.expand(nb, -1))
             B.ctl[:nb, self.POS].add_(B.off[:nb])
         h, xn, mo = B.h[:n], B.xn[:n], B.mo[:n]

@@ -402,3 +402,23 @@ def test_wide_prefill_as_the_engines_default(setup):
     assert auto.generate(prompt, 24) == eng.generate(prompt, 24, wide=True)
     assert ("wide", 64, False) in auto.graphs and ("wide", 8, False) in auto.graphs
     assert auto.generate(prompt, 24, wide=False) == eng.generate(prompt, 24)
+
+
+@pytest.mark.parametrize("splits,rows", [(16, 64), (200, 64), (300, 48), (1000, 16)])
+def test_attention_partials_of_a_wide_pass_are_bounded(setup, splits, rows):
+    """More splits: fewer rows per attention launch instead of more memory (bytes per row and split here:
+    8 heads x 64 dims x 4), with the same bits."""
+    from qengine_b200 import synth
+    from qengine_b200.engine import Engine
+    cfg, Wp, _ = setup
+    prompt = synth.prompt_ids(130, cfg.vocab, seed=34)
+    small, large = (Engine(cfg, synth.model_to(Wp, "cuda"), max_len=256, attn_splits=splits) for _ in range(2))
+    large.WIDE_PART_BYTES = 1 << 40  # all rows at once
+    a, b = (_prefill_and_snapshot(e, prompt, True) for e in (small, large))
+    assert small.wb.attn_rows == rows and large.wb.attn_rows == 64
+    assert small.wb.part_o.numel() * 4 <= max(Engine.WIDE_PART_BYTES, small.part_o.numel() * 4)
+    assert torch.equal(a[0], b[0]) and a[2:] == b[2:]
+    assert all(torch.equal(x, y) for p, q in zip(a[1], b[1]) for x, y in zip(p, q))
+    small.ATTN_SPLITS, small.wb = 2048, None  # sizes alone: the 8 rows' own buffers
+    assert small._wide_attn_rows() == 8
+    small.ATTN_SPLITS = splits
