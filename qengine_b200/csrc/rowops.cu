@@ -123,7 +123,8 @@ rmsnorm1p_any_kernel(bf16* x, const bf16* delta,
 // whatever NR and WR are, so neither shows in the result.
 // Bound by HBM (2 bytes per weight) for one row; with more rows by issue slots, since every 16 bytes of
 // weights cost the load and the widening of NR x 16 bytes of activations. Two weight rows per warp share
-// them, and weights leave no L1 lines. 62,080 x 5,120, us before (one row per warp) -> now:
+// them (which sizes take which: gemv_rows_per_warp), and weights leave no L1 lines. 62,080 x 5,120, us before (one
+// row per warp) -> now:
 // 1 row 90 -> 90, 3 rows 121 -> 99 (6.4 TB/s; 137 -> 102 called on its own), 5 rows 170 -> 134, 8 rows 270 -> 206.
 // Four rows per warp: the same at this size, 20 % slower at 1,000 rows x 3. Multiply-adds in pairs (even
 // and odd k, fma.rn.f32x2) take another 4 % (3 rows) to 12 % (8 rows) off, but the second accumulator costs
@@ -351,21 +352,50 @@ extern "C" int qe_rmsnorm1p(void* x, const void* delta, const void* w, void* out
                      ldd, ldo, eps);
 }
 
+// Weight rows per warp. Two share the activations, but both forms put 8 rows into a block, so half the
+// warps keep loads in flight; and a block costs more, so a last wave of few blocks does, too. Resident blocks per
+// SM by their registers: one row per warp 5 (2, 3 activation rows), 4 (4 to 7); two rows per warp 7 (2, 3),
+// 6 (4), 5 (5 to 7), 4 (8). Measured, one / two rows per warp, us (148 SMs, graph of 24 calls):
+//   * a single row: nothing to share. 8 rows: two (1,000 x 5,120 18.6 / 14.5; 62,080 x 5,120 270 / 206).
+//   * 2 to 4 rows: one, except where only two fit into one wave (6,144 x 5,120 16.8 / 13.1, 23.0 / 16.8, 21.3 / 19.6)
+//     and behind two full waves of one (three for 4 rows: 12,288 x 5,120, 3 rows 30.8 / 30.6; 62,080 124 / 98;
+//     14,336 x 5,120, 4 rows 39.7 / 39.4; 62,080 155 / 120). Between: 8,192 x 5,120, 4 rows 23.1 / 34.0; 10,240 x 5,120,
+//     2 rows 20.6 / 23.7. 2 rows, which win least, lose in a thin third wave too (17,300 x 3,584 23.2 / 25.0).
+//     Short rows gain from sharing earlier (8,700 x 512, 2 rows 3.6 / 3.2; 13,600 x 1,280, 4 rows 13.1 / 11.4; not yet
+//     at 9,500 x 1,440: 7.4 / 8.1, 11.0 / 12.4).
+//   * 5 to 7 rows: two (1,000 x 5,120 13.1 / 12.3, 14.6 / 13.5, 17.5 / 15.8; 62,080, 5 rows 174 / 134), except for a
+//     thin second wave of long rows (6,144 x 5,120 27.8 / 29.2, 30.1 / 31.5, 34.6 / 35.3; x 800 the other way,
+//     7.3 / 7.2, 8.1 / 7.7, 9.1 / 8.7) and 5 rows where one per warp just fits (4,096 x 5,120 15.5 / 16.5; x 2,560
+//     9.2 / 8.9).
+static int gemv_rows_per_warp(int nr, int N, int K) {
+  const int blocks = (N + kGemvRows - 1) / kGemvRows, sms = qe_sm_count();
+  auto within = [&](int lo, int hi) { return blocks > lo * sms && blocks <= hi * sms; };  // blocks per SM in (lo, hi]
+  auto above = [&](int lo) { return blocks > lo * sms; };
+  const bool brief = K < 1536;
+  switch (nr) {
+    case 1: return 1;
+    case 2: return within(5, 7) || (brief ? above(K <= 640 ? 7 : 9) : within(10, 14) || above(15)) ? 2 : 1;
+    case 3: return within(5, 7) || above(brief ? K <= 640 ? 7 : 9 : 10) ? 2 : 1;
+    case 4: return within(4, 6) || above(brief ? K <= 640 ? 8 : 9 : 12) ? 2 : 1;
+    case 5: return (within(3, 4) && K >= 4096) || (within(5, 8) && K >= 2048) ? 1 : 2;
+    case 6: return within(5, 7) && K >= 3584 ? 1 : 2;
+    case 7: return within(5, 7) && K >= 2048 ? 1 : 2;
+    default: return 2;
+  }
+}
+
 extern "C" int qe_gemv_bf16(const void* W, const void* x, void* out, int nr, int N, int K, long ldx,
                             long ldo, void* stream) {
   if (nr < 1 || nr > QE_MAX_ROWS || K % 8 || N < 1) return QE_ERR_ARG;
   if (!aligned16(W) || !aligned16(x) || ldx % 8) return QE_ERR_ARG;
-  // One weight row per warp for a single activation row (nothing to share), and for up to four where half
-  // the warps would not fill the chip (one against two rows per warp, us: 3,000 x 4,096, 4 rows 11.9 / 14.1;
-  // 20,000 x 2,000 24.3 / 20.9).
-  const int wr = nr == 1 || (nr <= 4 && N < 8192) ? 1 : 2;
+  const int wr = gemv_rows_per_warp(nr, N, K);
   const dim3 grid((N + kGemvRows - 1) / kGemvRows), block(kGemvRows / wr * 32);
   cudaStream_t s = (cudaStream_t)stream;
   const bf16 *w = (const bf16*)W, *xx = (const bf16*)x;
   bf16* o = (bf16*)out;
   switch (nr) {
 #define QB_ROWS(R) \
-  case R: return (int)launch(wr == 1 ? gemv_bf16_rows_kernel<R, R <= 4 ? 1 : 2> : gemv_bf16_rows_kernel<R, R == 1 ? 1 : 2>, grid, block, 0, s, pdl_on(), w, xx, o, N, K, ldx, ldo);
+  case R: return (int)launch(wr == 1 ? gemv_bf16_rows_kernel<R, R == 8 ? 2 : 1> : gemv_bf16_rows_kernel<R, R == 1 ? 1 : 2>, grid, block, 0, s, pdl_on(), w, xx, o, N, K, ldx, ldo);
     QB_ROWS(1) QB_ROWS(2) QB_ROWS(3) QB_ROWS(4) QB_ROWS(5) QB_ROWS(6) QB_ROWS(7) QB_ROWS(8)
 #undef QB_ROWS
   }

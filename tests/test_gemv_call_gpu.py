@@ -76,8 +76,8 @@ def test_refusals(w4):
 @pytest.mark.parametrize("N", [1, 2, 7, 8, 9, 4097])
 @pytest.mark.parametrize("nr,K", [(1, 8), (2, 264), (3, 1024), (8, 1032)])
 def test_bf16_gemv_tile_edges(N, nr, K):
-    """Two weight rows per warp, four warps per block: odd last rows, and lanes with zero to two packets.
-    Bound: one rounding to bf16 and K fp32 additions."""
+    """One weight row per warp (1, 2, 3 activation rows at these sizes) and two (8): odd last rows, and lanes
+    with zero to two packets. Bound: one rounding to bf16 and K fp32 additions."""
     from qengine_b200 import _C
     W, x = rand(N, K).to(BF), rand(nr, K, seed=1).to(BF)
     ob = torch.full((nr, N + 3), 7.0, dtype=BF, device=DEV)
@@ -85,6 +85,26 @@ def test_bf16_gemv_tile_edges(N, nr, K):
     ref = x.double() @ W.double().T
     bnd = 2.0 ** -8 * ref.abs() + K * 2.0 ** -23 * (x.double().abs() @ W.double().abs().T) + 1e-30
     assert ((ob[:, :N].double() - ref).abs() <= bnd).all() and (ob[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("nr,per_sm,K", [(nr, b, 72) for nr in (2, 3, 4, 5, 6, 7, 8) for b in (4, 5, 6, 7, 8, 10)] +
+                         [(2, b, 1536) for b in (10, 14, 15)] + [(nr, 9, 648) for nr in (2, 3, 4)] +
+                         [(3, 10, 1536), (4, 12, 1536), (5, 3, 4096), (5, 4, 4096), (5, 8, 2048), (6, 5, 3584),
+                          (6, 7, 3584), (7, 5, 2048), (7, 7, 2048)])
+def test_bf16_gemv_on_both_sides_of_each_rule(nr, per_sm, K):
+    """The number of weight rows per warp changes with the blocks (of 8 rows) per SM and with K: a last block
+    that is full, one row short, and one row alone, each with the bits of one activation row at a time."""
+    from qengine_b200 import _C
+    from qengine_b200._lib import lib
+    edge = 8 * per_sm * lib.qe_sm_count()
+    W, x = rand(edge + 8, K).to(BF), rand(nr, K, seed=1).to(BF)
+    one = torch.empty(nr, edge + 8, dtype=BF, device=DEV)
+    for r in range(nr):
+        _C.gemv_bf16(W, x[r:r + 1], one[r:r + 1])
+    for N in (edge - 8, edge - 1, edge, edge + 1, edge + 8):
+        ob = torch.full((nr, N + 3), 7.0, dtype=BF, device=DEV)
+        _C.gemv_bf16(W[:N], x, ob[:, :N])
+        assert torch.equal(ob[:, :N].view(torch.int16), one[:, :N].view(torch.int16)) and (ob[:, N:] == 7).all()
 
 
 @pytest.mark.parametrize("hd", [64, 128, 256])
