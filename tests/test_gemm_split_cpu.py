@@ -1,7 +1,7 @@
 """Index arithmetic of the prefill GEMM (qengine_b200/csrc/w4_gemm.cu), restated in Python and
-checked exhaustively on the CPU: every 1 KB unit of a matrix is multiplied exactly once, by the
-warp that also requested it from HBM in that order, for both kernels and for the shapes that
-exercise their corner cases. A change of the device-side split has to keep these invariants.
+checked exhaustively on the CPU: every 1 KB unit of a matrix is multiplied exactly once, for both
+kernels (in the mma.sync one by the warp that also requested it from HBM, in that order) and for the
+shapes that exercise their corner cases. A change of the device-side split has to keep these invariants.
 """
 from __future__ import annotations
 
@@ -59,10 +59,9 @@ def kparts(tiles, G, swiglu=False):
 
 @pytest.mark.parametrize("tiles,G", SHAPES)
 def test_tensor_memory_kernel_steps_and_rings(tiles, G):
-    """w4_gemm_tc_kernel: jobs (super-tile, part of K) round-robin over the CTAs; the steps of a CTA
-    in order; warps 0..7 prepare the even steps, 8..15 the odd ones, tile = warp % 8; a warp
-    requests its units from HBM in exactly the order in which it consumes them; with K split
-    every CTA has one job at most, so a super-tile without all its tiles is always a last job."""
+    """w4_gemm_tc_kernel: jobs (super-tile, part of K) round-robin over the CTAs; with K split every CTA has
+    one job at most, and a super-tile without all its tiles is always a CTA's last job. (How the warps of
+    a CTA walk through its jobs: test_gemm_walks_cpu.py.)"""
     KP = kparts(tiles, G)
     ST = (tiles + 7) // 8
     J = ST * KP
@@ -70,25 +69,16 @@ def test_tensor_memory_kernel_steps_and_rings(tiles, G):
     assert KP == 1 or J <= SMS
     seen = set()
     for cta in range(nctas):
-        nj = (J - cta + nctas - 1) // nctas if cta < J else 0
-        steps = []  # (job index, tile0, g)
-        for j in range(nj):
-            jidx = cta + j * nctas
-            st, part = divmod(jidx, KP)
-            for g in range(share_begin(G, KP, part), share_begin(G, KP, part + 1)):
-                steps.append((j, st * 8, g))
-        assert all(b[0] - a[0] in (0, 1) for a, b in zip(steps, steps[1:]))
-        for warp in range(16):
-            par, ti = warp >> 3, warp & 7
-            own = [s for z, s in enumerate(steps) if (z & 1) == par]
-            valid = [s[1] + ti < tiles for s in own]
-            # validity is monotone: once a tile is missing, the rest of the warp's stream is too
-            assert valid == sorted(valid, reverse=True)
-            for (j, tile0, g), ok in zip(own, valid):
-                if ok:
-                    u = (tile0 + ti) * G + g
-                    assert u not in seen
-                    seen.add(u)
+        jobs = [divmod(j, KP) for j in range(cta, J, nctas)]
+        assert jobs and (KP == 1 or len(jobs) == 1)
+        assert all(8 * st + 8 <= tiles for st, _ in jobs[:-1])
+        for st, part in jobs:
+            groups = range(share_begin(G, KP, part), share_begin(G, KP, part + 1))
+            assert len(groups) >= 1
+            for tile in range(8 * st, min(8 * st + 8, tiles)):
+                for g in groups:
+                    assert (tile, g) not in seen
+                    seen.add((tile, g))
     assert len(seen) == tiles * G
 
 

@@ -1,7 +1,7 @@
 """`_w4.gemv` / `gemv_swiglu` with default options take a short way to the launch (qe_w4_gemv_call);
 the general way (`job` + `_launch`) is what it is compared with, bit for bit, over the forms both
-accept, and what is refused there is refused here. Also: the two-row BF16 GEMV and the small merge of
-attention splits against the code they stand in for, at the sizes where they begin and end."""
+accept, and what is refused there is refused here. Also: the two-row BF16 GEMV against single rows, and the
+small merge of attention splits against the large one's arithmetic, at the sizes where they begin and end."""
 from __future__ import annotations
 
 import pytest
@@ -107,12 +107,28 @@ def test_bf16_gemv_on_both_sides_of_each_rule(nr, per_sm, K):
         assert torch.equal(ob[:, :N].view(torch.int16), one[:, :N].view(torch.int16)) and (ob[:, N:] == 7).all()
 
 
+def _large_merge(po, ml, gate):
+    """attn_merge_kernel on the partials a call left, for at most 16 splits: then each of its 16 warps has one
+    split at most, the warps are added in ascending order, and L is the butterfly sum of one warp."""
+    m, l = ml[..., 0], ml[..., 1]
+    f = torch.where(m == -torch.inf, 0.0, torch.exp(m - m.amax(-1, keepdim=True)))
+    lanes = torch.nn.functional.pad(l * f, (0, 32 - m.size(-1)))
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[..., torch.arange(32, device=DEV) ^ o]
+    O = torch.zeros_like(po[..., 0, :])
+    for s in range(po.size(-2)):
+        O = O + po[..., s, :] * f[..., s, None]
+    o = (O / lanes[..., :1]).to(BF).float()
+    return (o * (1.0 / (1.0 + torch.exp(-gate.float()))).to(BF).float()).to(BF)
+
+
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("NS", [1, 5, 15, 16, 17])
 @pytest.mark.parametrize("pos", [0, 3, 200])
 def test_merge_of_few_splits(hd, NS, pos):
-    """At most 16 splits merge without shared memory, more with it. The reference sums in fp64 over the
-    prefix; 2 bf16 ulps cover the rounding of O / L, of the gate and of their product."""
+    """At most 16 splits merge without shared memory, more with it: up to there the bits are those of the
+    large merge. The reference sums in fp64 over the prefix; 2 bf16 ulps cover the rounding of O / L, of
+    the gate and of their product."""
     from qengine_b200 import _C
     hq, hkv, L, n = 4, 2, 256, 3
     q, qg = rand(n, hq * hd).to(BF), rand(n, hq * 2 * hd, seed=1).to(BF)
@@ -120,6 +136,9 @@ def test_merge_of_few_splits(hd, NS, pos):
     out = torch.empty(n, hq * hd, dtype=BF, device=DEV)
     po, ml = torch.empty(n, hq, NS, hd, device=DEV), torch.empty(n, hq, NS, 2, device=DEV)
     _C.attn_decode(q, kc, vc, torch.tensor([pos], dtype=torch.int32, device=DEV), qg, po, ml, out)
+    if NS <= 16:
+        want = _large_merge(po, ml, qg.view(n, hq, 2 * hd)[..., hd:]).reshape(n, hq * hd)
+        assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     for t in range(n):
         for h in range(hq):
             k, v = (c[h // 2, :pos + t + 1].double() for c in (kc, vc))

@@ -42,6 +42,22 @@ def test_bits_of_the_torch_packer(M, K, dtype):
     _same(quant.quantize_w4_gate_up(w.cuda(), u.cuda()), quant.quantize_w4_gate_up(w, u))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_infinite_weights(dtype):
+    """An infinite weight makes its group's scale infinite: its own quotient is no number and gets code 0, the
+    finite ones of the group get code 8. As torch's operators have it on the GPU and on the CPU."""
+    from qengine_b200 import quant
+    w = _w(40, 300, torch.float32, seed=8)
+    w[~w.isfinite() | (w.abs() > 6e4)] = 1.0
+    w[5, 7], w[6, 140], w[7, 0], w[7, 1] = torch.inf, -torch.inf, torch.inf, -torch.inf
+    w = w.to(dtype)
+    p = quant.quantize_w4(w.cuda())
+    _same(p, quant.quantize_w4(w))
+    _same(p, quant._quantize_pack(w.cuda(), 40, 300, False).to("cpu"))
+    codes, _ = quant.unpack_codes(p)
+    assert codes[5, 7] == 0 and codes[6, 140] == 0 and (codes[7, :2] == 0).all() and (codes[5, :7] == 8).all()
+
+
 def test_views_and_misaligned_rows():
     from qengine_b200 import quant
     big = torch.randn(300, 1030, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
