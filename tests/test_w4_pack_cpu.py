@@ -19,6 +19,7 @@ def test_only_where_the_library_runs(monkeypatch, tmp_path, capability, built, t
         lib.touch()
     monkeypatch.setattr(quant, "_LIBRARY", lib, raising=False)
     monkeypatch.setattr(torch.cuda, "get_device_capability", lambda device=None: capability)
+    monkeypatch.setattr(quant, "_packer_runs_on", quant._packer_runs_on.__wrapped__)  # asked anew
     monkeypatch.setattr(quant, "_plain", lambda m: True, raising=False)  # the stand-in is no tensor
     m = SimpleNamespace(is_cuda=True, device=torch.device("cuda:0"), dtype=torch.bfloat16, shape=(16, 128),
                         numel=lambda: 2048, stride=lambda d: (128, 1)[d])
