@@ -161,7 +161,7 @@ def _pack_on_gpu(*mats: torch.Tensor) -> W4Packed:
     with torch.cuda.device(dev):
         check(lib.qe_w4_pack(mats[0].data_ptr(), mats[1].data_ptr() if gate_up else None, _PACK_DTYPE[mats[0].dtype], M, K,
                              mats[0].stride(0), mats[-1].stride(0), qw.data_ptr(), sc.data_ptr(),
-                             torch.cuda.current_stream().cuda_stream), "w4_pack")
+                             torch._C._cuda_getCurrentRawStream(dev.index)), "w4_pack")
     return W4Packed(qw, sc, M, K, gate_up)
 
 
