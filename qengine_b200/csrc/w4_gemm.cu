@@ -409,13 +409,6 @@ __device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap* map, i
       ::"r"(dst), "l"(map), "r"(0), "r"(c), "r"(sa(bar))
       : "memory");
 }
-// (a0, a1) += s * (b0, b1): two fp32 fused multiply-adds in one instruction.
-__device__ __forceinline__ void fma2(float& a0, float& a1, float s, float b0, float b1) {
-  asm("{\n\t.reg .b64 a, b, s;\n\t"
-      "mov.b64 a, {%0, %1};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 s, {%2, %2};\n\t"
-      "fma.rn.f32x2 a, s, b, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
-      : "+f"(a0), "+f"(a1) : "f"(s), "f"(b0), "f"(b1));
-}
 
 // Four consecutive output rows (from `row`) of activation row n.
 __device__ __forceinline__ void tc_put4(const OutDesc& o, bool vec, int n, int row, const float4& f) {
@@ -774,7 +767,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             float d[16];
             tc_ld16(t_lane + s * 64 + col0 + h * 16, d);
 #pragma unroll
-            for (int k = 0; k < 16; k += 2) fma2(acc[16 * h + k], acc[16 * h + k + 1], scale, d[k], d[k + 1]);
+            for (int k = 0; k < 16; k += 2) {
+              float* const to = acc + 16 * h + k;
+              const float2 sum = fma2(make_float2(scale, scale), make_float2(d[k], d[k + 1]), make_float2(to[0], to[1]));
+              to[0] = sum.x, to[1] = sum.y;
+            }
           }
           tc_fence_before();
           __syncwarp();
