@@ -317,9 +317,10 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_gemm_kernel(const __grid_consta
 // seen the products of a later step.
 //
 // What bounds it. Per unit of weights (1 KB, 46 clk of HBM time per SM at the copy rate) an SM issues
-// some 240 warp instructions on four schedulers (60 clk) and multiplies for 32 clk; it takes 110 clk:
+// some 270 warp instructions on four schedulers (68 clk) and multiplies for 32 clk; it takes 110 clk:
 // the turns of the issuing thread and of a drain warp, barrier waits of 200 clk and more among them,
-// come one after the other. 64 rows, 27B shapes: gate/up 81.8 -> 44.3 us, in_proj 41.0 -> 26.9,
+// come one after the other. 17 warps leave a thread 96 registers; a drain thread (64 sums, 16 values of D,
+// its cursors) spills 116 bytes (180 without a tensor map). 64 rows, 27B shapes: gate/up 81.8 -> 44.3 us, in_proj 41.0 -> 26.9,
 // down 53.0 -> 35.5, out 25.2 -> 21.2 against the form with A and the weight ring in shared memory,
 // where every warp did all three roles in turn and their latencies added up.
 //

@@ -16,7 +16,8 @@
 // The quotient is only ever rounded to a whole number, so one division per group is enough: w times
 // the reciprocal is within 4e-6 of the quotient where the code is not clamped (|w / scale| <= 8, four
 // roundings of 2^-24 relative each), and only where it lies within 1e-5 of the middle between two
-// whole numbers can the rounding differ: a lane that sees such a weight divides (4e-5 of random ones).
+// whole numbers can the rounding differ (2e-5 of random weights): a lane that has one among its 64
+// weights quantises them all again with divisions.
 #include <type_traits>
 
 #include "w4_dev.cuh"
