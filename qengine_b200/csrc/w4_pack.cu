@@ -11,7 +11,7 @@
 // once, whole sectors on both sides. Bound: HBM. The torch packer goes over the matrix about forty times
 // (int64 code words among them): 7.9 ms for a bf16 gate/up pair of 17,408 x 5,120; this kernel 0.154 ms
 // (2.9 TB/s; the floor at the copy rate is 0.069 ms, the rest is the arithmetic, about ten instructions
-// per weight).
+// per weight). Three blocks per SM cap the 16-bit types at 80 registers, of which they spill 28 to 40 bytes.
 //
 // The quotient is only ever rounded to a whole number, so one division per group is enough: w times
 // the reciprocal is within 4e-6 of the quotient where the code is not clamped (|w / scale| <= 8, four
