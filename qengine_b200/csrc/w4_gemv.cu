@@ -260,6 +260,81 @@ __device__ __forceinline__ void norm_prologue(const GemvArgs& a, unsigned char* 
   __syncthreads();
 }
 
+// The same for ONE row of at most 16 * NT elements, which is what a decode step has: every load of the
+// thread's packets is in flight before the first is used (the loop above takes a second trip to L2
+// for the packets beyond the first NT), the row stays in registers between the two passes, and the
+// code is a fraction of the four-row form's. Same thread -> packet map, same order of every sum: same bits.
+template <int NW>
+__device__ __forceinline__ bool one_row_fits(int K) { return K <= 16 * NW * 32; }
+template <int NW>
+__device__ __forceinline__ void norm_prologue_row(const GemvArgs& a, unsigned char* x_s, float* s_red, int tid, int r,
+                                                  bool writer) {
+  constexpr int NT = NW * 32, WP = 2;
+  const int npk = a.K >> 3;
+  const bf16* row = a.h_in + (long)r * a.ldh;
+  if (a.tok) {
+    const int id = a.tok[r];
+    row = id >= 0 && id < a.vocab ? a.h_in + (size_t)id * a.K : nullptr;  // else: a row of zeros
+  }
+  uint4 hv[WP], dv[WP], wv[WP];
+#pragma unroll
+  for (int i = 0; i < WP; ++i) {
+    const int p = tid + i * NT;
+    hv[i] = dv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (p < npk) {
+      if (row) hv[i] = reinterpret_cast<const uint4*>(row)[p];
+      if (a.delta) dv[i] = reinterpret_cast<const uint4*>(a.delta + (long)r * a.ldd)[p];
+      wv[i] = reinterpret_cast<const uint4*>(a.norm_w)[p];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < WP; ++i) {
+    const int p = tid + i * NT;
+    if (p < npk) {
+      float v[8];
+      widen8(hv[i], v);
+      if (a.delta) {
+        float d[8];
+        widen8(dv[i], d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = rnd(v[e] + d[e]);
+        hv[i] = narrow8(v);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+    }
+  }
+  ss = warp_allsum(ss);
+  if ((tid & 31) == 0) s_red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int w2 = 0; w2 < NW; ++w2) tot += s_red[w2];
+  const float inv = rsqrtf(tot / (float)a.K + a.eps);
+#pragma unroll
+  for (int i = 0; i < WP; ++i) {
+    const int p = tid + i * NT;
+    if (p < npk) {
+      float v[8], g[8];
+      widen8(hv[i], v);
+      widen8(wv[i], g);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * (1.0f + g[e]);
+      const uint4 q = narrow8(v);
+      if (a.xf16) widen8(q, v);  // the bf16-rounded values again, as fp16 (exact for normalised rows)
+      const uint4 q16 = half8(v);
+      if (x_s) reinterpret_cast<uint4*>(x_s)[p] = a.xf16 ? q16 : q;
+      if (writer) {
+        if (a.h_out) reinterpret_cast<uint4*>(a.h_out + (long)r * a.ldho)[p] = hv[i];
+        if (a.xn_out) reinterpret_cast<uint4*>(a.xn_out + (long)r * a.ldxo)[p] = q;
+        if (a.xn16_out) reinterpret_cast<uint4*>(a.xn16_out + (long)r * a.ldx16)[p] = q16;
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // The prologue as a launch of its own: one block per row, the same thread -> packet map and the
 // same reduction order as inside the GEMV, hence the same bits. A pass of several rows runs this
 // (the rows in parallel on as many SMs) in front of a plain GEMV instead of letting every block
@@ -271,7 +346,8 @@ __global__ void __launch_bounds__(NW * 32) norm_rows_kernel(const GemvArgs a) {
   dep_wait();
   __shared__ float s_red[QE_MAX_ROWS][NW];
   const int r = blockIdx.x;
-  norm_prologue<NW>(a, reinterpret_cast<unsigned char*>(a.xn_out), a.ldxo * 2, s_red, threadIdx.x, r, r + 1, true);
+  if (one_row_fits<NW>(a.K)) norm_prologue_row<NW>(a, nullptr, s_red[0], threadIdx.x, r, true);
+  else norm_prologue<NW>(a, reinterpret_cast<unsigned char*>(a.xn_out), a.ldxo * 2, s_red, threadIdx.x, r, r + 1, true);
 }
 
 // A chain is up to kMaxJobs GEMVs that depend on each other only through global memory (the
@@ -391,7 +467,8 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     bool xfast;
     if (a.h_in) {
       const long pitch = (long)a.K * 2 + 16;
-      norm_prologue<NW>(a, x_s, pitch, s_red, tid, 0, a.o.N, blockIdx.x == 0);
+      if (a.o.N == 1 && one_row_fits<NW>(a.K)) norm_prologue_row<NW>(a, x_s, s_red[0], tid, 0, blockIdx.x == 0);
+      else norm_prologue<NW>(a, x_s, pitch, s_red, tid, 0, a.o.N, blockIdx.x == 0);
       xbase = x_s + xrow * pitch + 32 * t;
       xfast = true;
     } else {
