@@ -75,6 +75,11 @@ struct GemvArgs {
   int nwarps;      // warps of a CTA that own work (small matrices keep min_units per warp)
   int quantum;     // warp ranges start at multiples of this many units (4 when G % 4 == 0, else 1)
   int cta_quantum; // CTA ranges start at multiples of this many units: `quantum`, or G (whole tiles)
+  // the deal of the stream, divided out on the host: a division costs a warp some 150 clk, and what
+  // happens before a launch's first weight request and after its last unit is time nothing hides
+  int cta_per, cta_rem;          // quanta (of cta_quantum units) per CTA; the first cta_rem CTAs hold one more
+  int warp_per[2], warp_rem[2];  // quanta per warp in a CTA of cta_per, and of cta_per + 1, CTA quanta
+  unsigned inv_g;                // floor(2^32 / G), see tile_of
   int two_way;     // every CTA range holds at least one tile's worth of units: a cut tile has two owners
   int xf16;        // the activations are fp16: `x` points to fp16 rows, or the prologue leaves fp16
                    // in shared memory (the normalised rows, which fp16 holds exactly, see make_job)
@@ -103,12 +108,18 @@ constexpr int kWaitLimit = 1 << 20;
 __device__ __host__ __forceinline__ int cta_begin(int total, int q, int nctas, int c) {
   return q * share_begin(total / q, nctas, c);
 }
-__device__ __forceinline__ void warp_range(int total, int q, int qc, int nctas, int nwarps, int cta, int warp,
-                                           int& u0, int& u1) {
-  if (cta >= nctas) { u0 = u1 = total; return; }
-  const int b = cta_begin(total, qc, nctas, cta), e = cta_begin(total, qc, nctas, cta + 1);
-  u0 = b + q * share_begin((e - b) / q, nwarps, min(warp, nwarps));
-  u1 = b + q * share_begin((e - b) / q, nwarps, min(warp + 1, nwarps));
+__device__ __forceinline__ void warp_range(const GemvArgs& a, int cta, int warp, int& u0, int& u1) {
+  if (cta >= a.nctas) { u0 = u1 = a.total; return; }
+  const int b = a.cta_quantum * (cta * a.cta_per + min(cta, a.cta_rem)), big = cta < a.cta_rem;
+  const int per = a.warp_per[big], rem = a.warp_rem[big], w0 = min(warp, a.nwarps), w1 = min(warp + 1, a.nwarps);
+  u0 = b + a.quantum * (w0 * per + min(w0, rem));
+  u1 = b + a.quantum * (w1 * per + min(w1, rem));
+}
+// unit / G. The product with floor(2^32 / G) is at most one too small: units are below 2^30, so what the
+// rounded reciprocal loses is below 1/4.
+__device__ __forceinline__ int tile_of(const GemvArgs& a, int unit) {
+  const int t = (int)__umulhi((unsigned)unit, a.inv_g);
+  return unit - t * a.G >= a.G ? t + 1 : t;
 }
 
 // x fragment of a lane for the ragged cases (misaligned rows, or the last group when K is not a
@@ -431,16 +442,18 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       if (++at == STAGES) at = 0;
     }
   };
-  auto range_of = [&](const GemvArgs& a, int& u0, int& u1) {
-    warp_range(a.total, a.quantum, a.cta_quantum, a.nctas, a.nwarps, blockIdx.x, warp, u0, u1);
-  };
+  auto range_of = [&](const GemvArgs& a, int& u0, int& u1) { warp_range(a, blockIdx.x, warp, u0, u1); };
 
   // weights never depend on the producer of x: the first stages are requested before the
   // programmatic-dependency wait
+  int u0, u1;
+  range_of(c.job[0], u0, u1);
+  if (lane == 0) fill(c.job[0], u0, u1, 0, min(STAGES, (u1 - u0 + PERW - 1) / PERW), 0);
   {
-    int u0, u1;
-    range_of(c.job[0], u0, u1);
-    if (lane == 0) fill(c.job[0], u0, u1, 0, min(STAGES, (u1 - u0 + PERW - 1) / PERW), 0);
+    // what follows the wait reads these at once: from a cold constant cache that is a memory latency
+    const GemvArgs& a = c.job[0];
+    asm volatile("" ::"l"(a.x), "l"(a.h_in), "l"(a.delta), "l"(a.norm_w), "l"(a.tok), "l"(a.ldx), "l"(a.ldh), "l"(a.ldd),
+                 "r"(a.K), "r"(a.G), "r"(a.o.N), "r"(a.xf16), "r"(a.xvec));
   }
   dep_wait();
 
@@ -448,8 +461,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
   for (int j = 0; j < c.njobs; ++j) {
     const GemvArgs& a = c.job[j];
     const int G = a.G, total = a.total;
-    int u0, u1;
-    range_of(a, u0, u1);
+    if (j) range_of(a, u0, u1);
     if (lane == 0) {
       s_rb[warp] = u0;
       if (warp == NW - 1) s_rb[NW] = u1;
@@ -478,7 +490,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     const bool tail_k = (a.K & 127) != 0;  // the last group reads past K unless guarded
 
     // ---- the stream ----
-    int tile = u0 / G;
+    int tile = tile_of(a, u0);
     int g = u0 - tile * G;   // group of the next unit
     int seg_gb = g;          // first group of the segment held in acc
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -679,8 +691,8 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       if (lane == 0) a.counters[T] = 0;
     };
 
-    if (ok && n_units > 0 && (u1 % G) != 0) {
-      const int T = (u1 - 1) / G;
+    const int T = n_units > 0 ? tile_of(a, u1 - 1) : 0;  // the tile this range ends in
+    if (ok && n_units > 0 && T * G + G != u1) {
       if (T * G >= u0) {  // the head of tile T is in this warp's slot 1
         const int tend = T * G + G;
         float f[4];
@@ -694,8 +706,9 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
         else publish(T, f, cta_e - T * G, 1);
       }
     }
-    if (warp == 0 && ok && cta_e > cta_b && (cta_b % G) != 0) {  // tile that began in an earlier CTA
-      const int T = cta_b / G, tend = T * G + G;
+    const int T0 = tile_of(a, cta_b);
+    if (warp == 0 && ok && cta_e > cta_b && T0 * G != cta_b) {  // tile that began in an earlier CTA
+      const int T = T0, tend = T * G + G;
       float f[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) f[k] = part[k * 32 + lane];
@@ -883,6 +896,15 @@ int make_job(const qe_w4_params* p, const qe_w4_norm* nrm, const qe_w4_cfg* cfg,
   a.nwarps = r.nwarps;
   a.quantum = r.quantum;
   a.cta_quantum = r.cta_quantum;
+  const int quanta = a.total / a.cta_quantum, inner = a.cta_quantum / a.quantum;
+  a.cta_per = quanta / a.nctas;
+  a.cta_rem = quanta % a.nctas;
+  for (int big = 0; big < 2; ++big) {
+    const int mine = (a.cta_per + big) * inner;
+    a.warp_per[big] = mine / a.nwarps;
+    a.warp_rem[big] = mine % a.nwarps;
+  }
+  a.inv_g = (unsigned)std::min<unsigned long long>((1ull << 32) / (unsigned)a.G, 0xFFFFFFFFull);
   a.two_way = r.two_way;
   a.xvec = ((p->ldx & 7) == 0 && aligned16(p->x)) ? 1 : 0;
   *smem_extra = 0;
