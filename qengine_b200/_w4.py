@@ -378,7 +378,7 @@ def auto_ksplit(Mp, Kp, N, warps=8):
 
 
 def ring_error():
-    """Sticky error word of the weight rings' bounded barrier waits (0 = none); synchronises."""
+    """Sticky error word of the bounded waits in the W4 kernels (the GEMM, the grid barrier of a chain; 0 = none); synchronises."""
     return int(lib.qe_w4_ring_error())
 
 

@@ -1,5 +1,5 @@
 // Device-side building blocks of the W4A16 GEMV (w4_gemv.cu): the int4 -> bf16 unpack feeding
-// mma.sync, mbarrier / bulk-copy wrappers for the per-warp weight rings, and the tile epilogues.
+// mma.sync, mbarrier / bulk-copy wrappers (the GEMM uses them), and the tile epilogues.
 //
 // Wire format (python/qengine/quant.py:1-30 of the reference): a matrix is a stream of 1 KB units,
 // unit u = tile * G + g = int4 codes of 16 rows x 128 k, stored as two 512-byte chunks of 32 lanes

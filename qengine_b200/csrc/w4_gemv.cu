@@ -13,10 +13,15 @@
 //   * one CTA per SM, NW warps; the unit stream is cut into one contiguous range per CTA (equal
 //     shares, to within four units) and that range into one contiguous range per warp, so every
 //     warp reads one contiguous slab of HBM and every SM has the same amount of work;
-//   * each warp owns a private ring in shared memory that its lane 0 keeps full with bulk copies
-//     (cp.async.bulk global -> shared, completion on an mbarrier): STAGES x PERW units in flight
-//     per warp, ~130 KB per SM, issued before the programmatic-dependency wait because weights
-//     never depend on the producer of x;
+//   * each warp owns a private ring in shared memory that its lanes keep full with asynchronous copies
+//     (cp.async, 16 bytes per lane, a group per stage): STAGES x PERW units in flight per warp, ~130 KB
+//     per SM, issued before the programmatic-dependency wait because weights never depend on the
+//     producer of x. The copies are the lanes' own and not the copy engine's (cp.async.bulk, two per
+//     stage: codes and scales): a bulk copy holds up its warp for a hundred clocks and more, and a lane
+//     that fetches what it multiplies needs no mbarrier. The four matrices of a 27B layer in order, one
+//     row: 53.6 -> 51.5 us, five rows 61.0 -> 57.7, eight 64.3 -> 60.1. More in flight is slower (3 x 4
+//     units: 55.5 us): it takes L1 from the activations and delays them at the start of a launch; so are
+//     smaller stages (3 x 2 units: 54.3);
 //   * ranges start at multiples of a ring stage whenever a tile is a whole number of stages long,
 //     so a stage never straddles two tiles and its PERW units run as straight-line code: 2 LDS.128
 //     of codes, 2 scales and 4 x 16 B of x per unit at immediate offsets, then the unpack feeding
@@ -39,7 +44,7 @@
 // plus a trip through L2), and CTA 0 writes the updated residual stream to h_out. h_out must not
 // alias h_in: other CTAs may still be reading h_in.
 //
-// Every mbarrier wait is bounded; on expiry the warp records g_w4_error, drains and leaves.
+// The grid barrier of a chain is bounded; on expiry the block records g_w4_error and goes on.
 #include <cuda/atomic>
 
 #include <algorithm>
@@ -99,8 +104,6 @@ struct GemvArgs {
 };
 
 __device__ int g_w4_error = 0;
-
-constexpr int kWaitLimit = 1 << 20;
 
 // The stream is dealt out in quanta of q units, in two levels: equal shares of quanta per CTA
 // (so every SM has the same amount of work to within one quantum), and inside a CTA equal shares
@@ -277,9 +280,10 @@ __device__ __forceinline__ void norm_prologue(const GemvArgs& a, unsigned char* 
 // code is a fraction of the four-row form's. Same thread -> packet map, same order of every sum: same bits.
 template <int NW>
 __device__ __forceinline__ bool one_row_fits(int K) { return K <= 16 * NW * 32; }
-template <int NW>
+// `requested` runs when the row has been asked for.
+template <int NW, typename F>
 __device__ __forceinline__ void norm_prologue_row(const GemvArgs& a, unsigned char* x_s, float* s_red, int tid, int r,
-                                                  bool writer) {
+                                                  bool writer, F requested) {
   constexpr int NT = NW * 32, WP = 2;
   const int npk = a.K >> 3;
   const bf16* row = a.h_in + (long)r * a.ldh;
@@ -298,6 +302,7 @@ __device__ __forceinline__ void norm_prologue_row(const GemvArgs& a, unsigned ch
       wv[i] = reinterpret_cast<const uint4*>(a.norm_w)[p];
     }
   }
+  requested();
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < WP; ++i) {
@@ -357,7 +362,7 @@ __global__ void __launch_bounds__(NW * 32) norm_rows_kernel(const GemvArgs a) {
   dep_wait();
   __shared__ float s_red[QE_MAX_ROWS][NW];
   const int r = blockIdx.x;
-  if (one_row_fits<NW>(a.K)) norm_prologue_row<NW>(a, nullptr, s_red[0], threadIdx.x, r, true);
+  if (one_row_fits<NW>(a.K)) norm_prologue_row<NW>(a, nullptr, s_red[0], threadIdx.x, r, true, [] {});
   else norm_prologue<NW>(a, reinterpret_cast<unsigned char*>(a.xn_out), a.ldxo * 2, s_red, threadIdx.x, r, r + 1, true);
 }
 
@@ -409,7 +414,6 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
   constexpr uint32_t kRing = STAGES * (kStageW + kStageS);
   dep_release();
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t full[NW][STAGES];
   __shared__ int s_rb[NW + 1];
   __shared__ float s_red[QE_MAX_ROWS][NW];
 
@@ -420,27 +424,31 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
   float* part = reinterpret_cast<float*>(smem + (size_t)NW * kRing);  // [NW][2][128]
   unsigned char* x_s = smem + (size_t)NW * kRing + (size_t)NW * 2 * 128 * sizeof(float);
 
-  if (lane == 0) {
-    for (int s = 0; s < STAGES; ++s) bar_init(&full[warp][s], 1);
-    bar_fence_init();
-  }
-  __syncwarp();
+  int slot = 0;  // ring position of the next stage to consume; it runs on across jobs
 
-  // Ring position of the next stage to consume; it runs on across jobs (a slot's barrier
-  // completes one phase per fill, whichever matrix the fill came from).
-  int slot = 0, phase = 0;
-  bool ok = true;
-
-  // lane 0: request stages [st0, st1) of the range [u0, u1) of job `a`, into consecutive ring
-  // slots starting at `at`
+  // Request stages [st0, st1) of the range [u0, u1) of job `a` into consecutive ring slots starting at
+  // `at`: one group of asynchronous copies per stage, an empty one for a stage beyond the range, so that
+  // the number of groups in flight tells which stages have landed. Every lane fetches the 16-byte pieces of
+  // codes that it will multiply, its scales come with other lanes' copies.
+  auto copy16 = [](uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   auto fill = [&](const GemvArgs& a, int u0, int u1, int st0, int st1, int at) {
     for (int st = st0; st < st1; ++st) {
       const int ub = u0 + st * PERW, cnt = min(PERW, u1 - ub);
-      bar_expect(&full[warp][at], (uint32_t)cnt * (1024 + 32));
-      bulk_g2s(ring_w + (size_t)at * kStageW, a.qw + (size_t)ub * 64, (uint32_t)cnt * 1024, &full[warp][at]);
-      bulk_g2s(ring_s + (size_t)at * kStageS, a.scales + (size_t)ub * 16, (uint32_t)cnt * 32, &full[warp][at]);
+      const uint32_t dw = sa(ring_w) + at * kStageW + lane * 16;
+      const uint4* gw = a.qw + (size_t)ub * 64 + lane;
+      for (int i = 0; i < 2 * cnt; ++i) copy16(dw + i * 512, gw + i * 32);
+      if (lane < 2 * cnt) copy16(sa(ring_s) + at * kStageS + lane * 16, a.scales + (size_t)ub * 16 + lane * 8);
+      commit();
       if (++at == STAGES) at = 0;
     }
+  };
+  // the oldest requested stage has landed, in every lane
+  auto await_stage = [] {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    __syncwarp();
   };
   auto range_of = [&](const GemvArgs& a, int& u0, int& u1) { warp_range(a, blockIdx.x, warp, u0, u1); };
 
@@ -448,7 +456,10 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
   // programmatic-dependency wait
   int u0, u1;
   range_of(c.job[0], u0, u1);
-  if (lane == 0) fill(c.job[0], u0, u1, 0, min(STAGES, (u1 - u0 + PERW - 1) / PERW), 0);
+  // A launch that starts with the norm of its row asks for one stage only: the rest of the ring, 68 KB per
+  // SM, would stand in front of that row on its way from L2 (the row took 2.1 us to arrive, 1.5 us so).
+  const bool row_first = c.job[0].h_in && c.job[0].o.N == 1 && one_row_fits<NW>(c.job[0].K);
+  fill(c.job[0], u0, u1, 0, row_first ? 1 : STAGES, 0);
   {
     // what follows the wait reads these at once: from a cold constant cache that is a memory latency
     const GemvArgs& a = c.job[0];
@@ -479,8 +490,13 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     bool xfast;
     if (a.h_in) {
       const long pitch = (long)a.K * 2 + 16;
-      if (a.o.N == 1 && one_row_fits<NW>(a.K)) norm_prologue_row<NW>(a, x_s, s_red[0], tid, 0, blockIdx.x == 0);
-      else norm_prologue<NW>(a, x_s, pitch, s_red, tid, 0, a.o.N, blockIdx.x == 0);
+      if (a.o.N == 1 && one_row_fits<NW>(a.K)) {
+        norm_prologue_row<NW>(a, x_s, s_red[0], tid, 0, blockIdx.x == 0, [&] {
+          if (!j) fill(a, u0, u1, 1, STAGES, 1);
+        });
+      } else {
+        norm_prologue<NW>(a, x_s, pitch, s_red, tid, 0, a.o.N, blockIdx.x == 0);
+      }
       xbase = x_s + xrow * pitch + 32 * t;
       xfast = true;
     } else {
@@ -524,17 +540,12 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
         const unsigned char* xg = xbase + (size_t)g * 256;
         // the next stage to request from HBM: whole stages only in this loop, so the copy sizes are
         // constants and the global addresses advance by constants
-        const unsigned char* gw = reinterpret_cast<const unsigned char*>(a.qw) + (size_t)(u0 + STAGES * PERW) * 1024;
-        const unsigned char* gs = reinterpret_cast<const unsigned char*>(a.scales) + (size_t)(u0 + STAGES * PERW) * 32;
+        const uint4* gw = a.qw + (size_t)(u0 + STAGES * PERW) * 64 + lane;
+        const __half* gs = a.scales + (size_t)(u0 + STAGES * PERW) * 16 + lane * 8;
         int to_request = nstage - STAGES;  // stages not yet requested
   #pragma unroll 1
-        for (int st = 0; st < nstage && ok; ++st) {
-          uint64_t* bar = &full[warp][slot];
-          if (!bar_wait(bar, phase, kWaitLimit)) {
-            ok = false;
-            atomicExch(&g_w4_error, 1);
-            break;
-          }
+        for (int st = 0; st < nstage; ++st) {
+          await_stage();
           unsigned char* stage_w = ring_w + (size_t)slot * kStageW;
           unsigned char* stage_s = ring_s + (size_t)slot * kStageS;
           const uint4* wp = reinterpret_cast<const uint4*>(stage_w) + lane;
@@ -563,28 +574,23 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
             close_segment();
             xg = xbase + (size_t)g * 256;
           }
-          __syncwarp();  // every lane has read this stage: hand its slot back to the copy engine
+          __syncwarp();  // every lane has read this stage: its slot may be filled again
           if (to_request > 0) {
-            if (lane == 0) {
-              async_proxy_fence();
-              bar_expect(bar, kStageW + kStageS);
-              bulk_g2s(stage_w, gw, kStageW, bar);
-              bulk_g2s(stage_s, gs, kStageS, bar);
-            }
-            gw += kStageW;
-            gs += kStageS;
+            const uint32_t dw = sa(stage_w) + lane * 16;
+  #pragma unroll
+            for (int i = 0; i < 2 * PERW; ++i) copy16(dw + i * 512, gw + i * 32);
+            if (lane < 2 * PERW) copy16(sa(stage_s) + lane * 16, gs);
+            gw += PERW * 64;
+            gs += PERW * 16;
             --to_request;
           }
-          if (++slot == STAGES) { slot = 0; phase ^= 1; }
+          commit();
+          if (++slot == STAGES) slot = 0;
         }
       } else {
   #pragma unroll 1
-        for (int st = 0; st < nstage && ok; ++st) {
-          if (!bar_wait(&full[warp][slot], phase, kWaitLimit)) {
-            ok = false;
-            atomicExch(&g_w4_error, 1);
-            break;
-          }
+        for (int st = 0; st < nstage; ++st) {
+          await_stage();
           const uint4* wp = reinterpret_cast<const uint4*>(ring_w + (size_t)slot * kStageW) + lane;
           const unsigned short* sp = reinterpret_cast<const unsigned short*>(ring_s + (size_t)slot * kStageS) + r;
           const int cnt = min(PERW, n_units - st * PERW);
@@ -607,11 +613,8 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
             if (g == G || (st == nstage - 1 && i == cnt - 1)) close_segment();
           }
           __syncwarp();
-          if (lane == 0 && st + STAGES < nstage) {
-            async_proxy_fence();
-            fill(a, u0, u1, st + STAGES, st + STAGES + 1, slot);
-          }
-          if (++slot == STAGES) { slot = 0; phase ^= 1; }
+          fill(a, u0, u1, st + STAGES, st + STAGES + 1, slot);
+          if (++slot == STAGES) slot = 0;
         }
       }
     };
@@ -620,14 +623,11 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
 
     // This warp's ring is empty: ask for the head of its slab of the next matrix now, so that the
     // copies run while the blocks finish this job and meet at the barrier.
-    if (ok && j + 1 < c.njobs) {
+    if (j + 1 < c.njobs) {
       int v0, v1;
       range_of(c.job[j + 1], v0, v1);
       __syncwarp();
-      if (lane == 0) {
-        async_proxy_fence();
-        fill(c.job[j + 1], v0, v1, 0, min(STAGES, (v1 - v0 + PERW - 1) / PERW), slot);
-      }
+      fill(c.job[j + 1], v0, v1, 0, STAGES, slot);
     }
     __syncthreads();  // every partial tile of this CTA is in shared memory, s_rb is complete
 
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     };
 
     const int T = n_units > 0 ? tile_of(a, u1 - 1) : 0;  // the tile this range ends in
-    if (ok && n_units > 0 && T * G + G != u1) {
+    if (n_units > 0 && T * G + G != u1) {
       if (T * G >= u0) {  // the head of tile T is in this warp's slot 1
         const int tend = T * G + G;
         float f[4];
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       }
     }
     const int T0 = tile_of(a, cta_b);
-    if (warp == 0 && ok && cta_e > cta_b && T0 * G != cta_b) {  // tile that began in an earlier CTA
+    if (warp == 0 && cta_e > cta_b && T0 * G != cta_b) {  // tile that began in an earlier CTA
       const int T = T0, tend = T * G + G;
       float f[4];
 #pragma unroll
@@ -719,11 +719,6 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       publish(T, f, min(tend, cta_e) - cta_b, 0);
     }
     if (j + 1 < c.njobs) grid_barrier(c.gbar, gridDim.x);  // also separates the uses of part / s_rb
-  }
-  if (!ok) {
-    // Give the copies that are still in flight a bounded chance to land before the CTA exits.
-    __syncwarp();
-    for (int s = 0; s < STAGES; ++s) bar_wait(&full[warp][s], 0, 1 << 10), bar_wait(&full[warp][s], 1, 1 << 10);
   }
 }
 

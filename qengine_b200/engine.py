@@ -706,7 +706,7 @@ class Engine:
         them where the host synchronises anyway; a set word means the tokens are not to be trusted."""
         bad = []
         if _w4.ring_error():
-            bad.append("W4 weight ring: a bulk copy did not complete")
+            bad.append("W4 kernels: a bounded wait (GEMM barrier, grid barrier of a chain) ran out")
             _w4.clear_error()
             _w4.reset_workspaces()
         if _C.attn_error():
