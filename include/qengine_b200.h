@@ -390,8 +390,8 @@ int qe_w4_pack(const void* w0, const void* w1, int dtype, int M, int K, long ld0
                void* scales, void* stream);
 
 /* The waits of the W4 kernels that depend on another warp or block (the GEMM's barriers, the grid
- * barrier of a chain) are bounded; this returns the sticky error word (0 = no wait ever ran out) after
- * synchronising the device. */
+ * barrier of a chain) are bounded; this returns the sticky error word that they set on expiry (0 = none)
+ * and qe_w4_clear_error resets it. Both synchronise with the device. No counterpart in the reference. */
 int qe_w4_ring_error(void);
 int qe_w4_clear_error(void);
 
