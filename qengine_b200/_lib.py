@@ -104,6 +104,9 @@ SIGNATURES = {
     "qe_w4_clear_error": (c_int, []),
     "qe_w4_gemv_static": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), P]),
     "qe_w4_gemm": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), P]),
+    "qe_w4_norm_rows_wire": (c_int, [C.POINTER(W4Norm), c_int, c_int, C.POINTER(W4Cfg), P]),
+    "qe_w4_rows": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, P]),
+    "qe_w4_rows_bounded": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, c_int, P]),
     "qe_w4_gemm_bounded": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, P]),
     "qe_w4_pack": (c_int, [P, P, c_int, c_int, c_int, c_long, c_long, P, P, P]),
     "qe_w4_plan_gemm": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), C.POINTER(W4Plan)]),

@@ -293,17 +293,17 @@ def gemv_fused(h_in, delta, norm_w, eps, qw, scales, out, M, *, h_out=None, xn_o
 
 
 def norm_rows(h_in, delta, norm_w, eps, xn_out, h_out=None, tok=None, xn16_out=None, warps=0, unroll=0, ksplit=0,
-              pdl=True, variant=0, mode=-1, blocks_per_sm=0, min_units=4):
+              pdl=True, variant=0, mode=-1, blocks_per_sm=0, min_units=4, wire=False):
     """Not in the reference: the prologue of `gemv_fused` as a launch of its own (one block per row),
     bit-identical to it for the same launch options: xn_out = RMSNorm1p(h_in + delta) * (1 + w),
     h_out = bf16(h_in + delta) (may alias h_in). `norm_rows` + `gemv` == `gemv_fused`.
     xn16_out (fp16 [N, K], optional) receives the same rows as fp16: the input of a GEMV job with
-    fp16 activations, which equals `gemv_fused(f16=True)`."""
+    fp16 activations, which equals `gemv_fused(f16=True)`. wire: xn_out in wire order (input of `rows`)."""
     bf = torch.bfloat16
     _req(xn_out.is_cuda and xn_out.dtype == bf and xn_out.dim() == 2 and xn_out.stride(1) == 1, "xn_out bf16 [N, K]")
     N, K = xn_out.shape
-    _req(1 <= N <= MAX_GEMM_ROWS and K % 8 == 0 and norm_w.dtype == bf and norm_w.numel() == K and
-         norm_w.is_contiguous(), "N in 1..64, K % 8 == 0, norm_w [K]")
+    _req(1 <= N <= (MAX_PASS_ROWS if wire else MAX_GEMM_ROWS) and K % 8 == 0 and norm_w.dtype == bf and norm_w.numel() == K and
+         norm_w.is_contiguous(), "N in 1..64 (1..128 in wire order), K % 8 == 0, norm_w [K]")
     _req(h_in.is_cuda and h_in.dtype == bf and h_in.dim() == 2 and h_in.stride(1) == 1 and h_in.size(1) == K, "h_in [*, K]")
     nrm = W4Norm()
     nrm.h_in, nrm.ldh, nrm.norm_w, nrm.eps = h_in.data_ptr(), h_in.stride(0), norm_w.data_ptr(), float(eps)
@@ -325,10 +325,12 @@ def norm_rows(h_in, delta, norm_w, eps, xn_out, h_out=None, tok=None, xn16_out=N
              xn16_out.stride(1) == 1, "xn16_out fp16 [N, K]")
         nrm.xn16_out, nrm.ldx16 = xn16_out.data_ptr(), xn16_out.stride(0)
     cfg = _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units)
-    check(lib.qe_w4_norm_rows(C.byref(nrm), N, K, C.byref(cfg), _stream()), "norm_rows")
+    fn = lib.qe_w4_norm_rows_wire if wire else lib.qe_w4_norm_rows
+    check(fn(C.byref(nrm), N, K, C.byref(cfg), _stream()), "norm_rows")
 
 
-MAX_GEMM_ROWS = 64
+MAX_GEMM_ROWS = 64   # rows of `gemm`
+MAX_PASS_ROWS = 128  # rows of `rows`
 _gemm_scratch: dict[int, tuple] = {}
 
 
@@ -375,6 +377,36 @@ def gemm(x, qw, scales, out, M, swiglu=False, pdl=True, variant=0):
 
 def auto_ksplit(Mp, Kp, N, warps=8):
     return int(lib.qe_w4_auto_ksplit(int(Mp), int(Kp), int(N), int(warps)))
+
+
+def wire_order(x):
+    """The rows of x with every 64-k chunk in the order of the wire format (its own inverse): element
+    16 t + 4 s + j at position 16 s + 4 t + j. Input order of `rows`."""
+    return x.unflatten(-1, (-1, 4, 4, 4)).transpose(-3, -2).reshape(x.shape)
+
+
+def rows(x, qw, scales, out, M, swiglu=False, wire_out=False, warps=0, unroll=0, ksplit=0, pdl=True, variant=0, mode=-1,
+         blocks_per_sm=0, min_units=4):
+    """Not in the reference: `gemv` of N = 1..128 rows with the matrix read once for all of them
+    (qe_w4_rows). Row r of out has the bits of `gemv` of row r with the same options. x is in wire order
+    (`wire_order`), and so is out with wire_out."""
+    for t in (x, qw, scales, out):
+        _req(isinstance(t, torch.Tensor) and t.is_cuda, "CUDA tensors")
+    out_f32 = out.dtype == torch.float32 and not swiglu
+    _req(x.dtype == torch.bfloat16 and (out.dtype == torch.bfloat16 or out_f32), "x bf16, out bf16 (or fp32 sums)")
+    Mp, Kp = _packed(qw, scales)
+    _req(x.dim() == 2 and out.dim() == 2 and x.stride(1) == 1 and out.stride(1) == 1, "x [N,K], out [N,M] rows")
+    N, K, M = x.size(0), x.size(1), int(M)
+    _req(1 <= N <= MAX_PASS_ROWS and out.size(0) == N and out.size(1) == M, "N in 1..128 and out [N, M]")
+    _req(K == Kp, "rows needs K == Kp")
+    _req(x.stride(0) % 8 == 0 and x.stride(0) >= K and x.data_ptr() % 16 == 0, "rows needs 16-byte aligned rows of x")
+    _req((Mp // 2 - 8 < M <= Mp // 2) if swiglu else (Mp - 16 < M <= Mp), "out width must match packed rows")
+    _req(not wire_out or M % 64 == 0, "wire order needs whole 64-k chunks")
+    _req(x.data_ptr() != out.data_ptr(), "in-place not supported")
+    p = W4Params(qw.data_ptr(), scales.data_ptr(), x.data_ptr(), out.data_ptr(), None, None, M, K, Mp, Kp, N,
+                 x.stride(0), out.stride(0), EPI_SWIGLU if swiglu else EPI_NONE, int(out_f32), 0)
+    cfg = _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units)
+    check(lib.qe_w4_rows(C.byref(p), C.byref(cfg), int(bool(wire_out)), _stream()), "w4 rows")
 
 
 def ring_error():

@@ -181,7 +181,15 @@ struct OutDesc {
   int M, N;
   int epi;      // QE_EPI_*
   int out_f32;  // plain epilogue only: unrounded fp32 sums (partial results of a K-split matrix)
+  int wire;     // w4_rows.cu only: columns of a row in the order of the wire format (wire_pos)
 };
+
+// Where element k of a row stands when the row is kept in the order in which the wire format multiplies
+// it: k = 64 c + 16 t + 4 s + j becomes 64 c + 16 s + 4 t + j, so that the 16 k of one mma step (word s of
+// the lanes t) lie side by side. Its own inverse; runs of four stay together.
+__device__ __host__ __forceinline__ int wire_pos(int k) {
+  return (k & ~60) | (k & 12) << 2 | (k >> 2 & 12);
+}
 
 __device__ __forceinline__ float silu_fast(float v) { return v / (1.0f + __expf(-v)); }
 
@@ -230,6 +238,55 @@ __device__ __host__ __forceinline__ int share_owner(int total, int parts, int it
   const int per = total / parts, rem = total - per * parts;
   const int big = rem * (per + 1);
   return item < big ? item / (per + 1) : rem + (item - big) / per;
+}
+
+// How the GEMV deals a matrix's stream of units out: in quanta, in two levels, equal shares per CTA and equal
+// shares of a CTA's quanta per warp. Shape and launch options only, never the row count. The order of a
+// tile's additions follows from it: groups ascending inside a warp's range, a CTA's ranges ascending, then
+// the CTAs ascending.
+struct Deal {
+  int total;        // units
+  int nctas;        // CTAs that own work
+  int nwarps;       // warps of a CTA that own work (small matrices keep min_units per warp)
+  int quantum;      // warp ranges start at multiples of this many units (4 when G % 4 == 0, else 1)
+  int cta_quantum;  // CTA ranges start at multiples of this many units: `quantum`, or G (whole tiles)
+  // Divided out on the host: a division costs a warp some 150 clk, and what happens before a launch's first
+  // weight request and after its last unit is time nothing hides.
+  int cta_per, cta_rem;          // quanta (of cta_quantum units) per CTA; the first cta_rem CTAs hold one more
+  int warp_per[2], warp_rem[2];  // quanta per warp in a CTA of cta_per, and of cta_per + 1, CTA quanta
+};
+__device__ __forceinline__ void warp_range(const Deal& d, int cta, int warp, int& u0, int& u1) {
+  if (cta >= d.nctas) { u0 = u1 = d.total; return; }
+  const int b = d.cta_quantum * (cta * d.cta_per + min(cta, d.cta_rem)), big = cta < d.cta_rem;
+  const int per = d.warp_per[big], rem = d.warp_rem[big], w0 = min(warp, d.nwarps), w1 = min(warp + 1, d.nwarps);
+  u0 = b + d.quantum * (w0 * per + min(w0, rem));
+  u1 = b + d.quantum * (w1 * per + min(w1, rem));
+}
+// A warp range: its CTA and warp, and where it and its CTA's range end.
+struct RangeAt {
+  int cta, warp, end, cta_end;
+};
+__device__ __host__ __forceinline__ void range_bounds(const Deal& d, RangeAt& r) {
+  const int big = r.cta < d.cta_rem, b = d.cta_quantum * (r.cta * d.cta_per + (big ? r.cta : d.cta_rem));
+  const int w = r.warp + 1, rem = d.warp_rem[big];
+  r.cta_end = b + d.cta_quantum * (d.cta_per + big);
+  r.end = b + d.quantum * (w * d.warp_per[big] + (w < rem ? w : rem));
+}
+// ... that holds unit u
+__device__ __host__ __forceinline__ RangeAt range_at(const Deal& d, int u) {
+  RangeAt r;
+  r.cta = share_owner(d.total / d.cta_quantum, d.nctas, u / d.cta_quantum);
+  const int big = r.cta < d.cta_rem, b = d.cta_quantum * (r.cta * d.cta_per + (big ? r.cta : d.cta_rem));
+  const int per = d.warp_per[big], rem = d.warp_rem[big], i = (u - b) / d.quantum, cut = rem * (per + 1);
+  r.warp = i < cut ? i / (per + 1) : rem + (i - cut) / per;
+  range_bounds(d, r);
+  return r;
+}
+// ... the next one (the warps that own nothing are a CTA's last)
+__device__ __host__ __forceinline__ void range_next(const Deal& d, RangeAt& r) {
+  if (r.end == r.cta_end) ++r.cta, r.warp = 0;
+  else ++r.warp;
+  range_bounds(d, r);
 }
 
 }  // namespace w4

@@ -63,6 +63,8 @@ namespace qb {
 // error word of the GEMM's bounded waits (w4_gemm.cu), reported together with the GEMV's
 int gemm_error_read();
 int gemm_error_clear();
+int rows_error_read();  // ... of w4_rows.cu
+int rows_error_clear();
 namespace {
 
 using namespace w4;
@@ -75,21 +77,15 @@ struct GemvArgs {
   OutDesc o;
   float* ws;       // 2 x 128 floats per CTA: partial tiles that cross a CTA boundary
   int* counters;   // one arrival counter per tile, zero on entry, left zero
-  int K, G, total;
-  int nctas;       // CTAs that own work (<= gridDim.x)
-  int nwarps;      // warps of a CTA that own work (small matrices keep min_units per warp)
-  int quantum;     // warp ranges start at multiples of this many units (4 when G % 4 == 0, else 1)
-  int cta_quantum; // CTA ranges start at multiples of this many units: `quantum`, or G (whole tiles)
-  // the deal of the stream, divided out on the host: a division costs a warp some 150 clk, and what
-  // happens before a launch's first weight request and after its last unit is time nothing hides
-  int cta_per, cta_rem;          // quanta (of cta_quantum units) per CTA; the first cta_rem CTAs hold one more
-  int warp_per[2], warp_rem[2];  // quanta per warp in a CTA of cta_per, and of cta_per + 1, CTA quanta
+  int K, G;
+  Deal d;          // the deal of the stream over CTAs and warps
   unsigned inv_g;                // floor(2^32 / G), see tile_of
   int two_way;     // every CTA range holds at least one tile's worth of units: a cut tile has two owners
   int xf16;        // the activations are fp16: `x` points to fp16 rows, or the prologue leaves fp16
                    // in shared memory (the normalised rows, which fp16 holds exactly, see make_job)
   __half* xn16_out;  // norm_rows_kernel only: optional fp16 copy of the normalised rows
   long ldx16;
+  int wire;        // norm_rows_kernel, one row at a time: xn_out in wire order (wire_pos)
   int xvec;        // x rows are 16-byte aligned with ldx % 8 == 0
   // fused residual + RMSNorm prologue (h_in != nullptr)
   const bf16* h_in;
@@ -110,13 +106,6 @@ __device__ int g_w4_error = 0;
 // of its quanta per warp.
 __device__ __host__ __forceinline__ int cta_begin(int total, int q, int nctas, int c) {
   return q * share_begin(total / q, nctas, c);
-}
-__device__ __forceinline__ void warp_range(const GemvArgs& a, int cta, int warp, int& u0, int& u1) {
-  if (cta >= a.nctas) { u0 = u1 = a.total; return; }
-  const int b = a.cta_quantum * (cta * a.cta_per + min(cta, a.cta_rem)), big = cta < a.cta_rem;
-  const int per = a.warp_per[big], rem = a.warp_rem[big], w0 = min(warp, a.nwarps), w1 = min(warp + 1, a.nwarps);
-  u0 = b + a.quantum * (w0 * per + min(w0, rem));
-  u1 = b + a.quantum * (w1 * per + min(w1, rem));
 }
 // unit / G. The product with floor(2^32 / G) is at most one too small: units are below 2^30, so what the
 // rounded reciprocal loses is below 1/4.
@@ -343,7 +332,12 @@ __device__ __forceinline__ void norm_prologue_row(const GemvArgs& a, unsigned ch
       if (x_s) reinterpret_cast<uint4*>(x_s)[p] = a.xf16 ? q16 : q;
       if (writer) {
         if (a.h_out) reinterpret_cast<uint4*>(a.h_out + (long)r * a.ldho)[p] = hv[i];
-        if (a.xn_out) reinterpret_cast<uint4*>(a.xn_out + (long)r * a.ldxo)[p] = q;
+        if (a.xn_out && a.wire) {
+          *reinterpret_cast<uint2*>(a.xn_out + (long)r * a.ldxo + wire_pos(8 * p)) = make_uint2(q.x, q.y);
+          *reinterpret_cast<uint2*>(a.xn_out + (long)r * a.ldxo + wire_pos(8 * p + 4)) = make_uint2(q.z, q.w);
+        } else if (a.xn_out) {
+          reinterpret_cast<uint4*>(a.xn_out + (long)r * a.ldxo)[p] = q;
+        }
         if (a.xn16_out) reinterpret_cast<uint4*>(a.xn16_out + (long)r * a.ldx16)[p] = q16;
       }
     }
@@ -450,7 +444,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
     __syncwarp();
   };
-  auto range_of = [&](const GemvArgs& a, int& u0, int& u1) { warp_range(a, blockIdx.x, warp, u0, u1); };
+  auto range_of = [&](const GemvArgs& a, int& u0, int& u1) { warp_range(a.d, blockIdx.x, warp, u0, u1); };
 
   // weights never depend on the producer of x: the first stages are requested before the
   // programmatic-dependency wait
@@ -471,7 +465,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
 #pragma unroll 1
   for (int j = 0; j < c.njobs; ++j) {
     const GemvArgs& a = c.job[j];
-    const int G = a.G, total = a.total;
+    const int G = a.G, total = a.d.total;
     if (j) range_of(a, u0, u1);
     if (lane == 0) {
       s_rb[warp] = u0;
@@ -535,7 +529,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       // Both loops below walk the ring stage by stage. The fast one serves ranges made of whole
       // stages that never straddle a tile (every matrix of the model): no per-unit decisions at
       // all, every operand at an immediate offset from three base pointers.
-      const bool all_fast = xfast && !tail_k && (a.quantum % PERW) == 0;
+      const bool all_fast = xfast && !tail_k && (a.d.quantum % PERW) == 0;
       if (all_fast) {
         const unsigned char* xg = xbase + (size_t)g * 256;
         // the next stage to request from HBM: whole stages only in this loop, so the copy sizes are
@@ -674,12 +668,12 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       done = __shfl_sync(0xffffffffu, done, 0);  // also orders lane 0's acquire before the loads below
       if (!done) return;
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
-      const int q = a.cta_quantum;
-      const int c_lo = share_owner(total / q, a.nctas, (T * G) / q);
-      const int c_hi = share_owner(total / q, a.nctas, (T * G + G - 1) / q);
+      const int q = a.d.cta_quantum;
+      const int c_lo = share_owner(total / q, a.d.nctas, (T * G) / q);
+      const int c_hi = share_owner(total / q, a.d.nctas, (T * G + G - 1) / q);
 #pragma unroll 1
       for (int cc = c_lo; cc <= c_hi; ++cc) {
-        const int cb = cta_begin(total, q, a.nctas, cc);
+        const int cb = cta_begin(total, q, a.d.nctas, cc);
         float* p = a.ws + ((size_t)cc * 2 + (cb > T * G ? 0 : 1)) * 128;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -805,7 +799,8 @@ const std::vector<ShapeCfg>& env_overrides() {
 struct Resolved {
   qe_w4_plan plan;
   const Geometry* geom;
-  int nctas, nwarps, quantum, cta_quantum, two_way;
+  Deal deal;
+  int two_way;
 };
 
 // Shape-only launch policy (never N): as many warps as there are units / min_units, at most one
@@ -831,18 +826,28 @@ Resolved resolve(const qe_w4_params& p, const qe_w4_cfg& c_in) {
   // small matrices: as many CTAs as possible (every SM pulls from HBM), fewer warps in each
   const long ctas = std::max<long>(1, std::min<long>({ctas_max, want, units / quantum}));
   const long per_cta = (units + ctas - 1) / ctas;
-  r.nwarps = (int)std::max<long>(1, std::min<long>(r.geom->nw, (per_cta + min_units - 1) / min_units));
-  r.quantum = (int)quantum;
+  Deal& d = r.deal;
+  d.total = (int)units;
+  d.nctas = (int)ctas;
+  d.nwarps = (int)std::max<long>(1, std::min<long>(r.geom->nw, (per_cta + min_units - 1) / min_units));
+  d.quantum = (int)quantum;
   // CTA ranges of whole tiles where that costs less than the exchange of cut tiles between CTAs
   // (two global round trips at the end of the launch, about a microsecond): the surplus of the
   // fullest CTA over the even share, at about 30 ns per unit, must stay well below that. Decided
   // from the shape alone, like everything else in the plan.
   const long tiles_max = (tiles + ctas - 1) / ctas;
   const bool whole_tiles = ctas > 1 && tiles >= ctas && (tiles_max * ctas - tiles) * G <= 26 * ctas;
-  r.cta_quantum = whole_tiles ? (int)G : (int)quantum;
+  d.cta_quantum = whole_tiles ? (int)G : (int)quantum;
+  const int quanta = d.total / d.cta_quantum, inner = d.cta_quantum / d.quantum;
+  d.cta_per = quanta / d.nctas;
+  d.cta_rem = quanta % d.nctas;
+  for (int big = 0; big < 2; ++big) {
+    const int mine = (d.cta_per + big) * inner;
+    d.warp_per[big] = mine / d.nwarps;
+    d.warp_rem[big] = mine % d.nwarps;
+  }
   // the smallest CTA range in units; at least a tile long means no tile has three owners
-  r.two_way = ((units / r.cta_quantum) / ctas) * r.cta_quantum >= G ? 1 : 0;
-  r.nctas = (int)ctas;
+  r.two_way = ((units / d.cta_quantum) / ctas) * d.cta_quantum >= G ? 1 : 0;
   r.plan.mode = 4;
   r.plan.grid_x = (int)ctas;
   r.plan.grid_y = 1;
@@ -886,21 +891,9 @@ int make_job(const qe_w4_params* p, const qe_w4_norm* nrm, const qe_w4_cfg* cfg,
   a.counters = p->counters;
   a.K = p->K;
   a.G = p->Kp / 128;
-  a.total = (p->Mp / 16) * a.G;
-  a.nctas = r.nctas;
-  a.nwarps = r.nwarps;
-  a.quantum = r.quantum;
-  a.cta_quantum = r.cta_quantum;
-  const int quanta = a.total / a.cta_quantum, inner = a.cta_quantum / a.quantum;
-  a.cta_per = quanta / a.nctas;
-  a.cta_rem = quanta % a.nctas;
-  for (int big = 0; big < 2; ++big) {
-    const int mine = (a.cta_per + big) * inner;
-    a.warp_per[big] = mine / a.nwarps;
-    a.warp_rem[big] = mine % a.nwarps;
-  }
-  a.inv_g = (unsigned)std::min<unsigned long long>((1ull << 32) / (unsigned)a.G, 0xFFFFFFFFull);
+  a.d = r.deal;
   a.two_way = r.two_way;
+  a.inv_g = (unsigned)std::min<unsigned long long>((1ull << 32) / (unsigned)a.G, 0xFFFFFFFFull);
   a.xvec = ((p->ldx & 7) == 0 && aligned16(p->x)) ? 1 : 0;
   *smem_extra = 0;
   if (nrm && nrm->h_in) {
@@ -988,6 +981,10 @@ int launch_chain(const qe_w4_params* const* ps, const qe_w4_norm* const* nrms, i
 }
 
 }  // namespace
+
+// How the GEMV of this matrix orders its additions (w4_rows.cu adds in the same order).
+w4::Deal gemv_deal(const qe_w4_params& p, const qe_w4_cfg& c) { return resolve(p, c).deal; }
+
 }  // namespace qb
 
 using namespace qb;
@@ -1021,15 +1018,16 @@ extern "C" int qe_w4_ring_error(void) {
   int v = 0;
   if (cudaDeviceSynchronize() != cudaSuccess) return -1;
   if (cudaMemcpyFromSymbol(&v, g_w4_error, sizeof(int)) != cudaSuccess) return -1;
-  const int m = gemm_error_read();
-  if (m < 0) return -1;
-  return v | (m ? 16 * m : 0);
+  const int m = gemm_error_read(), n = rows_error_read();
+  if (m < 0 || n < 0) return -1;
+  return v | 16 * m | 256 * n;
 }
 
 extern "C" int qe_w4_clear_error(void) {
   const int z = 0;
   if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-  const int rc = gemm_error_clear();
+  int rc = gemm_error_clear();
+  if (!rc) rc = rows_error_clear();
   if (rc) return rc;
   return (int)cudaMemcpyToSymbol(g_w4_error, &z, sizeof(int));
 }
@@ -1055,8 +1053,9 @@ extern "C" int qe_w4_gemv_ex(const qe_w4_params* p, const qe_w4_norm* nrm, const
   return launch_chain(&p, &nrm, 1, cfg, nullptr, (cudaStream_t)stream);
 }
 
-extern "C" int qe_w4_norm_rows(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, void* stream) {
-  if (!nrm || !cfg || N < 1 || N > QE_MAX_GEMM_ROWS || K < 8 || (K & 7) || !nrm->h_in || !nrm->norm_w || !nrm->xn_out)
+namespace {
+int norm_rows(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, bool wire, void* stream) {
+  if (!nrm || !cfg || N < 1 || N > (wire ? QE_MAX_PASS_ROWS : QE_MAX_GEMM_ROWS) || K < 8 || (K & 7) || !nrm->h_in || !nrm->norm_w || !nrm->xn_out)
     return QE_ERR_ARG;
   if (!aligned16(nrm->h_in) || !aligned16(nrm->norm_w) || !aligned16(nrm->xn_out) || (nrm->ldh & 7) || (nrm->ldxo & 7) ||
       (nrm->xn16_out && (!aligned16(nrm->xn16_out) || (nrm->ldx16 & 7))) ||
@@ -1082,6 +1081,8 @@ extern "C" int qe_w4_norm_rows(const qe_w4_norm* nrm, int N, int K, const qe_w4_
   }
   const bool pdl = cfg->pdl && pdl_launch_enabled() && pdl_trigger_enabled();
   const int nw = pick_geometry(*cfg).nw;  // the reduction order follows the CTA size of the GEMV
+  if (wire && (K % 64 || K > 16 * nw * 32)) return QE_ERR_ARG;  // whole chunks, rows that a block holds in registers
+  a.wire = wire ? 1 : 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (nw) {
     case 8: return (int)launch(norm_rows_kernel<8>, dim3(N), dim3(256), 0, s, pdl, a);
@@ -1089,6 +1090,15 @@ extern "C" int qe_w4_norm_rows(const qe_w4_norm* nrm, int N, int K, const qe_w4_
     case 24: return (int)launch(norm_rows_kernel<24>, dim3(N), dim3(768), 0, s, pdl, a);
     default: return (int)launch(norm_rows_kernel<20>, dim3(N), dim3(640), 0, s, pdl, a);
   }
+}
+}  // namespace
+
+extern "C" int qe_w4_norm_rows(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, void* stream) {
+  return norm_rows(nrm, N, K, cfg, false, stream);
+}
+
+extern "C" int qe_w4_norm_rows_wire(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, void* stream) {
+  return norm_rows(nrm, N, K, cfg, true, stream);
 }
 
 extern "C" int qe_w4_gemv_chain(const qe_w4_params* const* p, const qe_w4_norm* const* nrm, int njobs,

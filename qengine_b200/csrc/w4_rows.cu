@@ -1,0 +1,490 @@
+// W4A16 product for up to 128 activation rows with the GEMV's bits (sm_100a): every matrix is read once for
+// all rows of a prefill pass, and row r of the result equals qe_w4_gemv of that row, bit for bit.
+//
+//   out[n, m] = bf16( sum_g fp32(scale[m, g]) * sum_{k in group g} (code[m, k] - 8) * x[n, k] )
+//
+// No counterpart in the reference, which prefills in passes of at most 8 rows through its GEMV
+// (python/qengine/engine.py:558-573).
+//
+// Why the bits agree. One group's sum is a chain of eight tensor-core products of 16 k each. tcgen05.mma and
+// mma.sync leave the same fp32 sum when each step multiplies the same 16 k (measured: 15.7 million sums of
+// rows with exponents from -60 to 60, none differs; with the 16 k of a step in another order a third do). The
+// GEMV's step s of a 64-k chunk takes word s of the four lanes of a row pair, k = 16 t + 4 s + 0..3; so the
+// weights go into tensor memory word by word, as they are stored, and the activations come with each 64-k
+// chunk in that order (wire_pos): what produces them writes them so. Between groups the order of the
+// additions is the GEMV's deal of the unit stream (w4_dev.cuh, Deal): a warp's range of groups ascending,
+// then the ranges of a CTA, then the CTAs. Here one thread adds all of it, and closes a partial sum where a
+// range ends (range_end).
+//
+// Design: the tensor-memory GEMM of w4_gemm.cu (unpacking warps, one issuing thread, drain warps, coupled by
+// mbarriers) with another walk. A job is one super-tile of 128 weight rows over the whole of K and all
+// activation rows, or over a part of the columns where there are fewer super-tiles than half the SMs: a split
+// along K would close partial sums where the GEMV does not. Eight drain warps read each product, four the
+// first half of its columns and four the second: 64 sums per thread at 128 rows. Tensor memory: D in two
+// stages of 128 columns (four of 64 where that is enough), A in four of 64.
+//   * What bounds it: hand-over latency, as in w4_gemm.cu: a step (one group of a super-tile) costs some
+//     900-1100 clk whatever its rows, half of it the unpack (888 clk: 260 instructions of each of four
+//     warps), and unpack, issue and drain wait for one another. Hence 128 rows and not 64.
+// Every wait is bounded (see w4_gemm.cu).
+#include <algorithm>
+
+#include "w4_tc.cuh"
+
+namespace qb {
+w4::Deal gemv_deal(const qe_w4_params& p, const qe_w4_cfg& c);  // w4_gemv.cu
+namespace {
+
+using namespace w4;
+
+struct RowsArgs {
+  const uint4* qw;
+  const __half* scales;
+  OutDesc o;  // o.N = all activation rows
+  Deal d;
+  int G, tiles;
+  int cparts, cols;  // parts the columns (activation rows) are split into, columns of a part (a multiple of 16)
+  int wait_limit;
+};
+
+__device__ int g_rows_error = 0;
+
+constexpr int kThreads = 18 * 32, kAhead = 3, kB = 4;
+constexpr uint32_t kBStage = 128 * 256;  // 128 rows x 128 k
+constexpr uint32_t kPitch = 132;         // floats per column of the staging: 128 rows of the super-tile + 4
+constexpr int kChunk = 16;               // groups per request of scales
+constexpr uint32_t kScaleBytes = kChunk * 32;  // of one tile
+constexpr uint32_t kSmem = kB * kBStage + 128 * kPitch * sizeof(float) + 12 * 2 * 2 * kScaleBytes + 1024;
+static_assert(kB == 4, "the barriers `done` guard the stages of A and of B");
+static_assert(kSmem + 512 <= 227 * 1024, "shared memory of one block");
+constexpr uint32_t kACol = 256;  // tensor memory: D in columns 0..255, A in 256..511
+
+// rows x 128 k of the activations from row y: two 64-k chunks from chunk c
+__device__ __forceinline__ void tma_step(uint32_t dst, const CUtensorMap* map, int y, int c, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(map), "r"(0), "r"(y), "r"(c), "r"(sa(bar))
+      : "memory");
+}
+
+// 16 columns of D into registers: asked for, and (with every request before) arrived.
+__device__ __forceinline__ void ld16_ask(uint32_t taddr, uint32_t (&u)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+        "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void ld16_wait(uint32_t (&u)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]), "+r"(u[6]), "+r"(u[7]),
+                 "+r"(u[8]), "+r"(u[9]), "+r"(u[10]), "+r"(u[11]), "+r"(u[12]), "+r"(u[13]), "+r"(u[14]), "+r"(u[15])
+               :
+               : "memory");
+}
+
+// kU groups of four unpacking warps, which alternate steps; kP groups of four drain warps, which share the
+// columns. 1, 3: up to 128 columns, 48 sums per thread, and one group of unpacking warps keeps up with
+// them. 2, 2: up to 64 columns, where the unpack is the longer turn.
+template <int kU, int kP>
+__global__ void __launch_bounds__(kThreads, 1)
+    w4_rows_kernel(const __grid_constant__ RowsArgs a, const __grid_constant__ CUtensorMap xmap) {
+  constexpr int kDrain = 4 * kP, kBlocks = kP == 3 ? 3 : 2;  // drain warps; 16-column blocks of one of them
+  constexpr bool kPipe = kP == 2;
+  static_assert(2 + kDrain + 4 * kU == kThreads / 32, "warps");
+  dep_release();
+  extern __shared__ unsigned char smem_raw[];
+  // step may be multiplied: its A is stored (one arrival per unpacking warp), its B has landed (one), and the
+  // D of the step nd before has been read (one per drain warp)
+  __shared__ uint64_t ready[4];
+  __shared__ uint64_t done[4];    // its products are complete (tcgen05.commit): D readable, A and B free
+  __shared__ uint64_t b_full[kB];    // its activations have landed
+  __shared__ uint64_t s_full[kDrain][2];  // a drain warp's next scales have landed
+  __shared__ uint32_t tmem_slot;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned char* Bbase = smem_raw + ((1024u - (sa(smem_raw) & 1023u)) & 1023u);  // swizzle atoms: 1 KB aligned
+
+  if (warp == 1) {  // one barrier per lane
+    if (lane < 4) bar_init(&ready[lane], 4 + 1 + kDrain);
+    else if (lane < 8) bar_init(&done[lane - 4], 1);
+    else if (lane < 8 + kB) bar_init(&b_full[lane - 8], 1);
+    if (lane < 2 * kDrain) bar_init(&s_full[lane >> 1][lane & 1], 1);
+    bar_fence_init();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+
+  // ---- this CTA's jobs: (super-tile, part of the columns), dealt out round-robin ----
+  const int G = a.G, N = a.o.N, CP = a.cparts;
+  const int J = ((a.tiles + 7) >> 3) * CP;
+  const int cta = blockIdx.x, nctas = gridDim.x;
+  const int nj = cta < J ? (J - cta + nctas - 1) / nctas : 0, V = nj * G;  // jobs, steps
+  auto tile0_of = [&](int j) { return (cta + j * nctas) / CP * 8; };
+  auto col0_of = [&](int j) { return (cta + j * nctas) % CP * a.cols; };
+  auto blocks_of = [&](int j) { return (min(a.cols, N - col0_of(j)) + 15) >> 4; };  // of 16 columns
+
+  const int q = warp & 3;  // quarter of the tensor-memory lanes this warp can reach
+  // Unpacking warps: a cursor over the group's steps
+  const int grp = kU > 1 ? (warp - kDrain - 1) >> 2 : 0;
+  int cj = 0, cg = grp;  // job, group of the step
+  const uint4* cp = a.qw;
+  long second = 0;  // distance of the second tile's unit (0: beyond the matrix, never stored)
+  auto enter = [&] {
+    while (cg >= G) cg -= G, ++cj;
+    if (cj >= nj) return;
+    const int tile = min(tile0_of(cj) + 2 * q, a.tiles - 1);
+    cp = a.qw + ((long)tile * G + cg) * 64 + lane;
+    second = tile + 1 < a.tiles ? (long)G * 64 : 0;
+  };
+  uint4 wreg[kAhead][4];
+  auto load_next = [&](uint4 (&w)[4]) {  // request the own step under the cursor and move on
+    if (cj >= nj) return;
+    w[0] = ld_codes(cp);
+    w[1] = ld_codes(cp + 32);
+    w[2] = ld_codes(cp + second);
+    w[3] = ld_codes(cp + second + 32);
+    cp += kU * 64;
+    cg += kU;
+    if (cg >= G) enter();
+  };
+  if (warp > kDrain && warp <= kDrain + 4 * kU) {  // weights never depend on the kernel before: requested before anything is waited for
+    enter();
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) load_next(wreg[i]);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  const uint32_t half_bytes = (uint32_t)a.cols * 128;  // one 64-k chunk of a stage of B
+  const int nd = a.cols > 64 ? 2 : 4, dcols = 256 / nd;  // stages of D, columns of a stage
+
+  if (warp == 0) {
+    // ---- the issuing warp ----
+    const uint64_t db0 = tc_desc(sa(Bbase));
+    dep_wait();  // before the first bounded wait: its limit is not for the producer of x to use up
+    if (elect_one()) {
+      int v = 0;
+      bool ok = true;
+#pragma unroll 1
+      for (int j = 0; j < nj && ok; ++j) {
+        const uint32_t idesc =
+            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(blocks_of(j) * 2) << 17) | ((128u >> 4) << 24);
+#pragma unroll 1
+        for (int g = 0; g < G; ++g, ++v) {
+          const int s = v & 3;
+          ok = bar_wait(&ready[s], (v >> 2) & 1, a.wait_limit);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t d = tmem + (v & (nd - 1)) * dcols, ac = tmem + kACol + s * 64;
+          const uint64_t db = db0 + (uint64_t)(s * (kBStage >> 4));
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            tc_mma(d, ac + 8 * k, db + (uint64_t)((k >> 2) * (half_bytes >> 4) + (k & 3) * 2), idesc, k ? 1u : 0u);
+          tc_commit(&done[s]);
+        }
+      }
+      if (!ok) atomicExch(&g_rows_error, 2);
+      // The products in flight, which drain warps that gave up have not waited for.
+      if (v > 0) bar_wait(&done[(v - 1) & 3], ((v - 1) >> 2) & 1, kGemmWaitLimit);
+    }
+    __syncwarp();
+  } else if (warp == kDrain + 4 * kU + 1) {
+    // ---- the warp that asks for the activations, a step per request, kB ahead (a request holds its warp up
+    // for some hundred clocks), and passes on that they have landed ----
+    dep_wait();
+    if (elect_one()) {
+      int z = 0, landed = 0;
+      bool ok = true;
+      auto pass_on = [&] {
+        ok = bar_wait(&b_full[landed & (kB - 1)], (landed / kB) & 1, a.wait_limit);
+        if (ok) bar_arrive(&ready[landed & 3]);
+        ++landed;
+      };
+#pragma unroll 1
+      for (int j = 0; j < nj && ok; ++j) {
+#pragma unroll 1
+        for (int g = 0; g < G && ok; ++g) {
+          uint64_t* const bar = &b_full[z & (kB - 1)];
+          // the products that read the stage before are complete
+          if (z >= kB) ok = bar_wait(&done[z & (kB - 1)], (z / kB - 1) & 1, a.wait_limit);
+          if (!ok) break;
+          bar_expect(bar, 2 * half_bytes);
+          tma_step(sa(Bbase) + (z & (kB - 1)) * kBStage, &xmap, col0_of(j), 2 * g, bar);
+          ++z;
+          if (z > 1) pass_on();  // of the request before: the products need not wait for the next one's stage
+        }
+      }
+      while (landed < z && ok) pass_on();
+      if (!ok) atomicExch(&g_rows_error, 16);
+      // Shared memory may not be left with copies on their way.
+      for (int l = max(z - kB, 0); l < z; ++l) bar_wait(&b_full[l & (kB - 1)], (l / kB) & 1, kGemmWaitLimit);
+    }
+    __syncwarp();
+  } else if (warp > kDrain) {
+    // ---- unpacking warps ----
+    const uint32_t t_lane = tmem + kACol + ((uint32_t)(32 * q) << 16);
+    bool ok = true;
+#pragma unroll 1
+    for (int v0 = grp; v0 < V && ok; v0 += kU * kAhead) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int v = v0 + kU * i, s = v & 3;
+        if (v >= V || !ok) break;
+        // The stage of A is free when the products of step v - 4 are complete. A lone group asks for two steps at
+        // once (a wait costs it 270 clk even when there is nothing to wait for): products complete in order.
+        const int z = kU == 1 ? v - 3 : v - 4;
+        if (v >= 4 && (kU > 1 || !(v & 1))) {
+          if (v < 4 + kU) dep_wait();  // before the first bounded wait, as in the issuing warp
+          if (!warp_wait(&done[z & 3], (z >> 2) & 1, a.wait_limit)) {
+            ok = false;
+            atomicExch(&g_rows_error, 1);
+            break;
+          }
+        }
+        tc_fence_after();
+        const uint32_t t0 = t_lane + s * 64;
+        tc_st_chunk(t0, wreg[i][0]);
+        tc_st_chunk(t0 + 32, wreg[i][1]);
+        tc_st_chunk(t0 + (16u << 16), wreg[i][2]);
+        tc_st_chunk(t0 + (16u << 16) + 32, wreg[i][3]);
+        load_next(wreg[i]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(&ready[s]);
+      }
+    }
+  } else {
+    // ---- drain warps ----
+    const int wd = warp - 1;
+    const int m = 32 * q + lane;  // this thread's row of a super-tile
+    const uint32_t t_lane = tmem + ((uint32_t)(32 * q) << 16);
+    float* const stage = reinterpret_cast<float*>(Bbase + kB * kBStage);  // [128 columns][kPitch]
+    // Scales of the warp's two tiles (its 32 rows), kChunk groups at a time, two requests ahead.
+    unsigned char* const scales = Bbase + kB * kBStage + 128 * kPitch * sizeof(float) + wd * 4 * kScaleBytes;
+    int sj = 0, sg = 0, snext = 0;  // job, first group and number of the next request
+    auto request_scales = [&] {
+      if (sj >= nj) return;
+      const int n = min(kChunk, G - sg);
+      if (elect_one()) {
+        const int tile = tile0_of(sj) + 2 * q;
+        unsigned char* dst = scales + (snext & 1) * 2 * kScaleBytes;
+        uint64_t* bar = &s_full[wd][snext & 1];
+        const __half* src = a.scales + ((size_t)min(tile, a.tiles - 1) * G + sg) * 16;
+        bar_expect(bar, 2 * n * 32);
+        bulk_g2s(dst, src, n * 32, bar);
+        bulk_g2s(dst + kScaleBytes, tile + 1 < a.tiles ? src + (size_t)G * 16 : src, n * 32, bar);
+      }
+      __syncwarp();
+      ++snext;
+      sg += kChunk;
+      if (sg >= G) sg = 0, ++sj;
+    };
+    request_scales();  // constant like the weights: before the wait
+    request_scales();
+    auto sync_all = [&] { asm volatile("bar.sync 3, %0;" ::"n"(kDrain * 32) : "memory"); };
+
+    dep_wait();
+    if (lane == 0) {  // nothing to read out of D yet
+      for (int s = 0; s < nd; ++s) bar_arrive(&ready[s]);
+    }
+
+    bool ok = true;
+    int v = 0, chunk = 0;  // step, request of scales
+#pragma unroll 1
+    for (int j = 0; j < nj; ++j) {
+      const int nb = blocks_of(j), each = (nb + kP - 1) / kP;  // the warps of a quarter share the columns
+      const int blocks = min(each, max(0, nb - each * (wd >> 2))), col0 = 16 * each * (wd >> 2);
+      float* const mine = stage + col0 * kPitch + m;  // sums of the ranges closed so far
+      float* const older = mine + 64 * kPitch;        // ... of the CTAs closed so far (at most 64 columns then)
+      float acc[16 * kBlocks];
+#pragma unroll
+      for (int k = 0; k < 16 * kBlocks; ++k) acc[k] = 0.f;
+      // the range of the GEMV that this row's tile begins in, and the group at which it ends
+      const int unit0 = (tile0_of(j) + (m >> 4)) * G;
+      RangeAt at = range_at(a.d, min(unit0, a.d.total - 1));
+      int next = unit0 < a.d.total ? at.end - unit0 : G;  // (a tile beyond the matrix is never stored)
+      bool some = false, some_older = false;
+      if (j) sync_all();  // the job before is stored: the staging may be written
+      int i = 0;
+#pragma unroll 1
+      for (int c0 = 0; c0 < G; c0 += kChunk, ++chunk) {
+        if (!ok) break;
+        if (!warp_wait(&s_full[wd][chunk & 1], (chunk >> 1) & 1, a.wait_limit)) {
+          ok = false;
+          if (lane == 0) atomicExch(&g_rows_error, 8);
+          break;
+        }
+        const __half* const sc = reinterpret_cast<const __half*>(scales + ((chunk & 1) * 2 + (lane >> 4)) * kScaleBytes) +
+                                 (lane & 15) - c0 * 16;
+        const int end = min(c0 + kChunk, G);
+#pragma unroll 1
+        for (; i < end && ok; ++i, ++v) {
+          if (i == next) {  // a range of the GEMV ends here: its partial sum is closed
+            if (at.end == at.cta_end) {
+#pragma unroll
+              for (int k = 0; k < 16 * kBlocks; ++k) {
+                if ((k >> 4) >= blocks) break;
+                const float t = (some ? mine[k * kPitch] : 0.f) + acc[k];
+                older[k * kPitch] = (some_older ? older[k * kPitch] : 0.f) + t;
+                acc[k] = 0.f;
+              }
+              some = false;
+              some_older = true;
+            } else {
+#pragma unroll
+              for (int k = 0; k < 16 * kBlocks; ++k) {
+                if ((k >> 4) >= blocks) break;
+                mine[k * kPitch] = (some ? mine[k * kPitch] : 0.f) + acc[k];
+                acc[k] = 0.f;
+              }
+              some = true;
+            }
+            range_next(a.d, at);
+            next = at.end - unit0;
+          }
+          const int s = v & 3;
+          const float scale = __half2float(sc[i * 16]);
+          if (!warp_wait(&done[s], (v >> 2) & 1, a.wait_limit)) {
+            ok = false;
+            if (lane == 0) atomicExch(&g_rows_error, 4);
+            break;
+          }
+          tc_fence_after();
+          const uint32_t t0 = t_lane + (v & (nd - 1)) * dcols + col0;
+          uint32_t u[kPipe ? 2 : 1][16];
+          if (kPipe && blocks > 0) ld16_ask(t0, u[0]);
+#pragma unroll
+          for (int h = 0; h < kBlocks; ++h) {
+            if (h >= blocks) break;
+            if (!kPipe) ld16_ask(t0 + 16 * h, u[0]);
+            ld16_wait(u[kPipe ? h & 1 : 0]);
+            if (kPipe && h + 1 < kBlocks && h + 1 < blocks) ld16_ask(t0 + 16 * (h + 1), u[kPipe ? (h + 1) & 1 : 0]);  // on its way meanwhile
+#pragma unroll
+            for (int k = 0; k < 16; k += 2) {
+              float* const to = acc + 16 * h + k;
+              const float2 sum = fma2(make_float2(scale, scale),
+                                      make_float2(__uint_as_float(u[kPipe ? h & 1 : 0][k]), __uint_as_float(u[kPipe ? h & 1 : 0][k + 1])),
+                                      make_float2(to[0], to[1]));
+              to[0] = sum.x, to[1] = sum.y;
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) bar_arrive(&ready[(v + nd) & 3]);
+        }
+        if (!ok) break;
+        __syncwarp();  // every lane has read its scales
+        request_scales();
+      }
+#pragma unroll
+      for (int k = 0; k < 16 * kBlocks; ++k) {
+        if ((k >> 4) >= blocks) break;
+        float t = acc[k];
+        if (some) t = mine[k * kPitch] + t;
+        if (some_older) t = older[k * kPitch] + t;
+        mine[k * kPitch] = t;
+      }
+      // read again after the loops: kept over them, the output's description takes the sums' registers
+      const RowsArgs* late = &a;
+      asm volatile("" : "+l"(late));
+      sync_all();
+      if (ok) {
+        OutDesc o = late->o;
+        const int c0 = col0_of(j);
+        o.out = static_cast<unsigned char*>(o.out) + (size_t)c0 * o.ldo * (o.out_f32 ? 4 : 2);
+        o.N = min(late->cols, o.N - c0);
+        tc_store(o, tile0_of(j), tid - 32, kDrain * 32,
+                 [&](int n, int m0) { return *reinterpret_cast<const float4*>(stage + n * kPitch + m0); });
+      }
+    }
+    if (!ok) {
+      // Shared memory may not be left with copies on their way: the last request of scales per slot.
+      for (int r = max(snext - 2, 0); r < snext; ++r) bar_wait(&s_full[wd][r & 1], (r >> 1) & 1, kGemmWaitLimit);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+}  // namespace
+
+// Error word of the bounded waits above, for qe_w4_ring_error / qe_w4_clear_error (w4_gemv.cu).
+int rows_error_read() {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_rows_error, sizeof(int)) != cudaSuccess) return -1;
+  return v;
+}
+int rows_error_clear() {
+  const int z = 0;
+  return (int)cudaMemcpyToSymbol(g_rows_error, &z, sizeof(int));
+}
+
+}  // namespace qb
+
+using namespace qb;
+
+extern "C" int qe_w4_rows(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, void* stream) {
+  return qe_w4_rows_bounded(p, cfg, wire_out, kGemmWaitLimit, stream);
+}
+
+extern "C" int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, int wait_limit, void* stream) {
+  if (!p || !cfg || wait_limit < 0) return QE_ERR_ARG;
+  if (p->N < 1 || p->N > QE_MAX_PASS_ROWS || p->Mp % 16 || p->Kp % 128 || p->Mp <= 0 || p->Kp <= 0) return QE_ERR_ARG;
+  if (p->K != p->Kp || p->M <= 0 || p->x_f16 || !p->x || !p->out) return QE_ERR_ARG;
+  if (p->epilogue == QE_EPI_SWIGLU ? p->M > p->Mp / 2 : p->M > p->Mp) return QE_ERR_ARG;
+  if (p->epilogue != QE_EPI_NONE && p->epilogue != QE_EPI_SWIGLU) return QE_ERR_ARG;
+  if ((long)(p->Mp / 16) * (p->Kp / 128) >= (1L << 30)) return QE_ERR_ARG;
+  if (!aligned16(p->qw) || !aligned16(p->scales) || !aligned16(p->x) || (p->ldx & 7)) return QE_ERR_ARG;
+  if (wire_out && p->M % 64) return QE_ERR_ARG;  // only whole 64-k chunks have a wire order
+  static bool allowed[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+  if (!allowed[dev]) {
+    e = cudaFuncSetAttribute(w4_rows_kernel<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(w4_rows_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return (int)e;
+    allowed[dev] = true;
+  }
+  RowsArgs a{};
+  a.qw = reinterpret_cast<const uint4*>(p->qw);
+  a.scales = reinterpret_cast<const __half*>(p->scales);
+  a.o.out = p->out;
+  a.o.ldo = p->ldo;
+  a.o.M = p->M;
+  a.o.N = p->N;
+  a.o.epi = p->epilogue;
+  a.o.out_f32 = (p->out_f32 && p->epilogue == QE_EPI_NONE) ? 1 : 0;
+  a.o.wire = wire_out ? 1 : 0;
+  a.G = p->Kp / 128;
+  a.tiles = p->Mp / 16;
+  a.wait_limit = wait_limit;
+  a.d = gemv_deal(*p, *cfg);
+  // Few super-tiles: parts of the columns, as many as there are SMs for, so that every SM has a job. Tiles
+  // that the GEMV cuts between CTAs need room for a second level of sums: 64 columns at most.
+  const int ST = (a.tiles + 7) / 8, sms = qe_sm_count(), n16 = (p->N + 15) / 16;
+  int parts = ST * 2 > sms ? 1 : std::min(sms / ST, n16);
+  if (a.d.cta_quantum != a.G) parts = std::max(parts, (n16 + 3) / 4);
+  a.cols = 16 * ((n16 + parts - 1) / parts);
+  a.cparts = (p->N + a.cols - 1) / a.cols;
+  CUtensorMap map{};
+  if (!map_rows(p, a.cols, 2, &map)) return QE_ERR_ARG;
+  const bool pdl = cfg->pdl && pdl_launch_enabled() && pdl_trigger_enabled();
+  return (int)launch(a.cols > 64 ? w4_rows_kernel<1, 3> : w4_rows_kernel<2, 2>, dim3(std::min(sms, ST * a.cparts)), dim3(kThreads), kSmem, (cudaStream_t)stream, pdl,
+                     a, map);
+}

@@ -333,7 +333,7 @@ class Engine:
         self.truth = torch.zeros(1, dtype=I32, device=self.dev)
         self.l2_win = None      # (base, bytes) of the persisting window around the draft phase
         self.wide_prefill = bool(wide_prefill)
-        self.wb = None          # buffers of the wide prefill passes (allocated on first use)
+        self.wb = self.rb = None  # buffers of the passes of up to 64 / 128 rows (allocated on first use)
 
     @classmethod
     def from_cache(cls, path, cache_dir, device="cuda", linear=None, **kw):
@@ -748,8 +748,9 @@ class Engine:
         fit = self.WIDE_PART_BYTES // (c.hq * self.ATTN_SPLITS * c.head_dim * 4)
         return max(NMAX, min(self.WIDE, fit // NMAX * NMAX))
 
-    def _make_wide_buffers(self):
-        c, dev, W, H = self.cfg, self.dev, self.WIDE, self.cfg.hidden
+    def _pass_buffers(self, W):
+        """Buffers of a pass of up to W rows."""
+        c, dev, H = self.cfg, self.dev, self.cfg.hidden
 
         def buf(*shape, dt=BF16):
             return torch.zeros(*shape, dtype=dt, device=dev)
@@ -768,88 +769,125 @@ class Engine:
         if R > NMAX:
             B.part_o = buf(R, c.hq, self.ATTN_SPLITS, c.head_dim, dt=F32)
             B.part_ml = buf(R, c.hq, self.ATTN_SPLITS, 2, dt=F32)
-        if R < W:  # control words of the attention's sub-passes: positions R apart
-            B.ctl = buf(-(-W // R), 32, dt=I32)
-            B.off = (torch.arange(-(-W // R), dtype=I32, device=dev) * R).contiguous()
+        if R < W:  # control words of the mixers' sub-passes: positions 8 apart
+            B.ctl = buf(W // NMAX, 32, dt=I32)
+            B.off = (torch.arange(W // NMAX, dtype=I32, device=dev) * NMAX).contiguous()
         if self.has_mtp:
             B.cat, B.mh = buf(W, 2 * H), buf(W, H)
-        self.wb = B
+        if W > self.WIDE:  # inputs of `_w4.rows` in wire order whose producers write them plain
+            B.wire = buf(W, max(B.mix.size(1), 2 * H))
+        return B
 
-    def _wide_mixer(self, L, n, kv_only=False):
-        """Token mixing of a wide pass. DeltaNet takes all rows in one launch, and so does the attention over
+    def _wide_mixer(self, L, n, B, kv_only=False):
+        """Token mixing of a wide pass. DeltaNet takes up to 64 rows in one launch, and so does the attention over
         caches up to 8K positions; the tensor-core attention of longer caches takes 8 rows, and many
-        splits as many as `_wide_attn_rows` says: there the rows go through in sub-passes, each with
-        its own control words (position). kv_only: just write K and V (a draft layer during prefill:
-        nothing else of it is kept)."""
-        c, B = self.cfg, self.wb
+        splits as many as `_wide_attn_rows` says: beyond that the rows go through in sub-passes, each with
+        its own control words (position, pending rows). kv_only: just write K and V (a draft layer during
+        prefill: nothing else of it is kept)."""
+        c = self.cfg
+
+        def pieces(R):
+            for r in range(0, n, R):
+                yield slice(r, min(n, r + R)), B.ctl[r // NMAX] if r else self.ctl
+
         if L["type"] == "linear_attention":
             pr = B.proj[:n, :c.gdn_proj_rows]
             a0, a1 = c.conv_dim, c.conv_dim + c.value_dim
             out = B.mix[:n, :c.value_dim]
-            _C.gdn_prefill(pr[:, :a0], pr[:, a0:a1], pr[:, a1:a1 + c.hv], pr[:, a1 + c.hv:], L["ring"], L["conv_w"],
-                           L["A_log"], L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"], L["st_g"], self.ctl, out,
-                           c.hk, c.eps)
+            for rows, ctl in pieces(self.WIDE):
+                p = pr[rows]
+                _C.gdn_prefill(p[:, :a0], p[:, a0:a1], p[:, a1:a1 + c.hv], p[:, a1 + c.hv:], L["ring"], L["conv_w"],
+                               L["A_log"], L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"], L["st_g"], ctl,
+                               out[rows], c.hk, c.eps)
             return out
         pr = B.proj[:n, :c.attn_proj_rows]
         nq = c.hq * 2 * c.head_dim
         nk = nq + c.hkv * c.head_dim
         out = B.mix[:n, :c.hq * c.head_dim]
-        _C.attn_prep_rows(pr[:, :nq], pr[:, nq:nk], pr[:, nk:], L["q_norm"], L["k_norm"], self.inv_freq, self.ctl,
-                          B.q[:n], L["kc"], L["vc"], c.eps)
+        for rows, ctl in pieces(self.WIDE):
+            p = pr[rows]
+            _C.attn_prep_rows(p[:, :nq], p[:, nq:nk], p[:, nk:], L["q_norm"], L["k_norm"], self.inv_freq, ctl,
+                              B.q[rows], L["kc"], L["vc"], c.eps)
         if kv_only:
             return out
-        R = B.attn_rows
-        decode = _C.attn_decode if R == NMAX else _C.attn_decode_rows
-        for j in range(-(-n // R)):
-            rows = slice(j * R, min(n, (j + 1) * R))
-            decode(B.q[rows], L["kc"], L["vc"], B.ctl[j] if j else self.ctl, pr[rows, :nq], B.part_o, B.part_ml, out[rows])
+        decode = _C.attn_decode if B.attn_rows == NMAX else _C.attn_decode_rows
+        for rows, ctl in pieces(B.attn_rows):
+            decode(B.q[rows], L["kc"], L["vc"], ctl, pr[rows, :nq], B.part_o, B.part_ml, out[rows])
         return out
 
-    def _wide_pass(self, n, mtp):
-        """One prefill pass over n rows (a multiple of 8, at most WIDE) of wb.tok: what n / 8
+    def _wide_pass(self, n, mtp, exact=False, logits=False):
+        """One prefill pass over n rows (a multiple of 8) of the tokens in its buffers: what n / 8
         ordinary prefill passes do to the K/V caches, the DeltaNet state and the position, with
-        every matrix streamed once (`_w4.gemm`). No logits: the pass that follows emits them.
+        every matrix streamed once. No logits: the pass that follows emits them.
+        exact: up to 128 rows through `_w4.rows`, every bit as the ordinary passes leave it; else up to 64
+        through `_w4.gemm`, which adds in another order. logits (exact only): the final norm's rows are
+        left in rb.xn, in the order that `_w4.rows` takes.
         Follows python/qengine/engine.py:434-477 (layer, main) and :479-496 (draft layer) of the
         reference."""
-        c, B, lin, eps = self.cfg, self.wb, self.linear, self.cfg.eps
-        nb = -(-n // B.attn_rows)  # sub-passes of the attention
+        c, lin, eps = self.cfg, self.linear, self.cfg.eps
+        B = self.rb if exact else self.wb
         self._flush()
-        if nb > 1:
+        if n > min(B.attn_rows, self.WIDE):  # sub-passes of the mixers
+            nb = n // NMAX
             B.ctl[:nb].copy_(self.ctl.expand(nb, -1))
             B.ctl[:nb, self.POS].add_(B.off[:nb])
+            B.ctl[1:nb, self.PENDING].fill_(NMAX)
         h, xn, mo = B.h[:n], B.xn[:n], B.mo[:n]
 
-        def mm(x, p, out):
-            _w4.gemm(x, p.qw, p.scales, out, p.M, swiglu=p.gate_up)
+        def mm(x, p, out, wire_out=False):
+            if exact:
+                _w4.rows(x, p.qw, p.scales, out, p.M, swiglu=p.gate_up, wire_out=wire_out, **lin.kw)
+            else:
+                _w4.gemm(x, p.qw, p.scales, out, p.M, swiglu=p.gate_up)
+
+        def wired(x):  # rows in the order that `mm` takes
+            if not exact:
+                return x
+            y = B.wire[:n, :x.size(1)]
+            y.unflatten(1, (-1, 4, 4, 4)).copy_(x.unflatten(1, (-1, 4, 4, 4)).transpose(2, 3))
+            return y
+
+        def norm(x, delta, w, **kw):
+            lin.norm_rows(x, delta, w, eps, xn, wire=exact, **kw)
 
         def block(L, stream, delta, table_tok=None):
             width = c.gdn_proj_rows if L["type"] == "linear_attention" else c.attn_proj_rows
             if table_tok is not None:  # rows = embedding rows of the tokens
-                lin.norm_rows(self.embed, None, L["in_norm"], eps, xn, tok=table_tok, h_out=stream)
+                norm(self.embed, None, L["in_norm"], tok=table_tok, h_out=stream)
             else:
-                lin.norm_rows(stream, delta, L["in_norm"], eps, xn, h_out=stream if delta is not None else None)
+                norm(stream, delta, L["in_norm"], h_out=stream if delta is not None else None)
             mm(xn, L["in_proj"], B.proj[:n, :width])
 
         first = True
         for L in self.layers:
             block(L, h, None if first else mo, table_tok=B.tok if first else None)
             first = False
-            mixed = self._wide_mixer(L, n)
-            mm(mixed, L["out"], mo)
-            lin.norm_rows(h, mo, L["post_norm"], eps, xn, h_out=h)
-            mm(xn, L["gate_up"], B.act[:n])
+            mixed = self._wide_mixer(L, n, B)
+            mm(wired(mixed), L["out"], mo)
+            norm(h, mo, L["post_norm"], h_out=h)
+            mm(xn, L["gate_up"], B.act[:n], wire_out=exact)
             mm(B.act[:n], L["down"], mo)
+        if logits:
+            norm(h, mo, self.final_norm, h_out=h)
         if mtp:
             # draft layer on the same rows (reference :479-496): input fc([norm(embed(next token)) |
             # norm(final-normed trunk row)]); during prefill only its K/V rows (or DeltaNet state) stay
             M, H = self.mtp, c.hidden
-            lin.norm_rows(h, mo, self.final_norm, eps, B.hid[:n], h_out=h)
             cat = B.cat[:n]
-            lin.norm_rows(self.embed, None, M["pre_e"], eps, cat[:, :H], tok=B.tok[1:])
-            lin.norm_rows(B.hid[:n], None, M["pre_h"], eps, cat[:, H:])
-            mm(cat, M["fc"], B.mh[:n])
+            if exact:  # the kernels of `_trunk` (final norm) and `_draft_rows`
+                for r in range(0, n, self.WIDE):
+                    rows = slice(r, min(n, r + self.WIDE))
+                    lin.norm_rows(h[rows], mo[rows], self.final_norm, eps, B.hid[rows], h_out=h[rows])
+                _C.embed(self.embed, B.tok[1:], B.mh[:n])
+                _C.rmsnorm1p(B.mh[:n], None, M["pre_e"], cat[:, :H], eps)
+                _C.rmsnorm1p(B.hid[:n], None, M["pre_h"], cat[:, H:], eps)
+            else:
+                lin.norm_rows(h, mo, self.final_norm, eps, B.hid[:n], h_out=h)
+                lin.norm_rows(self.embed, None, M["pre_e"], eps, cat[:, :H], tok=B.tok[1:])
+                lin.norm_rows(B.hid[:n], None, M["pre_h"], eps, cat[:, H:])
+            mm(wired(cat), M["fc"], B.mh[:n])
             block(M, B.mh[:n], None)
-            self._wide_mixer(M, n, kv_only=M["type"] != "linear_attention")
+            self._wide_mixer(M, n, B, kv_only=M["type"] != "linear_attention")
         # commit: the position moves on by n; the last sub-pass left 8 DeltaNet rows pending
         self.ctl[self.POS].add_(n)
         self.ctl[self.PENDING].fill_(NMAX)
@@ -862,11 +900,14 @@ class Engine:
         if key in self.graphs:
             return self.graphs[key]
         if self.wb is None:
-            self._make_wide_buffers()
+            self.wb = self._pass_buffers(self.WIDE)
+        return self._capture_pass(key, lambda: self._wide_pass(n, mtp))
+
+    def _capture_pass(self, key, body):
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            self._wide_pass(n, mtp)
+            body()
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
@@ -876,7 +917,7 @@ class Engine:
         gc.disable()
         try:
             with torch.cuda.graph(g, capture_error_mode="global"):
-                self._wide_pass(n, mtp)
+                body()
         finally:
             if gc_was_on:
                 gc.enable()
@@ -895,6 +936,59 @@ class Engine:
         if fresh:
             self.reset()
 
+    # -- passes of up to 128 rows with the bits of the ordinary ones -----------------------------------
+    # A pass of n rows costs the four matrices of a 27B layer 171 us at 16 rows, 174 at 24, 214 at 128; a
+    # pass of 8 rows 58, and its mixers run per pass: from three of those on, one of the former is faster.
+    ROWS, ROWS_MIN = 128, 24
+
+    def rows_ok(self) -> bool:
+        """Prompts go through `_w4.rows` where that leaves what passes of 8 rows leave, bit for bit: the norms
+        have to be the GEMV's own (`fuse`), of rows that their kernel can write in wire order."""
+        nw = 8 if self.linear_warps() in (4, 8) else 16
+        return self.wide_ok() and self.fuse and self.cfg.hidden % 64 == 0 and self.cfg.hidden <= 16 * 32 * nw
+
+    def linear_warps(self):
+        return self.linear.kw.get("warps", 0)
+
+    def _row_blocks(self, P, chunk=NMAX, wide=None):
+        """Sizes of the 128-row passes that open a prompt of P tokens (the rest goes through wide passes
+        or 8-row passes). The last 1..8 tokens run as an ordinary pass. wide: full passes only, which are
+        faster per row than two 64-row passes of the GEMM; a rest is not."""
+        if chunk != NMAX or not self.rows_ok():
+            return []
+        full, rest = divmod(max(0, P - 1) // NMAX * NMAX, self.ROWS)
+        wide = self.wide_prefill if wide is None else wide
+        return [self.ROWS] * full + ([rest] if rest >= self.ROWS_MIN and not wide else [])
+
+    def row_graph(self, n, mtp=False, logits=False):
+        """The CUDA graph of an exact pass over n rows, captured on first use (like `graph`)."""
+        key = ("rows", n, bool(mtp), bool(logits))
+        if n % NMAX or not NMAX <= n <= self.ROWS or (mtp and not self.has_mtp) or not self.rows_ok():
+            raise ValueError(f"no such pass: {key}")
+        if key in self.graphs:
+            return self.graphs[key]
+        if self.rb is None:
+            self.rb = self._pass_buffers(self.ROWS)
+        return self._capture_pass(key, lambda: self._wide_pass(n, mtp, exact=True, logits=logits))
+
+    def _need_rows(self, blocks, mtp, logits=False):
+        fresh = [n for n in set(blocks) if ("rows", n, bool(mtp), logits) not in self.graphs]
+        for n in fresh:
+            self.row_graph(n, mtp, logits)
+        if fresh:
+            self.reset()
+
+    def _need_prompt(self, P, mtp, k, chunk, wide, keys):
+        """Capture the graphs that a prompt of P tokens goes through, and those of `keys`."""
+        blocks = self._row_blocks(P, chunk, wide)
+        head = max(self._wide_split(P, wide), sum(blocks))
+        self._need_rows(blocks, mtp)
+        self._need_wide(head - sum(blocks), mtp)
+        self._need(self._prefill_keys(P, mtp, k, chunk, skip=head) | keys)
+
+    def _feed_rows(self, B, tokens):
+        B.tok[:len(tokens)].copy_(torch.tensor(tokens, dtype=I32))
+
     # -- public loops ---------------------------------------------------------------------------
     def prefill(self, prompt, mtp=False, k=0, chunk=NMAX, wide=None):
         """Feed the prompt `chunk` rows per pass. The last row's greedy token is the first
@@ -903,14 +997,22 @@ class Engine:
         graphs (`generate*` take care of both).
         wide (default: the engine's `wide_prefill`): all but the last 1..8 tokens go through passes
         of up to 64 rows (`_wide_pass`); the state they leave agrees with the 8-row passes to
-        rounding (the GEMM adds a tile's groups in another order than the GEMV), not bit for bit."""
+        rounding (the GEMM adds a tile's groups in another order than the GEMV), not bit for bit.
+        Long prompts go through passes of up to 128 rows first (`_row_blocks`, where their graphs have been
+        captured), which change no bit of what the 8-row passes leave."""
         prompt = list(prompt)
-        head = self._wide_split(len(prompt), wide)
+        blocks = self._row_blocks(len(prompt), chunk, wide)
+        if any(("rows", n, bool(mtp), False) not in self.graphs for n in blocks):
+            blocks = []
+        head = max(self._wide_split(len(prompt), wide), sum(blocks))
         self.ctl[self.MODE].fill_(0)
         at = 0
-        for n in self._wide_blocks(head):
-            row = torch.tensor(prompt[at:at + n + 1], dtype=I32)
-            self.wb.tok[:n + 1].copy_(row)
+        for n in blocks:
+            self._feed_rows(self.rb, prompt[at:at + n + 1])
+            self.row_graph(n, mtp).replay()
+            at += n
+        for n in self._wide_blocks(head - at):
+            self._feed_rows(self.wb, prompt[at:at + n + 1])
             self.wide_graph(n, mtp).replay()
             at += n
         pieces = self._split(prompt[head:], chunk)
@@ -929,9 +1031,7 @@ class Engine:
         if first + n_new + 1 > self.max_len:
             raise ValueError("sequence does not fit max_len")
         step_key = (1, False, 0, False)
-        head = self._wide_split(P, wide)
-        self._need_wide(head, False)
-        self._need(self._prefill_keys(P, False, 0, chunk, skip=head) | {step_key})
+        self._need_prompt(P, False, 0, chunk, wide, {step_key})
         self.reset()
         t = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
         t[0].record()
@@ -967,9 +1067,7 @@ class Engine:
             self.force_a = int(force_accept)
             self.graphs.pop((k + 1, True, k, True), None)  # the graph holds the old truth buffer
         cycle_key = (k + 1, True, k, forced)
-        head = self._wide_split(P, wide)
-        self._need_wide(head, True)
-        self._need(self._prefill_keys(P, True, k, chunk, skip=head) | {cycle_key})
+        self._need_prompt(P, True, k, chunk, wide, {cycle_key})
         self.reset()
         t = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
         t[0].record()
@@ -1002,15 +1100,30 @@ class Engine:
     @torch.no_grad()
     def sequence_logits(self, seq, keep="full", chunk=NMAX):
         """Teacher forcing: `seq` goes through prefill passes; returns the logits of every position
-        [T, V] bf16 (keep='full') or their argmax [T] (keep='argmax')."""
-        pieces = self._split(list(seq), chunk)
+        [T, V] bf16 (keep='full') or their argmax [T] (keep='argmax'). Long sequences go through passes of
+        up to 128 rows (`_row_blocks`), with the bits of the 8-row passes."""
+        seq, head = list(seq), self.lm_head
+        packed = isinstance(self.lm_lin, W4Linear) and isinstance(head, W4Packed) and head.K % 128 == 0
+        blocks = self._row_blocks(len(seq), chunk, False) if packed and seq else []
+        at = sum(blocks)
+        pieces = self._split(seq[at:], chunk)
+        self._need_rows(blocks, False, logits=True)
         self._need({(len(p), False, 0, False) for p in pieces})
         self.reset()
         full = keep == "full"
         out = torch.empty((len(seq), self.cfg.vocab) if full else (len(seq),), dtype=BF16 if full else I32,
                           device=self.dev)
         self.ctl[self.MODE].fill_(0)
+        lg = None if full or not blocks else torch.empty(self.ROWS, self.cfg.vocab, dtype=BF16, device=self.dev)
         at = 0
+        for n in blocks:
+            self._feed_rows(self.rb, seq[at:at + n + 1])
+            self.row_graph(n, logits=True).replay()
+            to = out[at:at + n] if full else lg[:n]
+            _w4.rows(self.rb.xn[:n], head.qw, head.scales, to, head.M, **{**self.linear.kw, "pdl": False})
+            for r in range(0, 0 if full else n, NMAX):
+                _C.argmax(lg[r:r + NMAX], self.am_v, self.am_i, out[at + r:at + r + NMAX])
+            at += n
         for i, piece in enumerate(pieces):
             self._feed(piece, pieces[i + 1][0] if i + 1 < len(pieces) else -1)
             self.graph(len(piece), False, 0).replay()
