@@ -85,6 +85,7 @@ struct GemvArgs {
                    // in shared memory (the normalised rows, which fp16 holds exactly, see make_job)
   __half* xn16_out;  // norm_rows_kernel only: optional fp16 copy of the normalised rows
   long ldx16;
+  int stage_x;     // the rows are copied into shared memory first (stage_rows)
   int wire;        // norm_rows_kernel, one row at a time: xn_out in wire order (wire_pos)
   int xvec;        // x rows are 16-byte aligned with ldx % 8 == 0
   // fused residual + RMSNorm prologue (h_in != nullptr)
@@ -131,6 +132,43 @@ __device__ __noinline__ void load_x_slow(UnitOps& o, const bf16* row, int gg, in
   }
   o.x0 = make_uint4(v[0], v[1], v[2], v[3]);   o.x1 = make_uint4(v[4], v[5], v[6], v[7]);
   o.x2 = make_uint4(v[8], v[9], v[10], v[11]); o.x3 = make_uint4(v[12], v[13], v[14], v[15]);
+}
+
+// Rows that are not made of aligned 16-byte packets, or end inside a group: copied into shared memory once,
+// with zeros up to the end of the last group, so that the stream reads them like any others. Read element
+// by element inside it, a unit cost some 40 loads per lane. 5 rows, 5001 x 3407: 13.4 -> 8.9 us; 6
+// rows, 30000 x 7777: 125 -> 39; 8 rows, 17000 x 12001, in two launches of four: 123 -> 69. (With groups that
+// are no multiple of four, stages inside a tile as straight-line code: 5001 x 3456 8.7 -> 7.6.)
+template <int NW>
+__device__ __forceinline__ void stage_rows(const GemvArgs& a, unsigned char* x_s, long pitch, int tid) {
+  const int packets = a.G * 16, whole = a.K >> 3;
+#pragma unroll 1
+  for (int r = 0; r < a.o.N; ++r) {
+    const unsigned short* row = reinterpret_cast<const unsigned short*>(a.x + (long)r * a.ldx);
+    const int off = (int)(reinterpret_cast<uintptr_t>(row) & 3) >> 1;  // rows begin on a word, or in the middle of one
+    const unsigned* words = reinterpret_cast<const unsigned*>(row - off);
+    uint4* to = reinterpret_cast<uint4*>(x_s + r * pitch);
+#pragma unroll 2
+    for (int p = tid; p < packets; p += NW * 32) {
+      unsigned w[4] = {0u, 0u, 0u, 0u};
+      if (p < whole) {  // four words, and one more where the row begins in the middle of one
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = words[4 * p + i];
+        if (off) {
+          const unsigned last = row[8 * p + 7];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], 16);
+          w[3] = w[3] >> 16 | last << 16;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (8 * p + e < a.K) w[e >> 1] |= (unsigned)row[8 * p + e] << (16 * (e & 1));
+      }
+      to[p] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  __syncthreads();
 }
 
 // The fused prologue: x_s[r] = RMSNorm1p(h_in[r] + delta[r]) * (1 + w) for r < N, computed by the
@@ -402,7 +440,10 @@ __device__ __forceinline__ void grid_barrier(int* gbar, int nblocks) {
   __syncthreads();
 }
 
-template <int NW, int PERW, int STAGES>
+// kAny: serves every shape and every row of x. Without, whole groups, tiles of a whole number of stages and
+// aligned rows only (plain_job): every matrix of the 27B model, with a stream loop that has nothing to decide.
+// One function for both costs that loop 1..4 % (registers), whichever way the two share it.
+template <int NW, int PERW, int STAGES, bool kAny>
 __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_constant__ ChainArgs c) {
   constexpr uint32_t kStageW = PERW * 1024, kStageS = PERW * 32;
   constexpr uint32_t kRing = STAGES * (kStageW + kStageS);
@@ -493,11 +534,17 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       }
       xbase = x_s + xrow * pitch + 32 * t;
       xfast = true;
+    } else if (kAny && a.stage_x) {
+      const long pitch = (long)G * 256 + 16;
+      if (j) __syncthreads();  // the job before has left x_s
+      stage_rows<NW>(a, x_s, pitch, tid);
+      xbase = x_s + xrow * pitch + 32 * t;
+      xfast = true;
     } else {
       xbase = reinterpret_cast<const unsigned char*>(a.x + (long)xrow * a.ldx) + 32 * t;
       xfast = a.xvec != 0;
     }
-    const bool tail_k = (a.K & 127) != 0;  // the last group reads past K unless guarded
+    const bool tail_k = kAny && (a.K & 127) != 0 && !a.stage_x;  // the last group reads past K unless guarded
 
     // ---- the stream ----
     int tile = tile_of(a, u0);
@@ -526,15 +573,11 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
     // more in instruction fetch than the cheaper unpack saves.
     auto stream = [&](auto f16_tag) {
       constexpr bool F16 = decltype(f16_tag)::value;
-      // Both loops below walk the ring stage by stage. The fast one serves ranges made of whole
-      // stages that never straddle a tile (every matrix of the model): no per-unit decisions at
-      // all, every operand at an immediate offset from three base pointers.
-      const bool all_fast = xfast && !tail_k && (a.d.quantum % PERW) == 0;
-      if (all_fast) {
+      // Every stage holds PERW units of one tile, with activations that can be read as 16-byte packets:
+      // straight-line code, every operand at an immediate offset from three base pointers.
+      if (!kAny || (xfast && !tail_k && (a.d.quantum % PERW) == 0)) {
         const unsigned char* xg = xbase + (size_t)g * 256;
-        // the next stage to request from HBM: whole stages only in this loop, so the copy sizes are
-        // constants and the global addresses advance by constants
-        const uint4* gw = a.qw + (size_t)(u0 + STAGES * PERW) * 64 + lane;
+        const uint4* gw = a.qw + (size_t)(u0 + STAGES * PERW) * 64 + lane;  // the next stage to request
         const __half* gs = a.scales + (size_t)(u0 + STAGES * PERW) * 16 + lane * 8;
         int to_request = nstage - STAGES;  // stages not yet requested
   #pragma unroll 1
@@ -581,32 +624,63 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
           commit();
           if (++slot == STAGES) slot = 0;
         }
-      } else {
-  #pragma unroll 1
+        return;
+      }
+      if constexpr (kAny) {
+        // Any other matrix. Stages inside a tile whose activations are aligned packets run as above, those across
+        // a tile's end or with a ragged last group unit by unit.
+        const int g_fast = xfast ? (tail_k ? G - 1 : G) : 0;  // groups below: whole, and aligned
+        const int full = n_units / PERW;                      // whole stages
+    #pragma unroll 1
         for (int st = 0; st < nstage; ++st) {
           await_stage();
-          const uint4* wp = reinterpret_cast<const uint4*>(ring_w + (size_t)slot * kStageW) + lane;
-          const unsigned short* sp = reinterpret_cast<const unsigned short*>(ring_s + (size_t)slot * kStageS) + r;
-          const int cnt = min(PERW, n_units - st * PERW);
-  #pragma unroll 1
-          for (int i = 0; i < cnt; ++i) {
-            UnitOps o;
-            o.w0 = wp[i * 64];
-            o.w1 = wp[i * 64 + 32];
-            o.s_lo = sp[i * 16];
-            o.s_hi = sp[i * 16 + 8];
-            if (xfast && !(tail_k && g == G - 1)) {
-              const uint4* xp = reinterpret_cast<const uint4*>(xbase + (size_t)g * 256);
-              o.x0 = xp[0]; o.x1 = xp[1]; o.x2 = xp[8]; o.x3 = xp[9];
-            } else {
-              load_x_slow(o, a.x + (long)xrow * a.ldx, g, t, a.K);
+          unsigned char* stage_w = ring_w + (size_t)slot * kStageW;
+          unsigned char* stage_s = ring_s + (size_t)slot * kStageS;
+          const uint4* wp = reinterpret_cast<const uint4*>(stage_w) + lane;
+          const unsigned short* sp = reinterpret_cast<const unsigned short*>(stage_s) + r;
+          if (st < full && g + PERW <= g_fast) {
+            const uint4* xp = reinterpret_cast<const uint4*>(xbase + (size_t)g * 256);
+            UnitOps ops[PERW];
+    #pragma unroll
+            for (int i = 0; i < PERW; ++i) {
+              ops[i].w0 = wp[i * 64];
+              ops[i].w1 = wp[i * 64 + 32];
+              ops[i].s_lo = sp[i * 16];
+              ops[i].s_hi = sp[i * 16 + 8];
+              ops[i].x0 = xp[i * 16];
+              ops[i].x1 = xp[i * 16 + 1];
+              ops[i].x2 = xp[i * 16 + 8];
+              ops[i].x3 = xp[i * 16 + 9];
             }
-            if constexpr (F16) unit_fma_f16(acc, o);
-            else unit_fma(acc, o);
-            ++g;
-            if (g == G || (st == nstage - 1 && i == cnt - 1)) close_segment();
+    #pragma unroll
+            for (int i = 0; i < PERW; ++i) {
+              if constexpr (F16) unit_fma_f16(acc, ops[i]);
+              else unit_fma(acc, ops[i]);
+            }
+            g += PERW;
+            if (g == G || st == nstage - 1) close_segment();
+          } else {
+            const int cnt = min(PERW, n_units - st * PERW);
+    #pragma unroll 1
+            for (int i = 0; i < cnt; ++i) {
+              UnitOps o;
+              o.w0 = wp[i * 64];
+              o.w1 = wp[i * 64 + 32];
+              o.s_lo = sp[i * 16];
+              o.s_hi = sp[i * 16 + 8];
+              if (g < g_fast) {
+                const uint4* xp = reinterpret_cast<const uint4*>(xbase + (size_t)g * 256);
+                o.x0 = xp[0]; o.x1 = xp[1]; o.x2 = xp[8]; o.x3 = xp[9];
+              } else {
+                load_x_slow(o, a.x + (long)xrow * a.ldx, g, t, a.K);
+              }
+              if constexpr (F16) unit_fma_f16(acc, o);
+              else unit_fma(acc, o);
+              ++g;
+              if (g == G || (st == nstage - 1 && i == cnt - 1)) close_segment();
+            }
           }
-          __syncwarp();
+          __syncwarp();  // every lane has read this stage: its slot may be filled again
           fill(a, u0, u1, st + STAGES, st + STAGES + 1, slot);
           if (++slot == STAGES) slot = 0;
         }
@@ -720,13 +794,13 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
 using KernelFn = void (*)(const ChainArgs);
 
 struct Geometry {
-  KernelFn fn;
+  KernelFn plain, any;
   int nw, perw, stages;
   size_t ring_bytes() const { return (size_t)nw * stages * perw * (1024 + 32) + (size_t)nw * 2 * 128 * sizeof(float); }
 };
 template <int NW, int PERW, int STAGES>
 constexpr Geometry geometry() {
-  return Geometry{w4_chain_kernel<NW, PERW, STAGES>, NW, PERW, STAGES};
+  return Geometry{w4_chain_kernel<NW, PERW, STAGES, false>, w4_chain_kernel<NW, PERW, STAGES, true>, NW, PERW, STAGES};
 }
 // Selected by the reference's launch options. `warps`: 0 (auto) / 16 -> 16 warps per CTA, 4 / 8 -> 8;
 // variant 1 -> 24 warps, variant 2 -> 20 warps. `unroll` picks the ring: 2 -> 3 stages of 2 units, 4 -> 2
@@ -746,27 +820,31 @@ const Geometry& pick_geometry(const qe_w4_cfg& c, int ring = -1) {
   return kGeoms[3 * size + ring];
 }
 
-// Largest dynamic shared memory a launch of `fn` may ask for on the current device (the opt-in
-// maximum minus the kernel's static shared memory). Raising the per-function limit is a per-device
-// setting: done once per (function, device). Returns < 0 (minus the CUDA error) on failure.
-long dynamic_smem_limit(KernelFn fn) {
+// Largest dynamic shared memory a launch of the geometry's kernels may ask for on the current device (the opt-in
+// maximum minus the kernels' static shared memory). Raising the per-function limit is a per-device
+// setting: done once per (geometry, device). Returns < 0 (minus the CUDA error) on failure.
+long dynamic_smem_limit(const Geometry& geom) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, long> known;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return -(long)e;
   std::lock_guard<std::mutex> lk(mu);
-  auto it = known.find({(const void*)fn, dev});
+  auto it = known.find({(const void*)geom.plain, dev});
   if (it != known.end()) return it->second;
   int optin = 0;
-  cudaFuncAttributes fa{};
-  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess ||
-      (e = cudaFuncGetAttributes(&fa, fn)) != cudaSuccess)
-    return -(long)e;
-  const long limit = (long)optin - (long)fa.sharedSizeBytes;
-  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit)) != cudaSuccess)
-    return -(long)e;
-  known[{(const void*)fn, dev}] = limit;
+  long limit = 0;
+  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return -(long)e;
+  for (KernelFn fn : {geom.plain, geom.any}) {
+    cudaFuncAttributes fa{};
+    if ((e = cudaFuncGetAttributes(&fa, fn)) != cudaSuccess) return -(long)e;
+    const long own = (long)optin - (long)fa.sharedSizeBytes;
+    limit = limit ? std::min(limit, own) : own;
+  }
+  for (KernelFn fn : {geom.plain, geom.any})
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit)) != cudaSuccess)
+      return -(long)e;
+  known[{(const void*)geom.plain, dev}] = limit;
   return limit;
 }
 
@@ -924,6 +1002,12 @@ int make_job(const qe_w4_params* p, const qe_w4_norm* nrm, const qe_w4_cfg* cfg,
   return 0;
 }
 
+// Jobs of the kernel without kAny.
+bool plain_job(const GemvArgs& a, int perw) { return (a.h_in || a.xvec) && a.K % 128 == 0 && a.d.quantum % perw == 0; }
+
+// Shared memory for the rows of a job that the vector path cannot read as they are; 0: it can.
+size_t stage_bytes(const GemvArgs& a) { return a.xvec && a.K % 128 == 0 ? 0 : (size_t)a.o.N * (a.G * 256 + 16); }
+
 int launch_chain(const qe_w4_params* const* ps, const qe_w4_norm* const* nrms, int njobs, const qe_w4_cfg* cfg,
                  int* gridbar, cudaStream_t stream) {
   if (!ps || !cfg || njobs < 1 || njobs > kMaxJobs || (njobs > 1 && !gridbar)) return QE_ERR_ARG;
@@ -947,14 +1031,50 @@ int launch_chain(const qe_w4_params* const* ps, const qe_w4_norm* const* nrms, i
   if (cfg->unroll == 0 && cfg->variant != 1) {
     for (int ring : {1, 0, 2}) {
       const Geometry& cand = pick_geometry(*cfg, ring);
-      const long lim = dynamic_smem_limit(cand.fn);
+      const long lim = dynamic_smem_limit(cand);
       if (lim < 0) return (int)-lim;
       geom = &cand;
       if ((long)(cand.ring_bytes() + extra) <= lim) break;
     }
   }
+  // Rows that the vector path cannot read are copied into shared memory where all of a chain's fit.
+  size_t staged = 0;
+  for (int j = 0; j < njobs; ++j)
+    if (c.job[j].x && !c.job[j].h_in) staged = std::max(staged, stage_bytes(c.job[j]));
+  if (staged) {
+    for (int ring : {1, 0, 2}) {
+      const Geometry& cand = cfg->unroll == 0 && cfg->variant != 1 ? pick_geometry(*cfg, ring) : *geom;
+      const long lim = dynamic_smem_limit(cand);
+      if (lim < 0) return (int)-lim;
+      if ((long)(cand.ring_bytes() + std::max(extra, staged)) > lim) continue;
+      geom = &cand;
+      extra = std::max(extra, staged);
+      for (int j = 0; j < njobs; ++j) c.job[j].stage_x = c.job[j].x && !c.job[j].h_in && stage_bytes(c.job[j]) ? 1 : 0;
+      break;
+    }
+    // More than fit, in one job: as few launches as hold them, rows dealt out evenly (they are independent). A
+    // second stream of the matrix costs less than reading rows element by element.
+    if (njobs == 1 && !c.job[0].stage_x) {
+      const Geometry& least = cfg->unroll == 0 && cfg->variant != 1 ? pick_geometry(*cfg, 2) : *geom;
+      const long room = dynamic_smem_limit(least) - (long)least.ring_bytes(), row = (long)c.job[0].G * 256 + 16;
+      const int fit = (int)std::min<long>(room / row, ps[0]->N - 1);
+      if (fit >= 1) {
+        const int parts = (ps[0]->N + fit - 1) / fit, each = (ps[0]->N + parts - 1) / parts;
+        for (int r = 0; r < ps[0]->N; r += each) {
+          qe_w4_params q = *ps[0];
+          q.x = (const bf16*)q.x + (long)r * q.ldx;
+          q.out = (char*)q.out + (long)r * q.ldo * (c.job[0].o.out_f32 ? 4 : 2);
+          q.N = std::min(each, ps[0]->N - r);
+          const qe_w4_params* one = &q;
+          const int rc = launch_chain(&one, nullptr, 1, cfg, gridbar, stream);
+          if (rc) return rc;
+        }
+        return 0;
+      }
+    }
+  }
   const size_t smem = geom->ring_bytes() + extra;
-  const long limit = dynamic_smem_limit(geom->fn);
+  const long limit = dynamic_smem_limit(*geom);
   if (limit < 0) return (int)-limit;
   if ((long)smem > limit) return QE_ERR_ARG;  // prologue rows do not fit: run qe_rmsnorm1p + qe_w4_gemv
   const bool pdl = cfg->pdl && pdl_launch_enabled() && pdl_trigger_enabled();
@@ -977,7 +1097,9 @@ int launch_chain(const qe_w4_params* const* ps, const qe_w4_norm* const* nrms, i
   }
   lc.attrs = at;
   lc.numAttrs = na;
-  return (int)cudaLaunchKernelEx(&lc, geom->fn, c);
+  bool plain = true;
+  for (int j = 0; j < njobs; ++j) plain = plain && plain_job(c.job[j], geom->perw);
+  return (int)cudaLaunchKernelEx(&lc, plain ? geom->plain : geom->any, c);
 }
 
 }  // namespace

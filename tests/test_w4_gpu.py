@@ -558,3 +558,27 @@ def test_fp16_activations_are_not_part_of_the_reference_surface(api):
     p2 = api["q"](rand_w(32, 200, seed=84))              # K != Kp
     with pytest.raises(RuntimeError):
         w4.job(torch.randn(1, 200, device=DEV).half(), p2.qw, p2.scales, out, 32, allow_f16_x=True)
+
+
+@pytest.mark.parametrize("N,M,K,offset,pad", [(5, 5001, 3407, 0, 0), (1, 512, 513, 1, 0), (8, 300, 1000, 0, 2), (3, 100, 7, 1, 3),
+                                              (8, 400, 9001, 0, 0), (7, 200, 17407, 1, 0), (8, 64, 20000, 0, 0),
+                                              (4, 96, 1280, 1, 0), (2, 1000, 384, 4, 8), (2, 48, 80001, 0, 0)])
+def test_rows_that_are_not_aligned_packets(api, N, M, K, offset, pad):
+    """Rows of any length and alignment (odd row strides, views that begin in the middle of a word, ends inside
+    a group; more rows than shared memory holds at once; a row that it does not hold) have the bits of
+    the same rows in aligned memory with zeros up to the end of the last group."""
+    from qengine_b200 import _w4
+    from qengine_b200.quant import W4Packed
+    g = torch.Generator(device=DEV).manual_seed(N + M + K)
+    Mp, Kp = -(-M // 16) * 16, -(-K // 128) * 128
+    qw = torch.randint(-2**31, 2**31 - 1, (Mp // 16, Kp // 64, 32, 4), dtype=torch.int32, device=DEV, generator=g)
+    p = W4Packed(qw, torch.randn(Mp // 16, Kp // 128, 16, device=DEV, generator=g).half(), M, K)
+    flat = torch.full((N * (K + pad) + offset,), float("nan"), dtype=torch.bfloat16, device=DEV)
+    x = flat[offset:].as_strided((N, K), (K + pad, 1))
+    x.copy_(torch.randn(N, K, device=DEV, generator=g))
+    aligned = torch.zeros(N, Kp, dtype=torch.bfloat16, device=DEV)
+    aligned[:, :K] = x
+    got, want = (torch.empty(N, M, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    _w4.gemv(x, p.qw, p.scales, got, M)
+    _w4.gemv(aligned, p.qw, p.scales, want, M)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16)) and not got.isnan().any()
