@@ -9,15 +9,22 @@
 // of both 64-k chunks c, which are exactly the 2 x 16 bytes it writes, so nothing is exchanged but
 // the two row maxima (over the four lanes of a row). Every weight is read once and every word written
 // once, whole sectors on both sides. Bound: HBM. The torch packer goes over the matrix about forty times
-// (int64 code words among them): 7.9 ms for a bf16 gate/up pair of 17,408 x 5,120; this kernel 0.154 ms
-// (2.9 TB/s; the floor at the copy rate is 0.069 ms, the rest is the arithmetic, about ten instructions
-// per weight). Three blocks per SM cap the 16-bit types at 80 registers, of which they spill 28 to 40 bytes.
+// (int64 code words among them): 7.9 ms for a bf16 gate/up pair of 17,408 x 5,120; this kernel 0.080 ms
+// (5.6 TB/s; the floor at the copy rate is 0.069 ms). Four operations per weight, two weights to an
+// instruction; with a second pass of divisions for every unit that holds a half it was 0.157 ms. Four blocks per SM
+// cap the 16-bit types at 64 registers, of which they spill 88 bytes; three blocks without spills take 0.087 ms.
 //
 // The quotient is only ever rounded to a whole number, so one division per group is enough: w times
 // the reciprocal is within 4e-6 of the quotient where the code is not clamped (|w / scale| <= 8, four
-// roundings of 2^-24 relative each), and only where it lies within 1e-5 of the middle between two
-// whole numbers can the rounding differ (2e-5 of random weights): a lane that has one among its 64
-// weights quantises them all again with divisions.
+// roundings of 2^-24 relative each).
+//   * 16-bit types: w = a 2^p and scale = b 2^q with a, b < 2^11, so a quotient that is not exactly half way
+//     between two whole numbers is at least 1.2e-4 away from it ((2 a 2^(p-q) - (2 k + 1) b) / (2 b), whose
+//     numerator is a multiple of 1/2 or larger). Rounded to a multiple of 2^-14 first, the approximation of a
+//     half is the half again, and nothing else is: rounding that, ties to even, gives the code. Halves
+//     are common, not rare: a bf16 row maximum that 15 divides gives an exact scale and, where it is
+//     negative, the quotient -7.5. (Quantised again with divisions, as below, those were half of all warps.)
+//   * fp32: only where the approximation lies within 1e-5 of a half can the rounding differ (2e-5 of
+//     random weights): a lane that has one among its 64 weights quantises them all again with divisions.
 #include <type_traits>
 
 #include "w4_dev.cuh"
@@ -91,9 +98,18 @@ struct Row16 {
 // A sum with this number (1.5 * 2^23) is rounded to a whole number, ties to even: rounding costs one
 // addition on the FMA pipe instead of a conversion on the quarter-rate one.
 constexpr float kRound = 12582912.0f;
+// ... with this one (1.5 * 2^9) to a multiple of 2^-14.
+constexpr float kSnap = 768.0f;
+
+// max(|a|, |b|, |c|)
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float d;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) pack_kernel(const PackArgs a) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 4) pack_kernel(const PackArgs a) {
   const int lane = threadIdx.x & 31, r = lane >> 2, t = lane & 3;
   const long u = (long)blockIdx.x * 8 + (threadIdx.x >> 5);  // unit: tile * G + group
   if (u >= (long)a.tiles * a.G) return;
@@ -131,30 +147,42 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) pack_kernel(const
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        // the codes are whole numbers below 16: four of them are put together exactly in fp32
-        float half_word[2] = {0.f, 0.f};
+        // the codes are whole numbers below 16: four of them are put together exactly in fp32, those of even
+        // k in one half of the word and those of odd k in the other, so two at a time
+        float2 half_word = make_float2(0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float v = x[j][c].get(4 * w + e);
-            float q;
+          for (int e = 0; e < 4; e += 2) {
+            const float2 v = make_float2(x[j][c].get(4 * w + e), x[j][c].get(4 * w + e + 1));
+            float2 minus;  // the codes, negative
             if constexpr (decltype(exact)::value) {
-              q = fminf(fmaxf((v / s[j] + kRound) - kRound, -8.f), 7.f) + 8.f;
+              minus.x = -(fminf(fmaxf((v.x / s[j] + kRound) - kRound, -8.f), 7.f) + 8.f);
+              minus.y = -(fminf(fmaxf((v.y / s[j] + kRound) - kRound, -8.f), 7.f) + 8.f);
             } else {
-              const float y = __saturatef(fmaf(v, inv[j], 8.f / 15.f));  // (quotient + 8) / 15, clamped
-              q = fmaf(y, 15.f, kRound) - kRound;
-              far = fmaxf(far, fabsf(fmaf(y, 15.f, -q)));
+              const float2 y = make_float2(__saturatef(fmaf(v.x, inv[j], 8.f / 15.f)),  // (quotient + 8) / 15, clamped
+                                           __saturatef(fmaf(v.y, inv[j], 8.f / 15.f)));
+              const float2 k15 = make_float2(15.f, 15.f), round = make_float2(kRound, kRound);
+              if constexpr (sizeof(T) == 2) {
+                // first to a multiple of 2^-14, which an exact half survives, then to a whole number
+                const float2 z = fma2(y, k15, make_float2(kSnap, kSnap));
+                const float2 q = fma2(z, make_float2(1.f, 1.f), make_float2(kRound - kSnap, kRound - kSnap));
+                minus = fma2(q, make_float2(-1.f, -1.f), round);
+              } else {
+                minus = fma2(fma2(y, k15, round), make_float2(-1.f, -1.f), round);
+                const float2 d = fma2(y, k15, minus);
+                far = max3_abs(far, d.x, d.y);
+              }
             }
-            const int nib = j + 2 * (e >> 1) + 4 * (e & 1);
-            half_word[nib >> 2] = fmaf(q, (float)(1 << (4 * (nib & 3))), half_word[nib >> 2]);
+            const float place = -(float)(1 << (4 * (j + e)));
+            half_word = fma2(minus, make_float2(place, place), half_word);
           }
-        const uint32_t lo = __float_as_uint(half_word[0] + kRound), hi = __float_as_uint(half_word[1] + kRound);
+        const uint32_t lo = __float_as_uint(half_word.x + kRound), hi = __float_as_uint(half_word.y + kRound);
         word[c][w] = (__byte_perm(lo, hi, 0x5410) & keep) | (0x88888888u & ~keep);
       }
   };
   quantise(std::false_type{});
-  if (far > 0.5f - 1e-5f) quantise(std::true_type{});
+  if (sizeof(T) == 4 && far > 0.5f - 1e-5f) quantise(std::true_type{});
 #pragma unroll
   for (int c = 0; c < 2; ++c)
     a.qw[(size_t)u * 64 + c * 32 + lane] = make_uint4(word[c][0], word[c][1], word[c][2], word[c][3]);

@@ -77,3 +77,20 @@ def test_lazily_negated_and_traced_matrices():
     _same(quant.quantize_w4(torch._neg_view(a.cuda())), quant.quantize_w4(-a))
     traced = make_fx(lambda w: quant.quantize_w4(w).qw)(a.cuda())
     assert torch.equal(traced(b.cuda()).cpu(), quant.quantize_w4(b).qw)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_quotients_half_way_between_codes(dt):
+    """Rows whose quotients are exact halves or next to one (a maximum that 15 divides has an exact scale; a
+    negative one then is the quotient -7.5): the codes are those of a division, ties to even."""
+    from qengine_b200.quant import quantize_w4
+    g = torch.Generator().manual_seed(3)
+    top = 256 if dt == torch.bfloat16 else 2048
+    m = torch.randint(1, top, (4096, 1), generator=g).float()
+    m[:1024] = 15 * torch.randint(1, top // 15, (1024, 1), generator=g)
+    w = torch.randint(-top, top + 1, (4096, 256), generator=g).float().clamp(-m, m)
+    w[:, 1::2] = (torch.randint(-15, 16, (4096, 128), generator=g) * m / 15).round()  # at and around k + 1/2
+    w[:, 0], w[:, 128] = -m[:, 0], m[:, 0]
+    w = (w * 2.0 ** torch.randint(-9, 2, (4096, 1), generator=g)).to(dt)
+    a, b = quantize_w4(w.cuda()), quantize_w4(w)
+    assert torch.equal(a.scales.cpu().view(torch.int16), b.scales.view(torch.int16)) and torch.equal(a.qw.cpu(), b.qw)
