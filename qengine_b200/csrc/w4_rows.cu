@@ -19,12 +19,17 @@
 // Design: the tensor-memory GEMM of w4_gemm.cu (unpacking warps, one issuing thread, drain warps, coupled by
 // mbarriers) with another walk. A job is one super-tile of 128 weight rows over the whole of K and all
 // activation rows, or over a part of the columns where there are fewer super-tiles than half the SMs: a split
-// along K would close partial sums where the GEMV does not. Eight drain warps read each product, four the
-// first half of its columns and four the second: 64 sums per thread at 128 rows. Tensor memory: D in two
-// stages of 128 columns (four of 64 where that is enough), A in four of 64.
-//   * What bounds it: hand-over latency, as in w4_gemm.cu: a step (one group of a super-tile) costs some
-//     900-1100 clk whatever its rows, half of it the unpack (888 clk: 260 instructions of each of four
-//     warps), and unpack, issue and drain wait for one another. Hence 128 rows and not 64.
+// along K would close partial sums where the GEMV does not. Eighteen warps: one issues the products; one asks
+// for the activations (a request holds its warp up for some hundred clocks, which the drain warps cannot
+// spare) and passes on that they have landed, so that the issuing thread has one barrier to wait for; the
+// other sixteen are shared out by the columns of a job (below). Tensor memory: D in two stages of 128 columns
+// or four of 64, A in four of 64.
+//   * What bounds it: hand-over latency, as in w4_gemm.cu. A barrier wait costs 270 clk even when there is
+//     nothing to wait for, an unpacking warp's turn 700, a drain warp's 500 (32 columns) to 800 (48), and a
+//     step (one group of a super-tile) takes 900 clk at 16 columns, 1150 at 64, 1500 at 128. Hence 128 rows.
+//   * us, the four matrices of a 27B layer (in the order in_proj, out, gate/up, down): 128 rows 32 + 33 + 65 + 79 = 210,
+//     64 rows 26 + 30 + 50 + 73 = 180, 24 rows 163; eight rows through the GEMV 57, 64 through w4_gemm.cu 130. First
+//     form (requests by the drain warps, eight drain and eight unpacking warps whatever the columns): 385, 323, 300.
 // Every wait is bounded (see w4_gemm.cu).
 #include <algorithm>
 
@@ -83,14 +88,24 @@ __device__ __forceinline__ void ld16_wait(uint32_t (&u)[16]) {
                : "memory");
 }
 
+// (Arrived with an earlier wait: what stays is that no use of them moves in front of that.)
+__device__ __forceinline__ void ld16_arrived(uint32_t (&u)[16]) {
+  asm volatile(""
+               : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]), "+r"(u[6]), "+r"(u[7]),
+                 "+r"(u[8]), "+r"(u[9]), "+r"(u[10]), "+r"(u[11]), "+r"(u[12]), "+r"(u[13]), "+r"(u[14]), "+r"(u[15])
+               :
+               : "memory");
+}
+
 // kU groups of four unpacking warps, which alternate steps; kP groups of four drain warps, which share the
-// columns. 1, 3: up to 128 columns, 48 sums per thread, and one group of unpacking warps keeps up with
-// them. 2, 2: up to 64 columns, where the unpack is the longer turn.
+// columns, at most 48 of them per thread (96 registers). Where the line lies, us of gate/up and of down at
+// that many columns: up to 128, <1, 3>, 65 against 106 for two groups of drain warps with 64 sums; up to
+// 64, <2, 2>, 50 against 56 for <1, 3>; up to 48, where the unpack is the longer turn, <3, 1>, 43 against 46 for
+// <2, 2> at 16 columns, and 79 against 83 for down at 48.
 template <int kU, int kP>
 __global__ void __launch_bounds__(kThreads, 1)
     w4_rows_kernel(const __grid_constant__ RowsArgs a, const __grid_constant__ CUtensorMap xmap) {
-  constexpr int kDrain = 4 * kP, kBlocks = kP == 3 ? 3 : 2;  // drain warps; 16-column blocks of one of them
-  constexpr bool kPipe = kP == 2;
+  constexpr int kDrain = 4 * kP, kBlocks = kP == 2 ? 2 : 3;  // drain warps; 16-column blocks of one of them
   static_assert(2 + kDrain + 4 * kU == kThreads / 32, "warps");
   dep_release();
   extern __shared__ unsigned char smem_raw[];
@@ -358,21 +373,35 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           tc_fence_after();
           const uint32_t t0 = t_lane + (v & (nd - 1)) * dcols + col0;
-          uint32_t u[kPipe ? 2 : 1][16];
-          if (kPipe && blocks > 0) ld16_ask(t0, u[0]);
-#pragma unroll
-          for (int h = 0; h < kBlocks; ++h) {
-            if (h >= blocks) break;
-            if (!kPipe) ld16_ask(t0 + 16 * h, u[0]);
-            ld16_wait(u[kPipe ? h & 1 : 0]);
-            if (kPipe && h + 1 < kBlocks && h + 1 < blocks) ld16_ask(t0 + 16 * (h + 1), u[kPipe ? (h + 1) & 1 : 0]);  // on its way meanwhile
+          auto add = [&](const uint32_t (&u)[16], int h) {
 #pragma unroll
             for (int k = 0; k < 16; k += 2) {
               float* const to = acc + 16 * h + k;
-              const float2 sum = fma2(make_float2(scale, scale),
-                                      make_float2(__uint_as_float(u[kPipe ? h & 1 : 0][k]), __uint_as_float(u[kPipe ? h & 1 : 0][k + 1])),
+              const float2 sum = fma2(make_float2(scale, scale), make_float2(__uint_as_float(u[k]), __uint_as_float(u[k + 1])),
                                       make_float2(to[0], to[1]));
               to[0] = sum.x, to[1] = sum.y;
+            }
+          };
+          if constexpr (kBlocks == 2) {  // both blocks in one trip to tensor memory (three would spill)
+            uint32_t u0[16], u1[16];
+            if (blocks > 0) {
+              ld16_ask(t0, u0);
+              if (blocks > 1) ld16_ask(t0 + 16, u1);
+              ld16_wait(u0);
+              add(u0, 0);
+              if (blocks > 1) {
+                ld16_arrived(u1);
+                add(u1, 1);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int h = 0; h < kBlocks; ++h) {
+              if (h >= blocks) break;
+              uint32_t u[16];
+              ld16_ask(t0 + 16 * h, u);
+              ld16_wait(u);
+              add(u, h);
             }
           }
           tc_fence_before();
@@ -458,6 +487,8 @@ extern "C" int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, i
     e = cudaFuncSetAttribute(w4_rows_kernel<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(w4_rows_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(w4_rows_kernel<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return (int)e;
     allowed[dev] = true;
   }
@@ -485,6 +516,6 @@ extern "C" int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, i
   CUtensorMap map{};
   if (!map_rows(p, a.cols, 2, &map)) return QE_ERR_ARG;
   const bool pdl = cfg->pdl && pdl_launch_enabled() && pdl_trigger_enabled();
-  return (int)launch(a.cols > 64 ? w4_rows_kernel<1, 3> : w4_rows_kernel<2, 2>, dim3(std::min(sms, ST * a.cparts)), dim3(kThreads), kSmem, (cudaStream_t)stream, pdl,
+  return (int)launch(a.cols > 64 ? w4_rows_kernel<1, 3> : a.cols > 48 ? w4_rows_kernel<2, 2> : w4_rows_kernel<3, 1>, dim3(std::min(sms, ST * a.cparts)), dim3(kThreads), kSmem, (cudaStream_t)stream, pdl,
                      a, map);
 }

@@ -937,8 +937,8 @@ class Engine:
             self.reset()
 
     # -- passes of up to 128 rows with the bits of the ordinary ones -----------------------------------
-    # A pass of n rows costs the four matrices of a 27B layer 171 us at 16 rows, 174 at 24, 214 at 128; a
-    # pass of 8 rows 58, and its mixers run per pass: from three of those on, one of the former is faster.
+    # The four matrices of a 27B layer take 157 us at 16 rows, 163 at 24, 210 at 128; in a pass of 8 rows 57,
+    # and its mixers run per pass: from three of those on, one of the former is faster.
     ROWS, ROWS_MIN = 128, 24
 
     def rows_ok(self) -> bool:

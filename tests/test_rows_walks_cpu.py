@@ -114,7 +114,7 @@ def test_walk(tiles, G, N):
                 for n in range(c0, min(c0 + cols, N)):
                     assert (t, n) not in seen
                     seen.add((t, n))
-        U, P = (1, 3) if cols > 64 else (2, 2)
+        U, P = (1, 3) if cols > 64 else (2, 2) if cols > 48 else (3, 1)
         for grp in range(U):  # the cursor of a group of unpacking warps
             cj, cg, out = 0, grp, []
             while True:
@@ -129,7 +129,7 @@ def test_walk(tiles, G, N):
             nb = -(-min(cols, N - c0) // 16)
             each = (nb + P - 1) // P
             mine3 = [(each * h, min(each, max(0, nb - each * h))) for h in range(P)]
-            assert [b for b0, n in mine3 for b in range(b0, b0 + n)] == list(range(nb)) and each <= P
+            assert [b for b0, n in mine3 for b in range(b0, b0 + n)] == list(range(nb)) and each <= (2 if P == 2 else 3)
             assert whole or 16 * (mine3[-1][0] + mine3[-1][1]) <= 64 or nb <= 4
     assert len(seen) == tiles * N
 
