@@ -173,6 +173,15 @@ int qe_gdn_prefill(const void* qkv, const void* z, const void* b, const void* a,
                    const int* ctl, void* out, long ldo, int n, int Hk, int Hv, int D, float eps,
                    void* stream);
 
+/* The same for n = 8, 16 .. 128 rows in four launches whose serial part alone runs on few SMs; wire_out: the
+ * rows of out in the order that qe_w4_rows takes. workspace: qe_gdn_rows_workspace bytes, 16-byte
+ * aligned, any contents. */
+long qe_gdn_rows_workspace(int n, int Hk, int Hv, int D);
+int qe_gdn_rows(const void* qkv, const void* z, const void* b, const void* a, long ldp, void* ring,
+                const void* conv_w, const void* A_log, const void* dt_bias, const void* norm_w, float* S,
+                float* st_k, float* st_v, float* st_g, const int* ctl, void* out, long ldo, int n, int Hk,
+                int Hv, int D, float eps, int wire_out, void* workspace, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Gated GQA attention for n rows at positions pos[0] + t (csrc/ops.h:25-30, csrc/attn.cu).
  * hd = head dim (64, 128 or 256; the reference fixes 256, csrc/bindings.cpp:155).
@@ -374,6 +383,7 @@ int qe_w4_gemv_static(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream)
  * split is skipped (same result up to fp32 rounding of the order of additions, fewer SMs busy).
  * Of cfg only pdl and variant are read. */
 #define QE_MAX_GEMM_ROWS 64
+#define QE_MAX_PASS_ROWS 128
 int qe_w4_plan_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, qe_w4_plan* plan);
 int qe_w4_gemm(const qe_w4_params* p, const qe_w4_cfg* cfg, void* stream);
 /* qe_w4_gemm whose default kernel gives a wait up after wait_limit polls of its barrier instead of the
@@ -387,7 +397,6 @@ int qe_w4_gemm_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wait_lim
  * 64-k chunk with element 16 t + 4 s + j at position 16 s + 4 t + j (s, t, j < 4); wire_out: the rows of out
  * are left in that order (M a multiple of 64), as input of the next product. Needs K == Kp, bf16 x with
  * 16-byte aligned rows, ldx % 8 == 0 and ldx >= K. _bounded: see qe_w4_gemm_bounded. */
-#define QE_MAX_PASS_ROWS 128
 /* qe_w4_norm_rows for N = 1..QE_MAX_PASS_ROWS with xn_out in wire order (K a multiple of 64 that the launch options' CTA holds in
  * registers: at most 16 per thread); the bits are the same. */
 int qe_w4_norm_rows_wire(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, void* stream);

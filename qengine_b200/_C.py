@@ -261,6 +261,27 @@ def gdn_prefill(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_
                              float(eps), _stream()), "gdn_prefill", kernels=2)
 
 
+def gdn_rows_workspace(n, Hk, Hv, D):
+    """Bytes of workspace of `gdn_rows`."""
+    return int(lib.qe_gdn_rows_workspace(int(n), int(Hk), int(Hv), int(D)))
+
+
+def gdn_rows(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g, ctl, out, Hk, eps, workspace,
+             wire_out=False):
+    """`gdn_prefill` for up to 128 rows, the same bits, faster from 24 rows on: four launches around a
+    workspace (uint8, `gdn_rows_workspace` bytes). wire_out: out in the order that `_w4.rows` takes. Not in
+    the reference."""
+    n, Hk, Hv, D, qld, old = _gdn_check(qkv, z, b, a, ring, conv_w, A_log, dt_bias, norm_w, S, st_k, st_v, st_g,
+                                        ctl, out, Hk, range(8, 129, 8), "8, 16 .. 128 rows")
+    _req(workspace.is_cuda and workspace.dtype == torch.uint8 and workspace.is_contiguous() and
+         workspace.numel() >= gdn_rows_workspace(n, Hk, Hv, D) and workspace.data_ptr() % 16 == 0, "workspace")
+    check(lib.qe_gdn_rows(qkv.data_ptr(), z.data_ptr(), b.data_ptr(), a.data_ptr(), qld,
+                          ring.data_ptr(), conv_w.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
+                          norm_w.data_ptr(), S.data_ptr(), st_k.data_ptr(), st_v.data_ptr(),
+                          st_g.data_ptr(), ctl.data_ptr(), out.data_ptr(), old, n, Hk, Hv, D,
+                          float(eps), int(bool(wire_out)), workspace.data_ptr(), _stream()), "gdn_rows", kernels=4)
+
+
 def _attn_prep(fn, rows, qg, k, v, qnw, knw, inv_freq, pos, q_out, kc, vc, eps):
     gn, gw, gld = _rows(qg, BF, "qg")
     kn, kw, kld = _rows(k, BF, "k")

@@ -73,6 +73,9 @@ SIGNATURES = {
     "qe_force_drafts": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P]),
     "qe_gdn_step_n": (c_int, [P, P, P, P, c_long, P, P, P, P, P, P, P, P, P, P, P, c_long, c_int,
                               c_int, c_int, c_int, c_float, c_int, P]),
+    "qe_gdn_rows_workspace": (c_long, [c_int] * 4),
+    "qe_gdn_rows": (c_int, [P, P, P, P, c_long, P, P, P, P, P, P, P, P, P, P, P, c_long, c_int, c_int, c_int, c_int,
+                            C.c_float, c_int, P, P]),
     "qe_gdn_prefill": (c_int, [P, P, P, P, c_long, P, P, P, P, P, P, P, P, P, P, P, c_long, c_int,
                                c_int, c_int, c_int, c_float, P]),
     "qe_attn_prep_rows": (c_int, [P, P, P, c_long, P, P, P, P, P, P, P, c_int, c_int, c_int, c_int,

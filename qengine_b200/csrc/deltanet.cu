@@ -577,6 +577,15 @@ __global__ void gdn_ring_kernel(const bf16* qkv, long ldp, bf16* ring, const int
   if (c < C) ring[(size_t)((ctl[0] + t) & (kRing - 1)) * C + c] = qkv[(long)t * ldp + c];
 }
 
+}  // namespace
+
+cudaError_t launch_gdn_ring(const bf16* qkv, long ldp, bf16* ring, const int* ctl, int n, int C, cudaStream_t s, bool pdl) {
+  return launch(gdn_ring_kernel, dim3((C + 255) / 256, n < kRing ? n : kRing), dim3(256), 0, s, pdl, qkv, ldp, ring, ctl, n,
+                C);
+}
+
+namespace {
+
 template <int D>
 cudaError_t launch_gdn_prefill(const GdnArgs& g, cudaStream_t s, bool pdl) {
   static bool allowed[64] = {};
@@ -605,9 +614,7 @@ cudaError_t launch_gdn_prefill(const GdnArgs& g, cudaStream_t s, bool pdl) {
   c.numAttrs = pdl ? 2 : 1;
   e = cudaLaunchKernelEx(&c, gdn_prefill_kernel<D>, g);
   if (e != cudaSuccess) return e;
-  const int C = (2 * g.Hk + g.Hv) * D;
-  return launch(gdn_ring_kernel, dim3((C + 255) / 256, g.n < kRing ? g.n : kRing), dim3(256), 0, s, pdl, g.qkv, g.ldp,
-                g.ring, g.ctl, g.n, C);
+  return launch_gdn_ring(g.qkv, g.ldp, g.ring, g.ctl, g.n, (2 * g.Hk + g.Hv) * D, s, pdl);
 }
 
 // Off by default: the early state load assumes that no launch on the same state is still in

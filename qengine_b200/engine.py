@@ -776,10 +776,12 @@ class Engine:
             B.cat, B.mh = buf(W, 2 * H), buf(W, H)
         if W > self.WIDE:  # inputs of `_w4.rows` in wire order whose producers write them plain
             B.wire = buf(W, max(B.mix.size(1), 2 * H))
+            B.gdn_ws = buf(_C.gdn_rows_workspace(W, c.hk, c.hv, c.dk), dt=torch.uint8)
         return B
 
-    def _wide_mixer(self, L, n, B, kv_only=False):
-        """Token mixing of a wide pass. DeltaNet takes up to 64 rows in one launch, and so does the attention over
+    def _wide_mixer(self, L, n, B, exact=False, kv_only=False):
+        """Token mixing of a wide pass. DeltaNet takes all rows at once (exact: `_C.gdn_rows`, its result in the
+        order that `_w4.rows` takes), and up to 64 so does the attention over
         caches up to 8K positions; the tensor-core attention of longer caches takes 8 rows, and many
         splits as many as `_wide_attn_rows` says: beyond that the rows go through in sub-passes, each with
         its own control words (position, pending rows). kv_only: just write K and V (a draft layer during
@@ -794,11 +796,12 @@ class Engine:
             pr = B.proj[:n, :c.gdn_proj_rows]
             a0, a1 = c.conv_dim, c.conv_dim + c.value_dim
             out = B.mix[:n, :c.value_dim]
-            for rows, ctl in pieces(self.WIDE):
-                p = pr[rows]
-                _C.gdn_prefill(p[:, :a0], p[:, a0:a1], p[:, a1:a1 + c.hv], p[:, a1 + c.hv:], L["ring"], L["conv_w"],
-                               L["A_log"], L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"], L["st_g"], ctl,
-                               out[rows], c.hk, c.eps)
+            args = (pr[:, :a0], pr[:, a0:a1], pr[:, a1:a1 + c.hv], pr[:, a1 + c.hv:], L["ring"], L["conv_w"], L["A_log"],
+                    L["dt_bias"], L["norm_w"], L["S"], L["st_k"], L["st_v"], L["st_g"], self.ctl, out, c.hk, c.eps)
+            if exact:
+                _C.gdn_rows(*args, B.gdn_ws, wire_out=True)
+            else:
+                _C.gdn_prefill(*args)
             return out
         pr = B.proj[:n, :c.attn_proj_rows]
         nq = c.hq * 2 * c.head_dim
@@ -862,8 +865,8 @@ class Engine:
         for L in self.layers:
             block(L, h, None if first else mo, table_tok=B.tok if first else None)
             first = False
-            mixed = self._wide_mixer(L, n, B)
-            mm(wired(mixed), L["out"], mo)
+            mixed = self._wide_mixer(L, n, B, exact)
+            mm(mixed if L["type"] == "linear_attention" else wired(mixed), L["out"], mo)
             norm(h, mo, L["post_norm"], h_out=h)
             mm(xn, L["gate_up"], B.act[:n], wire_out=exact)
             mm(B.act[:n], L["down"], mo)
@@ -887,7 +890,7 @@ class Engine:
                 lin.norm_rows(B.hid[:n], None, M["pre_h"], eps, cat[:, H:])
             mm(wired(cat), M["fc"], B.mh[:n])
             block(M, B.mh[:n], None)
-            self._wide_mixer(M, n, B, kv_only=M["type"] != "linear_attention")
+            self._wide_mixer(M, n, B, exact, kv_only=M["type"] != "linear_attention")
         # commit: the position moves on by n; the last sub-pass left 8 DeltaNet rows pending
         self.ctl[self.POS].add_(n)
         self.ctl[self.PENDING].fill_(NMAX)

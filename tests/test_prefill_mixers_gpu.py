@@ -34,6 +34,40 @@ def prefill(L, rows):
     return out
 
 
+def split(L, rows, wire):
+    """`gdn_rows`: the same in four launches."""
+    from qengine_b200 import _w4
+    cfg, n = L.cfg, rows.shape[0]
+    c0, c1 = cfg.conv_dim, cfg.conv_dim + cfg.value_dim
+    r = rows.to(dev)[:, :c1 + 2 * cfg.hv]
+    out = torch.empty(n, cfg.value_dim, dtype=BF, device=dev)
+    size = L.C.gdn_rows_workspace(n, cfg.hk, cfg.hv, cfg.dk)
+    ws = torch.full((size + 64,), 255, dtype=torch.uint8, device=dev)
+    L.C.gdn_rows(r[:, :c0], r[:, c0:c1], r[:, c1:c1 + cfg.hv], r[:, c1 + cfg.hv:], L.ring, L.W["conv_w"],
+                 L.W["A_log"], L.W["dt_bias"], L.W["norm_w"], L.S, *L.st, L.ctl, out, cfg.hk, 1e-6, ws[:size], wire)
+    assert (ws[size:] == 255).all()
+    L.ctl[0] += n
+    L.ctl[1] = 8
+    return _w4.wire_order(out) if wire else out
+
+
+@pytest.mark.parametrize("hk,hv,d", [(16, 48, 128), (2, 4, 64), (1, 1, 128), (1, 3, 64)])
+@pytest.mark.parametrize("before,n", [(0, 8), (3, 24), (21, 40), (8, 64), (5, 72), (1, 128)])
+def test_deltanet_rows_equal_the_8_row_steps(C, hk, hv, d, before, n):
+    cfg, g = gdn_cfg(hk, hv, d), torch.Generator().manual_seed(before * 100 + n)
+    W = gdn_weights(cfg, seed=d)
+    A, B = GdnLayer(C, cfg, W), GdnLayer(C, cfg, W)
+    first, rows, last = (gdn_rows(cfg, k, g) for k in (before, n, 5))
+    for L in (A, B):
+        for i in range(0, before, 8):
+            L.run(first[i:i + 8], min(8, before - i))
+    want, got = steps(A, rows), split(B, rows, wire=n % 16 == 0)
+    assert torch.equal(want, got)
+    for a, b in zip((A.S, A.ring, A.ctl, *A.st), (B.S, B.ring, B.ctl, *B.st)):
+        assert torch.equal(a, b)
+    assert torch.equal(A.run(last, 5), B.run(last, 5))
+
+
 @pytest.mark.parametrize("hk,hv,d", [(16, 48, 128), (2, 4, 64), (1, 1, 128)])
 @pytest.mark.parametrize("before,n", [(0, 8), (0, 16), (3, 24), (8, 64), (21, 40), (1, 64)])
 def test_deltanet_prefill_equals_the_8_row_steps(C, hk, hv, d, before, n):
