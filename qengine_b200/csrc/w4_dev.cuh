@@ -181,7 +181,6 @@ struct OutDesc {
   int M, N;
   int epi;      // QE_EPI_*
   int out_f32;  // plain epilogue only: unrounded fp32 sums (partial results of a K-split matrix)
-  int wire;     // w4_rows.cu only: columns of a row in the order of the wire format (wire_pos)
 };
 
 // Where element k of a row stands when the row is kept in the order in which the wire format multiplies

@@ -47,6 +47,7 @@ struct RowsArgs {
   OutDesc o;  // o.N = all activation rows
   Deal d;
   int G, tiles;
+  int wire_out;      // rows of the output in wire order
   int cparts, cols;  // parts the columns (activation rows) are split into, columns of a part (a multiple of 16)
   int wait_limit;
 };
@@ -430,7 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         o.out = static_cast<unsigned char*>(o.out) + (size_t)c0 * o.ldo * (o.out_f32 ? 4 : 2);
         o.N = min(late->cols, o.N - c0);
         tc_store(o, tile0_of(j), tid - 32, kDrain * 32,
-                 [&](int n, int m0) { return *reinterpret_cast<const float4*>(stage + n * kPitch + m0); });
+                 [&](int n, int m0) { return *reinterpret_cast<const float4*>(stage + n * kPitch + m0); }, late->wire_out != 0);
       }
     }
     if (!ok) {
@@ -501,7 +502,7 @@ extern "C" int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, i
   a.o.N = p->N;
   a.o.epi = p->epilogue;
   a.o.out_f32 = (p->out_f32 && p->epilogue == QE_EPI_NONE) ? 1 : 0;
-  a.o.wire = wire_out ? 1 : 0;
+  a.wire_out = wire_out ? 1 : 0;
   a.G = p->Kp / 128;
   a.tiles = p->Mp / 16;
   a.wait_limit = wait_limit;

@@ -92,9 +92,9 @@ __device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap* map, i
 }
 
 // Four consecutive output rows (from `row`) of activation row n.
-__device__ __forceinline__ void tc_put4(const OutDesc& o, bool vec, int n, int row, const float4& f) {
+__device__ __forceinline__ void tc_put4(const OutDesc& o, bool vec, int n, int row, const float4& f, bool wire) {
   if (row >= o.M) return;
-  if (o.wire) row = wire_pos(row);
+  if (wire) row = wire_pos(row);
   const float e[4] = {f.x, f.y, f.z, f.w};
   if (o.out_f32) {
     float* p = static_cast<float*>(o.out) + (long)n * o.ldo + row;
@@ -116,9 +116,10 @@ __device__ __forceinline__ void tc_put4(const OutDesc& o, bool vec, int n, int r
     }
   }
 }
-// The finished sums of a super-tile, get(n, m) = those of its rows m .. m + 3, by `threads` threads.
+// The finished sums of a super-tile, get(n, m) = those of its rows m .. m + 3, by `threads` threads; wire: the
+// columns of an output row in the order of the wire format (wire_pos).
 template <typename Get>
-__device__ __forceinline__ void tc_store(const OutDesc& o, int tile0, int ti, int threads, Get get) {
+__device__ __forceinline__ void tc_store(const OutDesc& o, int tile0, int ti, int threads, Get get, bool wire = false) {
   const bool vec = (o.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(o.out) & (o.out_f32 ? 15 : 7)) == 0;
   if (o.epi == QE_EPI_SWIGLU) {  // rows 0..7 of a tile are gate rows, 8..15 the matching up rows
 #pragma unroll 2
@@ -126,12 +127,12 @@ __device__ __forceinline__ void tc_store(const OutDesc& o, int tile0, int ti, in
       const int n = e >> 4, m0 = (e & 14) * 8 + (e & 1) * 4;
       const float4 g = get(n, m0), u = get(n, m0 + 8);
       tc_put4(o, vec, n, tile0 * 8 + (e & 15) * 4,
-              make_float4(silu_fast(g.x) * u.x, silu_fast(g.y) * u.y, silu_fast(g.z) * u.z, silu_fast(g.w) * u.w));
+              make_float4(silu_fast(g.x) * u.x, silu_fast(g.y) * u.y, silu_fast(g.z) * u.z, silu_fast(g.w) * u.w), wire);
     }
   } else {
 #pragma unroll 2
     for (int e = ti; e < o.N * 32; e += threads)
-      tc_put4(o, vec, e >> 5, tile0 * 16 + (e & 31) * 4, get(e >> 5, (e & 31) * 4));
+      tc_put4(o, vec, e >> 5, tile0 * 16 + (e & 31) * 4, get(e >> 5, (e & 31) * 4), wire);
   }
 }
 // Tensor map over the rows of x as (64 k, rows, 64-k chunks): boxes of `chunks` chunks of `rows` rows in the

@@ -940,9 +940,9 @@ class Engine:
             self.reset()
 
     # -- passes of up to 128 rows with the bits of the ordinary ones -----------------------------------
-    # The four matrices of a 27B layer take 157 us at 16 rows, 163 at 24, 210 at 128; in a pass of 8 rows 57,
-    # and its mixers run per pass: from three of those on, one of the former is faster.
-    ROWS, ROWS_MIN = 128, 24
+    # The four matrices of a 27B layer take 163 us at 24 rows, 166 at 32, 210 at 128; in a pass of 8 rows 57, and
+    # its mixers run per pass. At 24 rows there is little to gain for the graph that every size needs once.
+    ROWS, ROWS_MIN = 128, 32
 
     def rows_ok(self) -> bool:
         """Prompts go through `_w4.rows` where that leaves what passes of 8 rows leave, bit for bit: the norms

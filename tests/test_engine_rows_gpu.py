@@ -63,13 +63,13 @@ def test_state_after_a_prompt(kind, P, kw):
                                b.view(torch.int16) if b.dtype == torch.bfloat16 else b), (name, mtp)
 
 
-@pytest.mark.parametrize("kind,T", [("tiny", 24), ("tiny", 25), ("small", 203), ("27b", 137)])
+@pytest.mark.parametrize("kind,T", [("tiny", 32), ("tiny", 33), ("small", 203), ("27b", 137)])
 def test_sequence_logits(kind, T):
     from qengine_b200 import synth
     cfg, eng = build(kind, mtp=False)
     seq = synth.prompt_ids(T, cfg.vocab, seed=7)
     got, best = eng.sequence_logits(seq), eng.sequence_logits(seq, keep="argmax")
-    assert bool(eng._row_blocks(T)) == (T > 24) == any(key[0] == "rows" for key in eng.graphs)
+    assert bool(eng._row_blocks(T)) == (T > 32) == any(key[0] == "rows" for key in eng.graphs)
     eng.rows_ok = lambda: False
     want = eng.sequence_logits(seq)
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
@@ -80,12 +80,12 @@ def test_requests():
     """Whole requests, plain, speculative and wide; options that leave the 8-row passes alone."""
     from qengine_b200 import synth
     cfg, eng = build("tiny")
-    prompt = synth.prompt_ids(285, cfg.vocab, seed=8)
+    prompt = synth.prompt_ids(293, cfg.vocab, seed=8)
     plain = eng.generate(prompt, 40)
-    assert ("rows", 128, False, False) in eng.graphs and ("rows", 24, False, False) in eng.graphs  # 128 + 128 + 24
+    assert ("rows", 128, False, False) in eng.graphs and ("rows", 32, False, False) in eng.graphs  # 128 + 128 + 32
     assert eng.generate_spec(prompt, 40, 3) == plain and eng.generate(prompt, 40, chunk=5) == plain
-    assert eng._row_blocks(285, 5) == [] and eng._row_blocks(285, 8, True) == [128, 128] and eng._row_blocks(24) == []
+    assert eng._row_blocks(293, 5) == [] and eng._row_blocks(293, 8, True) == [128, 128] and eng._row_blocks(32) == []
     wide = eng.generate(prompt, 40, wide=True)
     assert eng.generate_spec(prompt, 40, 4, wide=True) == wide
     _, plainer = build("tiny", fuse=False)
-    assert not plainer.rows_ok() and plainer._row_blocks(285) == []
+    assert not plainer.rows_ok() and plainer._row_blocks(293) == []
