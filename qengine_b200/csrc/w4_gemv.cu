@@ -440,7 +440,7 @@ __device__ __forceinline__ void grid_barrier(int* gbar, int nblocks) {
   __syncthreads();
 }
 
-// kAny: serves every shape and every row of x. Without, whole groups, tiles of a whole number of stages and
+// kAny: serves chains, every shape and every row of x. Without, one job of whole groups, tiles of a whole number of stages and
 // aligned rows only (plain_job): every matrix of the 27B model, with a stream loop that has nothing to decide.
 // One function for both costs that loop 1..4 % (registers), whichever way the two share it.
 template <int NW, int PERW, int STAGES, bool kAny>
@@ -503,8 +503,9 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
   }
   dep_wait();
 
+  const int njobs = kAny ? c.njobs : 1;  // chains are kAny's
 #pragma unroll 1
-  for (int j = 0; j < c.njobs; ++j) {
+  for (int j = 0; j < njobs; ++j) {
     const GemvArgs& a = c.job[j];
     const int G = a.G, total = a.d.total;
     if (j) range_of(a, u0, u1);
@@ -691,7 +692,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
 
     // This warp's ring is empty: ask for the head of its slab of the next matrix now, so that the
     // copies run while the blocks finish this job and meet at the barrier.
-    if (j + 1 < c.njobs) {
+    if (j + 1 < njobs) {
       int v0, v1;
       range_of(c.job[j + 1], v0, v1);
       __syncwarp();
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(NW * 32, 1) w4_chain_kernel(const __grid_const
       }
       publish(T, f, min(tend, cta_e) - cta_b, 0);
     }
-    if (j + 1 < c.njobs) grid_barrier(c.gbar, gridDim.x);  // also separates the uses of part / s_rb
+    if (j + 1 < njobs) grid_barrier(c.gbar, gridDim.x);  // also separates the uses of part / s_rb
   }
 }
 
@@ -1097,8 +1098,7 @@ int launch_chain(const qe_w4_params* const* ps, const qe_w4_norm* const* nrms, i
   }
   lc.attrs = at;
   lc.numAttrs = na;
-  bool plain = true;
-  for (int j = 0; j < njobs; ++j) plain = plain && plain_job(c.job[j], geom->perw);
+  const bool plain = njobs == 1 && plain_job(c.job[0], geom->perw);
   return (int)cudaLaunchKernelEx(&lc, plain ? geom->plain : geom->any, c);
 }
 
