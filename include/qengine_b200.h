@@ -396,12 +396,17 @@ int qe_w4_gemm_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wait_lim
  * decide the order of the additions). No counterpart in the reference. The rows of x are in wire order: every
  * 64-k chunk with element 16 t + 4 s + j at position 16 s + 4 t + j (s, t, j < 4); wire_out: the rows of out
  * are left in that order (M a multiple of 64), as input of the next product. Needs K == Kp, bf16 x with
- * 16-byte aligned rows, ldx % 8 == 0 and ldx >= K. _bounded: see qe_w4_gemm_bounded. */
+ * 16-byte aligned rows, ldx % 8 == 0 and ldx >= K. p->ws: NULL, or qe_w4_rows_ws_floats(p, cfg) floats (16-byte
+ * aligned, any contents, of no other launch that may run at the same time), with which a matrix of few rows is
+ * split along K and takes less time; 0 floats: no use for any. The bits are the same. _bounded: see
+ * qe_w4_gemm_bounded. */
+int qe_w4_rows(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, void* stream);
+long qe_w4_rows_ws_floats(const qe_w4_params* p, const qe_w4_cfg* cfg);
+int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, int wait_limit, void* stream);
+
 /* qe_w4_norm_rows for N = 1..QE_MAX_PASS_ROWS with xn_out in wire order (K a multiple of 64 that the launch options' CTA holds in
  * registers: at most 16 per thread); the bits are the same. */
 int qe_w4_norm_rows_wire(const qe_w4_norm* nrm, int N, int K, const qe_w4_cfg* cfg, void* stream);
-int qe_w4_rows(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, void* stream);
-int qe_w4_rows_bounded(const qe_w4_params* p, const qe_w4_cfg* cfg, int wire_out, int wait_limit, void* stream);
 
 /* Packs W [M, K] (row stride ld0; dtype 0 bf16, 1 fp16, 2 fp32) into the wire format on the GPU: qw
  * int32 [Mp/16, Kp/64, 32, 4] (16-byte aligned), scales fp16 [Mp/16, Kp/128, 16]. With w1 != NULL w0 / w1

@@ -109,6 +109,7 @@ SIGNATURES = {
     "qe_w4_gemm": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), P]),
     "qe_w4_norm_rows_wire": (c_int, [C.POINTER(W4Norm), c_int, c_int, C.POINTER(W4Cfg), P]),
     "qe_w4_rows": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, P]),
+    "qe_w4_rows_ws_floats": (c_long, [C.POINTER(W4Params), C.POINTER(W4Cfg)]),
     "qe_w4_rows_bounded": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, c_int, P]),
     "qe_w4_gemm_bounded": (c_int, [C.POINTER(W4Params), C.POINTER(W4Cfg), c_int, P]),
     "qe_w4_pack": (c_int, [P, P, c_int, c_int, c_int, c_long, c_long, P, P, P]),

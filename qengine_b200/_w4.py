@@ -406,6 +406,10 @@ def rows(x, qw, scales, out, M, swiglu=False, wire_out=False, warps=0, unroll=0,
     p = W4Params(qw.data_ptr(), scales.data_ptr(), x.data_ptr(), out.data_ptr(), None, None, M, K, Mp, Kp, N,
                  x.stride(0), out.stride(0), EPI_SWIGLU if swiglu else EPI_NONE, int(out_f32), 0)
     cfg = _cfg(warps, unroll, ksplit, pdl, variant, mode, blocks_per_sm, min_units)
+    floats = lib.qe_w4_rows_ws_floats(C.byref(p), C.byref(cfg))
+    if floats > 0:  # a split along K
+        ws = torch.empty(floats, dtype=torch.float32, device=x.device)
+        p.ws = ws.data_ptr()
     check(lib.qe_w4_rows(C.byref(p), C.byref(cfg), int(bool(wire_out)), _stream()), "w4 rows")
 
 

@@ -72,6 +72,38 @@ def test_swiglu_wire_order_options_and_sums(n, opts):
     assert torch.equal(sums.view(torch.int32), one.view(torch.int32))
 
 
+@pytest.mark.parametrize("M,K", [(5120, 17408), (5120, 6144), (4096, 4096), (1040, 3456), (1008, 16384), (72, 8064)])
+@pytest.mark.parametrize("n", [1, 16, 49, 67, 128])
+@pytest.mark.parametrize("limit", [1 << 20, 0, 3])
+def test_split_along_k(M, K, n, limit):
+    """With scratch a matrix of few rows is split along K: the bits of the unsplit product, nothing outside of the
+    scratch and the output, and a way out when waits run out."""
+    import ctypes as C
+
+    from qengine_b200 import _w4
+    from qengine_b200._lib import W4Cfg, W4Params, lib
+    p, x = packed(M, K, 12), _w4.wire_order(rand_x(n, K, 13, wild=True))
+    want, got = (torch.full((n, M), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    cfg, stream = W4Cfg(0, 0, 0, 1, 0, -1, 0, 4), torch.cuda.current_stream().cuda_stream
+    a = W4Params(p.qw.data_ptr(), p.scales.data_ptr(), x.data_ptr(), want.data_ptr(), None, None, M, K, 16 * p.qw.size(0),
+                 K, n, K, M, 0, 0, 0)
+    assert lib.qe_w4_rows(C.byref(a), C.byref(cfg), 0, stream) == 0
+    floats = lib.qe_w4_rows_ws_floats(C.byref(a), C.byref(cfg))
+    assert floats > 0 if M > 2000 else floats >= 0
+    ws = torch.full((floats + 64,), float("nan"), device=DEV)
+    a.ws, a.out = ws.data_ptr(), got.data_ptr()
+    assert lib.qe_w4_rows_bounded(C.byref(a), C.byref(cfg), 0, limit, stream) == 0
+    error = _w4.ring_error()
+    assert error == 0 if limit > 3 else error > 0 if limit == 0 else error >= 0
+    assert error or same(got, want)
+    assert ws[floats:].isnan().all()
+    assert lib.qe_w4_clear_error() == 0
+    assert lib.qe_w4_rows(C.byref(a), C.byref(cfg), 0, stream) == 0
+    assert _w4.ring_error() == 0 and same(got, want)
+    a.ws = ws.data_ptr() + 4
+    assert lib.qe_w4_rows(C.byref(a), C.byref(cfg), 0, stream) == -22
+
+
 def test_special_values():
     """Rows of zeros, infinities and NaN stay what the GEMV makes of them, and among themselves."""
     from qengine_b200 import _w4
