@@ -15,7 +15,7 @@
 //     memory; described in front of it, further down.
 //   * w4_gemm_kernel (cfg->variant == 1): mma.sync.m16n8k16 on register fragments, described
 //     next. With 8 row tiles it issues eight times the mma.sync instructions of the GEMV per
-//     unit and saturates near 130 TFLOP/s, the rate of the legacy tensor path on this part: 64
+//     unit and saturates near 130 TFLOP/s (mma.sync alone reaches 541 on this part): 64
 //     rows cost about as much as the eight GEMV passes they replace. It is kept as the measured
 //     baseline of the tensor-memory kernel and as a second implementation the tests compare.
 //
